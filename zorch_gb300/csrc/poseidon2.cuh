@@ -55,21 +55,93 @@ ZC_HD uint32_t ark_sbox_a(uint32_t x, uint32_t c, uint32_t alpha) {
   return mpow<F>(madd<F>(x, c), alpha);
 }
 
-// Multiplications by the built-in BabyBear diagonal entries without a
-// Montgomery product (the representation is linear, so a constant c acts on
-// Mont(x) as on x). p = 15 * 2^27 + 1, so for k <= 27 and q = (-x) mod 2^k,
-// x + q*p is divisible by 2^k and x * 2^-k = ((x + q) >> k) + q * 15 * 2^(27-k).
+// Constants of the built-in instance less p, so that the round-constant addition
+// into (-p, p) is a plain two-operand add (ark_sbox_bb16).
+struct Bb16Ext {
+  uint32_t v[64];
+};
+constexpr Bb16Ext bb16_less_p(const uint32_t (&c)[64]) {
+  Bb16Ext t{};
+  for (int i = 0; i < 64; i++) t.v[i] = c[i] - BabyBear::P;
+  return t;
+}
+constexpr uint32_t kBb16ExtInit[64] = ZC_BB16_EXT_INIT_MONT_INIT;
+constexpr uint32_t kBb16ExtTerm[64] = ZC_BB16_EXT_TERM_MONT_INIT;
+static __constant__ Bb16Ext c_bb16_init_lp = bb16_less_p(kBb16ExtInit);
+static __constant__ Bb16Ext c_bb16_term_lp = bb16_less_p(kBb16ExtTerm);
+// Zero, but not to the compiler: see smul3.
+static __constant__ uint32_t c_zero = 0;
+
+// smul with its subtraction as a three-operand add. The S-boxes of a
+// permutation keep the FMA pipe's integer multiplier busy (a 32 x 32 -> 64 or
+// high product takes it 4 cycles of a warp, a low product 2, 10 in all per
+// Montgomery product; measured), and the compiler likes to spread two-operand
+// adds onto that pipe as multiply-adds. A third operand it cannot see to be
+// zero keeps the subtraction on the ALU pipe: 8 % less time for the whole
+// permutation (1.90 against 2.03 ms for 2^20 threads x 8 permutations, before
+// the partial rounds below were rearranged; 1.74 against 1.83 ms after).
+template <class F>
+__device__ __forceinline__ int32_t smul3(int32_t a, int32_t b) {
+  const int64_t c = (int64_t)a * b;
+  const uint32_t m = (uint32_t)c * F::MU;
+  const int32_t mp = __mulhi((int32_t)m, (int32_t)F::P);
+  return (int32_t)((uint32_t)(c >> 32) - (uint32_t)mp + c_zero);
+}
+
+// The built-in BabyBear-16 instance (x^7, 4 + 4 full and 13 partial rounds),
+// one state per thread.
+//
+// What bounds it: the FMA pipe's multiplier (564 Montgomery products, 5,640
+// cycles of a warp) and the ALU pipe, which every high or wide product also
+// holds for 2 cycles and every other instruction for 2; together 93 % of what
+// the two pipes can give. So an instruction saved is about a cycle saved, and
+// the partial rounds, 13 x 118 instructions as written in the definition, are
+// rearranged to need fewer:
+//  - The diagonal [-2, 1, 2, 1/2, 3, 4, -1/2, -3, -4, 2^-8, 1/4, 1/8, 2^-27,
+//    -2^-8, -1/16, -2^-27] holds five pairs (d, -d), at words (3, 6), (4, 7),
+//    (5, 8), (9, 13), (12, 15). A pair (a, b) is carried as h = (a + b)/2 and
+//    g = (a - b)/2: then h' = sum + d g and g' = d h, so the sum over the
+//    words needs one addition per pair, the update one addition per pair, and
+//    over two rounds h'' = sum' + d^2 h with no g at all.
+//  - Multiplications by 2^-k need no product: p = 15 * 2^27 + 1, so with q the
+//    low k bits of x, x 2^-k = (x >> k) - q * 15 * 2^(27-k), in (-p, p).
+// 87 instructions per partial round, 5,190 per permutation (5,880 before):
+// 1.654 against 1.911 ms for 2^20 threads x 8 permutations at the same clock.
 struct Bb {
-  static constexpr uint32_t P = BabyBear::P;
-  __device__ __forceinline__ static uint32_t dbl(uint32_t x) { return madd<BabyBear>(x, x); }
+  using F = BabyBear;
+  static constexpr uint32_t P = F::P;
+  __device__ __forceinline__ static uint32_t add(uint32_t a, uint32_t b) { return madd<F>(a, b); }
+  __device__ __forceinline__ static uint32_t dbl(uint32_t x) { return madd<F>(x, x); }
   __device__ __forceinline__ static uint32_t half(uint32_t x) {
-    return (x & 1u) ? (x >> 1) + ((P + 1) >> 1) : (x >> 1);
+    return (x >> 1) + (x & 1u) * ((P + 1) >> 1);
+  }
+  // x 2^-K in (-p, p / 2^K] for x in [0, p).
+  template <int K>
+  __device__ __forceinline__ static int32_t shr(uint32_t x) {
+    static_assert(K >= 1 && K <= 27, "k out of range");
+    return (int32_t)((x >> K) - (x & ((1u << K) - 1u)) * (15u << (27 - K)));
   }
   template <int K>
   __device__ __forceinline__ static uint32_t div2exp(uint32_t x) {
+    return snorm<F>(shr<K>(x));
+  }
+  // sum + x 2^-K in [0, p): the sum of the three terms lies in (-p, p + p/2^K],
+  // so one correction from below and one from above (an instruction less than
+  // normalising x 2^-K first).
+  template <int K>
+  __device__ __forceinline__ static uint32_t add_div2exp(uint32_t sum, uint32_t x) {
     static_assert(K >= 1 && K <= 27, "k out of range");
-    const uint32_t q = (0u - x) & ((1u << K) - 1u);
-    const uint32_t r = ((x + q) >> K) + q * (15u << (27 - K));
+    const uint32_t r =
+        snorm<F>((int32_t)((sum + (x >> K)) - (x & ((1u << K) - 1u)) * (15u << (27 - K))));
+    const uint32_t t = r - P;
+    return t < r ? t : r;
+  }
+  // 2^K x: the bits above 2^31 come back as 2^31 = 2^27 - 1 (mod p); below 2p
+  // for x in [0, p) and K <= 4.
+  template <int K>
+  __device__ __forceinline__ static uint32_t mul2exp(uint32_t x) {
+    static_assert(K >= 1 && K <= 4, "k out of range");
+    const uint32_t r = ((x << K) & 0x7fffffffu) + (x >> (31 - K)) * ((1u << 27) - 1u);
     const uint32_t t = r - P;
     return t < r ? t : r;
   }
@@ -77,49 +149,103 @@ struct Bb {
 
 struct Bb16Builtin {
   using F = BabyBear;
-  // Internal layer s_i <- sum + d_i s_i for the built-in diagonal
-  // [-2, 1, 2, 1/2, 3, 4, -1/2, -3, -4, 2^-8, 1/4, 1/8, 2^-27, -2^-8, -1/16, -2^-27]
-  // on the integer ALU pipe instead of 16 Montgomery products.
-  __device__ __forceinline__ void internal_layer(uint32_t* s) const {
+  static constexpr bool kOwnPermute = true;
+  // x + c in (-p, p), c_lp = c - p; the power chain is unnormalised.
+  __device__ __forceinline__ static uint32_t sbox(uint32_t x, uint32_t c_lp) {
+    const int32_t a = (int32_t)(x + c_lp);
+    const int32_t a2 = smul3<F>(a, a);
+    return snorm<F>(smul3<F>(smul3<F>(a2, a), smul3<F>(a2, a2)));
+  }
+  // One full round, M4 block by block: the next block's S-boxes (FMA pipe) are
+  // independent of this block's additions (ALU pipe).
+  __device__ __forceinline__ static void full_round(uint32_t* s, const uint32_t* c_lp);
+
+  // One partial round. For each pair h = h_r and hp = h_{r-1}; for the last one
+  // (d = 2^-27, whose square is no power of two that shr takes) hp = g_r =
+  // d h_{r-1}, in (-p, 16). FIRST: hp = a - b of the words as they came in.
+  template <bool FIRST>
+  __device__ __forceinline__ static void partial_round(uint32_t* s, uint32_t (&h)[5],
+                                                       uint32_t (&hp)[5], uint32_t c) {
     using B = Bb;
-    uint32_t part = madd<F>(madd<F>(madd<F>(s[1], s[2]), madd<F>(s[3], s[4])),
-                            madd<F>(madd<F>(s[5], s[6]), madd<F>(s[7], s[8])));
-    part = madd<F>(part, madd<F>(madd<F>(madd<F>(s[9], s[10]), madd<F>(s[11], s[12])),
-                                 madd<F>(madd<F>(s[13], s[14]), s[15])));
-    const uint32_t sum = madd<F>(part, s[0]);
-    s[0] = msub<F>(part, s[0]);  // sum - 2 s0
-    s[1] = madd<F>(sum, s[1]);
-    s[2] = madd<F>(sum, B::dbl(s[2]));
-    s[3] = madd<F>(sum, B::half(s[3]));
-    s[4] = madd<F>(sum, madd<F>(B::dbl(s[4]), s[4]));
-    s[5] = madd<F>(sum, B::dbl(B::dbl(s[5])));
-    s[6] = msub<F>(sum, B::half(s[6]));
-    s[7] = msub<F>(sum, madd<F>(B::dbl(s[7]), s[7]));
-    s[8] = msub<F>(sum, B::dbl(B::dbl(s[8])));
-    s[9] = madd<F>(sum, B::div2exp<8>(s[9]));
-    s[10] = madd<F>(sum, B::div2exp<2>(s[10]));
-    s[11] = madd<F>(sum, B::div2exp<3>(s[11]));
-    s[12] = madd<F>(sum, B::div2exp<27>(s[12]));
-    s[13] = msub<F>(sum, B::div2exp<8>(s[13]));
+    const uint32_t y = sbox(s[0], c - F::P);
+    const uint32_t H = B::add(B::add(B::add(h[0], h[1]), B::add(h[2], h[3])), h[4]);
+    const uint32_t part = B::add(B::add(B::add(s[1], s[2]), B::add(s[10], s[11])),
+                                 B::add(s[14], B::dbl(H)));  // words 1..15
+    const uint32_t sum = B::add(part, y);
+    s[0] = msub<F>(part, y);  // sum - 2 y
+    s[1] = B::add(sum, s[1]);
+    s[2] = B::add(sum, B::dbl(s[2]));
+    s[10] = B::add(sum, B::div2exp<2>(s[10]));
+    s[11] = B::add(sum, B::div2exp<3>(s[11]));
     s[14] = msub<F>(sum, B::div2exp<4>(s[14]));
-    s[15] = msub<F>(sum, B::div2exp<27>(s[15]));
+    // h_{r+1} takes hp's place: sum + d^2 h_{r-1}, or sum + d (a - b) / 2
+    if (FIRST) {
+      hp[0] = B::add(sum, B::div2exp<2>(hp[0]));
+      hp[1] = B::add(B::add(sum, hp[1]), B::half(hp[1]));
+      hp[2] = B::add(sum, B::dbl(hp[2]));
+      hp[3] = B::add_div2exp<9>(sum, hp[3]);
+      const uint32_t hn = B::add_div2exp<27>(sum, B::half(hp[4]));
+      hp[4] = (uint32_t)B::shr<27>(h[4]);
+      h[4] = hn;
+    } else {
+      hp[0] = B::add(sum, B::div2exp<2>(hp[0]));
+      hp[1] = B::add(B::add(sum, hp[1]), B::mul2exp<3>(hp[1]));
+      hp[2] = B::add(sum, B::mul2exp<4>(hp[2]));
+      hp[3] = B::add_div2exp<16>(sum, hp[3]);
+      // d = 2^-27: h' = sum + d g, g' = d h. For g in (-p, 16) the shift is in
+      // [-15, 0], so the sum of the terms is in (-p, p): one correction.
+      const int32_t g = (int32_t)hp[4];
+      const uint32_t hn =
+          snorm<F>((int32_t)((sum + (uint32_t)(g >> 27)) - (hp[4] & 0x7ffffffu) * 15u));
+      hp[4] = (uint32_t)B::shr<27>(h[4]);
+      h[4] = hn;
+    }
   }
-  static constexpr int RF_HALF = ZC_BB16_ROUNDS_F_HALF;
-  __device__ __forceinline__ int rf_half() const { return RF_HALF; }
-  __device__ __forceinline__ int rp() const { return ZC_BB16_ROUNDS_P; }
-  __device__ __forceinline__ uint32_t ei(int r, int i) const { return c_bb16_ext_init[r * 16 + i]; }
-  __device__ __forceinline__ uint32_t et(int r, int i) const { return c_bb16_ext_term[r * 16 + i]; }
-  __device__ __forceinline__ uint32_t ir(int r) const { return c_bb16_int_rc[r]; }
-  __device__ __forceinline__ uint32_t dg(int i) const { return c_bb16_diag[i]; }
-  __device__ __forceinline__ uint32_t ark_sbox(uint32_t x, uint32_t c) const {
-    return ark_sbox_a<F, 7>(x, c, 7);
+  __device__ __forceinline__ static void partial_rounds(uint32_t* s) {
+    using B = Bb;
+    constexpr int ia[5] = {3, 4, 5, 9, 12}, ib[5] = {6, 7, 8, 13, 15};
+    uint32_t h[5], hp[5];
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+      h[i] = B::half(B::add(s[ia[i]], s[ib[i]]));
+      hp[i] = msub<F>(s[ia[i]], s[ib[i]]);
+    }
+    partial_round<true>(s, h, hp, c_bb16_int_rc[0]);
+    static_assert(ZC_BB16_ROUNDS_P % 2 == 1, "the remaining rounds run in twos");
+    // two rounds per turn: h and hp of the first four pairs change places
+#pragma unroll 1
+    for (int r = 1; r < ZC_BB16_ROUNDS_P; r += 2) {
+      uint32_t cur[5] = {hp[0], hp[1], hp[2], hp[3], h[4]};
+      uint32_t old[5] = {h[0], h[1], h[2], h[3], hp[4]};
+      partial_round<false>(s, cur, old, c_bb16_int_rc[r]);
+      uint32_t cur2[5] = {old[0], old[1], old[2], old[3], cur[4]};
+      uint32_t old2[5] = {cur[0], cur[1], cur[2], cur[3], old[4]};
+      partial_round<false>(s, cur2, old2, c_bb16_int_rc[r + 1]);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        h[i] = cur2[i];
+        hp[i] = old2[i];
+      }
+      h[4] = cur2[4];
+      hp[4] = old2[4];
+    }
+    // hp[0..3] = h_13 and h[0..3] = h_12 (g_13 = d h_12); h[4], hp[4] = h_13, g_13
+    const uint32_t g[5] = {B::half(h[0]), B::add(B::dbl(h[1]), h[1]), B::dbl(B::dbl(h[2])),
+                           B::div2exp<8>(h[3]), snorm<F>((int32_t)hp[4])};
+    const uint32_t hh[5] = {hp[0], hp[1], hp[2], hp[3], h[4]};
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+      s[ia[i]] = B::add(hh[i], g[i]);
+      s[ib[i]] = msub<F>(hh[i], g[i]);
+    }
   }
-  __device__ __forceinline__ uint32_t jsum(uint32_t s) const { return s; }
+  __device__ __forceinline__ void permute(uint32_t* s) const;
 };
 
 template <class F_>
 struct RtParams {
   using F = F_;
+  static constexpr bool kOwnPermute = false;
   const P2Params* p;  // shared memory on the device, plain memory on the host
   ZC_HD int rf_half() const { return (int)p->rounds_f_half; }
   ZC_HD int rp() const { return (int)p->rounds_p; }
@@ -148,19 +274,29 @@ struct RtParams {
   }
 };
 
+// M4 = circ(2, 3, 1, 1) on one 4-word block.
+template <class F>
+ZC_HD void m4_block(uint32_t (&x)[4]) {
+  const uint32_t t01 = madd<F>(x[0], x[1]), t23 = madd<F>(x[2], x[3]);
+  const uint32_t t0123 = madd<F>(t01, t23);
+  const uint32_t t01123 = madd<F>(t0123, x[1]), t01233 = madd<F>(t0123, x[3]);
+  const uint32_t y3 = madd<F>(t01233, madd<F>(x[0], x[0]));
+  const uint32_t y1 = madd<F>(t01123, madd<F>(x[2], x[2]));
+  x[0] = madd<F>(t01123, t01);
+  x[2] = madd<F>(t01233, t23);
+  x[1] = y1;
+  x[3] = y3;
+}
+
 // External (M4 block-circulant) linear layer.
 template <class F>
 ZC_HD void p2_ext_linear(uint32_t* s) {
 #pragma unroll
   for (int c = 0; c < 16; c += 4) {
-    uint32_t x0 = s[c], x1 = s[c + 1], x2 = s[c + 2], x3 = s[c + 3];
-    uint32_t t01 = madd<F>(x0, x1), t23 = madd<F>(x2, x3);
-    uint32_t t0123 = madd<F>(t01, t23);
-    uint32_t t01123 = madd<F>(t0123, x1), t01233 = madd<F>(t0123, x3);
-    s[c + 3] = madd<F>(t01233, madd<F>(x0, x0));
-    s[c + 1] = madd<F>(t01123, madd<F>(x2, x2));
-    s[c + 0] = madd<F>(t01123, t01);
-    s[c + 2] = madd<F>(t01233, t23);
+    uint32_t x[4] = {s[c], s[c + 1], s[c + 2], s[c + 3]};
+    m4_block<F>(x);
+#pragma unroll
+    for (int k = 0; k < 4; k++) s[c + k] = x[k];
   }
   uint32_t sums[4];
 #pragma unroll
@@ -170,27 +306,58 @@ ZC_HD void p2_ext_linear(uint32_t* s) {
   for (int i = 0; i < 16; i++) s[i] = madd<F>(s[i], sums[i & 3]);
 }
 
+__device__ __forceinline__ void Bb16Builtin::full_round(uint32_t* s, const uint32_t* c_lp) {
+  uint32_t col[4];
+#pragma unroll
+  for (int c = 0; c < 16; c += 4) {
+    uint32_t x[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) x[k] = sbox(s[c + k], c_lp[c + k]);
+    m4_block<F>(x);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      s[c + k] = x[k];
+      col[k] = c ? madd<F>(col[k], x[k]) : x[k];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 16; i++) s[i] = madd<F>(s[i], col[i & 3]);
+}
+
+__device__ __forceinline__ void Bb16Builtin::permute(uint32_t* s) const {
+  p2_ext_linear<F>(s);
+#pragma unroll 1
+  for (int r = 0; r < ZC_BB16_ROUNDS_F_HALF; r++) full_round(s, c_bb16_init_lp.v + 16 * r);
+  partial_rounds(s);
+#pragma unroll 1
+  for (int r = 0; r < ZC_BB16_ROUNDS_F_HALF; r++) full_round(s, c_bb16_term_lp.v + 16 * r);
+}
+
 #pragma nv_exec_check_disable
 template <class K>
 ZC_HD void p2_permute(uint32_t* s, const K& k) {
-  using F = typename K::F;
-  p2_ext_linear<F>(s);
-#pragma unroll 1
-  for (int r = 0; r < k.rf_half(); r++) {
-#pragma unroll
-    for (int i = 0; i < 16; i++) s[i] = k.ark_sbox(s[i], k.ei(r, i));
+  if constexpr (K::kOwnPermute) {
+    k.permute(s);
+  } else {
+    using F = typename K::F;
     p2_ext_linear<F>(s);
-  }
 #pragma unroll 1
-  for (int r = 0; r < k.rp(); r++) {
-    s[0] = k.ark_sbox(s[0], k.ir(r));
-    k.internal_layer(s);
-  }
-#pragma unroll 1
-  for (int r = 0; r < k.rf_half(); r++) {
+    for (int r = 0; r < k.rf_half(); r++) {
 #pragma unroll
-    for (int i = 0; i < 16; i++) s[i] = k.ark_sbox(s[i], k.et(r, i));
-    p2_ext_linear<F>(s);
+      for (int i = 0; i < 16; i++) s[i] = k.ark_sbox(s[i], k.ei(r, i));
+      p2_ext_linear<F>(s);
+    }
+#pragma unroll 1
+    for (int r = 0; r < k.rp(); r++) {
+      s[0] = k.ark_sbox(s[0], k.ir(r));
+      k.internal_layer(s);
+    }
+#pragma unroll 1
+    for (int r = 0; r < k.rf_half(); r++) {
+#pragma unroll
+      for (int i = 0; i < 16; i++) s[i] = k.ark_sbox(s[i], k.et(r, i));
+      p2_ext_linear<F>(s);
+    }
   }
 }
 
@@ -309,19 +476,6 @@ __device__ __forceinline__ uint32_t p2_permute_half(uint32_t x, const P2Params* 
 // half-warp form, at no longer a dependency chain; it is the form used where
 // many latency-bound permutations run side by side (tree tops, transcript).
 // Every lane of the warp must make the call (full-warp shuffles).
-template <class F>
-__device__ __forceinline__ void m4_block(uint32_t (&x)[4]) {
-  const uint32_t t01 = madd<F>(x[0], x[1]), t23 = madd<F>(x[2], x[3]);
-  const uint32_t t0123 = madd<F>(t01, t23);
-  const uint32_t t01123 = madd<F>(t0123, x[1]), t01233 = madd<F>(t0123, x[3]);
-  const uint32_t y3 = madd<F>(t01233, madd<F>(x[0], x[0]));
-  const uint32_t y1 = madd<F>(t01123, madd<F>(x[2], x[2]));
-  x[0] = madd<F>(t01123, t01);
-  x[2] = madd<F>(t01233, t23);
-  x[1] = y1;
-  x[3] = y3;
-}
-
 template <class F>
 __device__ __forceinline__ void quarter_ext_linear(uint32_t (&x)[4]) {
   m4_block<F>(x);

@@ -385,26 +385,28 @@ __global__ void __launch_bounds__(1024) k_subtree(Leaf leaf, uint32_t* layers, i
   }
 }
 
-// Resident 256-thread CTAs per SM k_leaf is compiled for: five for the
-// built-in instance (its level and leaf forms then use 40-46 registers, where
-// the unbounded build gave the level form 32; the 2^22 x 64 trace hash went
-// 9.18 -> 9.00 ms); no bound for run-time parameter sets, whose constants come
-// from shared memory and which would spill under it. The batched tree kernel
-// keeps the compiler's choice: bounding it to five or six resident CTAs
-// measured slower on the served stream (1.136 / 1.153 against 1.163 G elem/s).
+// Threads of a k_leaf CTA, and the CTAs per SM it is compiled for: eight for the
+// built-in instance (46 registers; the register file then holds ten, and 128
+// threads measured 1.74 ms where 256 took 1.76-1.79 for 2^20 x 8 permutations);
+// no bound for run-time parameter sets, whose constants come from shared memory
+// and which would spill under it. Small CTAs also spread a narrow level over
+// every SM: 2^15 parents are 256 CTAs, not 128. The batched tree kernel keeps
+// the compiler's choice: bounding it to five or six resident CTAs measured
+// slower on the served stream (1.136 / 1.153 against 1.163 G elem/s).
+constexpr int kLeafT = 128;
 template <class K>
 struct HashOcc {
   static constexpr int v = 1;
 };
 template <>
 struct HashOcc<Bb16Builtin> {
-  static constexpr int v = 5;
+  static constexpr int v = 8;
 };
 
 // One thread per leaf (or per parent for NodeLeaf): no shared memory, no
 // barriers, so every warp stays busy for the whole launch.
 template <class K, class Leaf>
-__global__ void __launch_bounds__(kMaxT, HashOcc<K>::v) k_leaf(Leaf leaf, uint32_t* out, int64_t count,
+__global__ void __launch_bounds__(kLeafT, HashOcc<K>::v) k_leaf(Leaf leaf, uint32_t* out, int64_t count,
                                                 const P2Params* rt) {
   __shared__ P2Params s_rt;
   K k = KIn<K>::make(rt, &s_rt);
@@ -430,7 +432,7 @@ zc_status finish_tree(uint32_t* layers, int64_t L, int l_done, const P2Params* r
     const int64_t parents = (L >> l) >> 1;
     NodeLeaf nl{layers + 8 * level_offset(L, l)};
     if (parents > tree_shape().levelwise_min) {
-      k_leaf<K, NodeLeaf><<<(unsigned)((parents + kMaxT - 1) / kMaxT), kMaxT, 0, st>>>(
+      k_leaf<K, NodeLeaf><<<(unsigned)((parents + kLeafT - 1) / kLeafT), kLeafT, 0, st>>>(
           nl, layers + 8 * level_offset(L, l + 1), parents, rt);
       ZC_TRY(launch_check());
       l += 1;
@@ -450,7 +452,7 @@ template <class K, class Leaf>
 zc_status commit_tree(const Leaf& leaf, uint32_t* layers, int64_t L, const P2Params* rt,
                       cudaStream_t st, RootHop hop = RootHop{nullptr, nullptr, 0}) {
   if (L > tree_shape().levelwise_min) {
-    k_leaf<K, Leaf><<<(unsigned)((L + kMaxT - 1) / kMaxT), kMaxT, 0, st>>>(leaf, layers, L, rt);
+    k_leaf<K, Leaf><<<(unsigned)((L + kLeafT - 1) / kLeafT), kLeafT, 0, st>>>(leaf, layers, L, rt);
     ZC_TRY(launch_check());
     return finish_tree<K>(layers, L, 0, rt, st, hop);
   }
