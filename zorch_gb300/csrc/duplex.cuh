@@ -75,100 +75,120 @@ struct HostPerm {
   void operator()(uint32_t* s) const { p2_permute(s, k); }
 };
 
-// Every lane of the (single) warp holds the same Duplex state and runs the same
-// control flow; a permutation runs on each half-warp (both compute the same
-// result) and is gathered back into every lane's copy.
-template <class HP>
-__device__ __forceinline__ void half_apply(uint32_t* s, const HP& perm) {
-  const int lane = threadIdx.x & 31;
-  uint32_t x = 0;
-#pragma unroll
-  for (int j = 0; j < 16; j++) x = (lane & 15) == j ? s[j] : x;
-  x = perm.half(x);
-#pragma unroll
-  for (int j = 0; j < 16; j++) s[j] = __shfl_sync(kFullMask, x, (lane & 16) | j);
-}
-
+// The half-warp permutation of a transcript kernel: run-time instances
+// (constants in shared memory) and the built-in one (this lane's constants in
+// registers, loaded once when the kernel starts).
 template <class F>
 struct HalfPerm {
   const P2Params* p;  // shared memory
   __device__ uint32_t half(uint32_t x) const { return p2_permute_half<F>(x, p); }
-  __device__ void operator()(uint32_t* s) const { half_apply(s, *this); }
 };
-
-// The built-in BabyBear-16 instance (half_permute_bb16): the constants of this
-// lane's word are loaded into registers once, when the transcript kernel
-// starts.
 struct HalfPermBb16 {
-  uint32_t ei[4], et[4], dg;
-  __device__ HalfPermBb16() {
-    const int l = threadIdx.x & 15;
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      ei[r] = c_bb16_ext_init[r * 16 + l];
-      et[r] = c_bb16_ext_term[r * 16 + l];
-    }
-    dg = c_bb16_diag[l];
-  }
-  __device__ uint32_t half(uint32_t x) const { return half_permute_bb16(x, ei, et, dg); }
-  __device__ void operator()(uint32_t* s) const { half_apply(s, *this); }
+  HalfBb16 h;
+  __device__ explicit HalfPermBb16(const P2Params* p) : h(p) {}
+  __device__ uint32_t half(uint32_t x) const { return h.permute(x); }
 };
 
-// duplex_observe on the device (same result): full rate blocks are absorbed
-// with the sponge kept one word per lane (lane l of each half holds word l),
-// each block's eight values loaded straight into lanes 0..7 -- the next
-// block's loads issued before the current permutation -- so a long observe
-// (a final fold layer, a sponge chain of hundreds of blocks) costs one
-// half-warp permutation per block and no per-word state shuffling. The
-// pending prefix and the tail take the generic path.
-template <class HP>
-__device__ void half_observe(Duplex& t, const uint32_t* v, int64_t m, const HP& perm) {
-  if (m <= 0) return;
-  int pos = t.in_pos & 7;
-  int64_t i = 0;
-  for (; pos != 0 && i < m; i++) {  // complete a pending block first
-    t.in_buf[pos++] = v[i];
-    if (pos == 8) {
-      for (int j = 0; j < 8; j++) t.sponge[j] = t.in_buf[j];
-      perm(t.sponge);
-      pos = 0;
+// The duplex on one warp: lane l of each half (both run the same) holds sponge
+// word l and, for l < 8, words l of the input and output buffers. The same
+// steps as duplex_observe and duplex_sample with no word-by-word state in
+// memory: a step costs its permutations and a few shuffles (a hop of one
+// absorbed block and four squeezed words took 8 us with the state in local
+// arrays, of which the permutation 2.5).
+struct LaneDuplex {
+  uint32_t in, out, x;
+  int in_pos, out_pos;
+
+  // buffers of the wire layout: in_buf[8], out_buf[8], sponge[16]
+  __device__ __forceinline__ void load(const uint32_t* in_buf, const uint32_t* out_buf,
+                                       const uint32_t* sponge, const uint32_t* in_p,
+                                       const uint32_t* out_p) {
+    const int l = threadIdx.x & 15;
+    in = l < 8 ? in_buf[l] : 0u;
+    out = l < 8 ? out_buf[l] : 0u;
+    x = sponge[l];
+    in_pos = (int)in_p[0];
+    out_pos = (int)out_p[0];
+  }
+  // Inputs may alias outputs: every lane has read them by now.
+  __device__ __forceinline__ void store(uint32_t* in_buf, uint32_t* out_buf, uint32_t* sponge,
+                                        uint32_t* in_p, uint32_t* out_p) const {
+    __syncwarp();
+    const int lane = threadIdx.x & 31;
+    if (lane < 8) {
+      in_buf[lane] = in;
+      out_buf[lane] = out;
+    }
+    if (lane < 16) sponge[lane] = x;
+    if (lane == 0) {
+      in_p[0] = (uint32_t)in_pos;
+      out_p[0] = (uint32_t)out_pos;
     }
   }
-  if (m - i >= 8) {
-    const int lane = threadIdx.x & 31, l = lane & 15;
-    uint32_t x = 0;
-#pragma unroll
-    for (int j = 0; j < 16; j++) x = l == j ? t.sponge[j] : x;
-    uint32_t nxt = l < 8 ? v[i + l] : 0u;
-    for (; m - i >= 8; i += 8) {
-      const uint32_t cur = nxt;
-      if (m - i >= 16 && l < 8) nxt = v[i + 8 + l];  // issued before the permutation
-      if (l < 8) x = cur;
+  __device__ __forceinline__ void load(const uint32_t* st) {
+    load(st, st + 8, st + 16, st + 32, st + 33);
+  }
+  __device__ __forceinline__ void store(uint32_t* st) const {
+    store(st, st + 8, st + 16, st + 32, st + 33);
+  }
+
+  template <class HP>
+  __device__ __forceinline__ void observe(const uint32_t* v, int64_t m, const HP& perm) {
+    if (m <= 0) return;
+    const int l = threadIdx.x & 15;
+    int pos = in_pos & 7;  // a corrupt caller state cannot index past the buffer
+    int64_t i = 0;
+    // a pending block is completed first; then whole blocks, each one's words
+    // loaded before the permutation that precedes them; the tail stays pending
+    uint32_t nxt = 0;
+    if (pos != 0) {
+      const int take = m < 8 - pos ? (int)m : 8 - pos;
+      if (l >= pos && l < pos + take) in = v[l - pos];
+      pos += take;
+      i = take;
+      if (pos == 8) nxt = in;
+    } else if (m >= 8) {
+      nxt = l < 8 ? v[l] : 0u;
+      pos = 8;
+      i = 8;
+    }
+    while (pos == 8) {
+      if (l < 8) x = nxt;
+      pos = 0;
+      if (m - i >= 8) {
+        if (l < 8) nxt = v[i + l];
+        pos = 8;
+        i += 8;
+      }
       x = perm.half(x);
     }
-#pragma unroll
-    for (int j = 0; j < 16; j++) t.sponge[j] = __shfl_sync(kFullMask, x, (lane & 16) | j);
+    if (pos == 0 && i < m) {
+      pos = (int)(m - i);
+      if (l < pos) in = v[i + l];
+    }
+    if (l >= pos) in = 0u;
+    in_pos = pos;
+    out = pos == 0 && l < 8 ? x : 0u;
+    out_pos = pos == 0 ? 8 : 0;
   }
-  for (; i < m; i++) {  // the tail stays pending (m - i < 8)
-    t.in_buf[pos++] = v[i];
+
+  // The next challenge word, on every lane.
+  template <class HP>
+  __device__ __forceinline__ uint32_t sample(const HP& perm) {
+    const int l = threadIdx.x & 15;
+    in_pos &= 7;
+    if (out_pos < 0 || out_pos > 8) out_pos = 0;
+    if (in_pos > 0 || out_pos == 0) {
+      if (l < in_pos) x = in;
+      x = perm.half(x);
+      in = 0u;
+      out = l < 8 ? x : 0u;
+      in_pos = 0;
+      out_pos = 8;
+    }
+    out_pos -= 1;
+    return __shfl_sync(kFullMask, out, out_pos);
   }
-  for (int j = pos; j < 8; j++) t.in_buf[j] = 0;
-  t.in_pos = pos;
-  if (pos == 0) {
-    for (int j = 0; j < 8; j++) t.out_buf[j] = t.sponge[j];
-    t.out_pos = 8;
-  } else {
-    for (int j = 0; j < 8; j++) t.out_buf[j] = 0;
-    t.out_pos = 0;
-  }
-}
-template <class F>
-__device__ void duplex_observe(Duplex& t, const uint32_t* v, int64_t m, const HalfPerm<F>& perm) {
-  half_observe(t, v, m, perm);
-}
-__device__ inline void duplex_observe(Duplex& t, const uint32_t* v, int64_t m,
-                                      const HalfPermBb16& perm) {
-  half_observe(t, v, m, perm);
-}
+};
 
 }  // namespace zc

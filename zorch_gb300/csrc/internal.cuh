@@ -28,11 +28,14 @@ struct KIn<Bb16Builtin> {
 template <class F>
 struct KIn<RtParams<F>> {
   __device__ static RtParams<F> make(const P2Params* g, P2Params* s) {
-    stage_params(s, g);
+    stage_params<0, kP2ThreadWords>(s, g);
     return RtParams<F>{s};
   }
-  // Already staged by make (same shared copy).
-  __device__ static const P2Params* half(const P2Params*, P2Params* s) { return s; }
+  // make has staged the front of the same shared copy.
+  __device__ static const P2Params* half(const P2Params* g, P2Params* s) {
+    stage_params<kP2ThreadWords, kP2Words>(s, g);
+    return s;
+  }
 };
 
 // Calls fn(K{}, device_params) with the provider matching the handle.

@@ -11,6 +11,8 @@
 //  - RtParams:    any width-16 instance passed at run time (the reference's
 //    Poseidon2Params), staged into shared memory by the kernel.
 #pragma once
+#include <stddef.h>
+
 #include "field.cuh"
 #include "poseidon2_babybear16.h"
 
@@ -29,12 +31,41 @@ struct P2Params {
   uint32_t diag[16];
   uint32_t j_scale;
   uint32_t j_is_one;
+  // Derived tables of the half-warp partial rounds (half_partials), for runs of
+  // up to `chain` rounds: chain_m[k][i] = j d_i^k as an int32 of least
+  // magnitude (0 for word 0), chain_t[k] = j sum_{i>=1} d_i^k, chain_e = j + d_0,
+  // chain_mode: 1 where d_0 = -2 j, 2 where j = 1 as well.
+  uint32_t chain;
+  uint32_t chain_mode;
+  uint32_t chain_e;
+  uint32_t chain_t[16];
+  alignas(16) int32_t chain_m[16][20];  // rows of 16, padded to spread 16-byte reads over the banks
 };
+constexpr int kChainMax = 16;
 
-static __constant__ uint32_t c_bb16_ext_init[64] = ZC_BB16_EXT_INIT_MONT_INIT;
-static __constant__ uint32_t c_bb16_ext_term[64] = ZC_BB16_EXT_TERM_MONT_INIT;
+// Fills the derived tables from diag, j_scale and rounds_p.
+template <class F>
+inline void p2_chain_tables(P2Params* p) {
+  const uint32_t runs = (p->rounds_p + kChainMax - 1) / kChainMax;
+  p->chain = runs ? (p->rounds_p + runs - 1) / runs : 0;
+  p->chain_e = madd<F>(p->j_scale, p->diag[0]);
+  p->chain_mode = madd<F>(p->chain_e, p->j_scale) ? 0 : (p->j_is_one ? 2 : 1);
+  uint32_t pw[16];
+  for (int i = 0; i < 16; i++) pw[i] = F::ONE;
+  for (int k = 0; k < kChainMax; k++) {
+    uint32_t t = 0;
+    for (int i = 0; i < 20; i++) p->chain_m[k][i] = 0;
+    for (int i = 1; i < 16; i++) {
+      t = madd<F>(t, pw[i]);
+      const uint32_t m = mmul<F>(p->j_scale, pw[i]);
+      p->chain_m[k][i] = m > F::P / 2 ? (int32_t)(m - F::P) : (int32_t)m;
+      pw[i] = mmul<F>(pw[i], p->diag[i]);
+    }
+    p->chain_t[k] = mmul<F>(p->j_scale, t);
+  }
+}
+
 static __constant__ uint32_t c_bb16_int_rc[ZC_BB16_ROUNDS_P] = ZC_BB16_INT_RC_MONT_INIT;
-static __constant__ uint32_t c_bb16_diag[16] = ZC_BB16_DIAG_MONT_INIT;
 
 // Round-constant addition and S-box x -> (x + c)^alpha for x, c in [0, p):
 // x + c - p lies in [-p, p) and is one three-operand add, and the power chain
@@ -380,37 +411,96 @@ ZC_HD void p2_compress(const uint32_t* l, const uint32_t* r, uint32_t* out,
 // ------------------------------------------------------------- halves ---
 // The same permutation on a half-warp (lanes 16h .. 16h+15): lane l of the
 // half holds state word l. One thread's permutation is a dependency chain of
-// ~7000 instructions (~9.4 us at 2.07 GHz, measured); on a half-warp each lane
-// runs one S-box per round and the linear layers are butterflies of shuffles,
-// which brings a permutation to ~3 us. The latency-bound parts of a commit --
-// the narrow top levels of a tree and the transcript -- use halves.
+// ~5,200 instructions (~9 us at 2.07 GHz); on a half-warp each lane runs one
+// S-box per round. The latency-bound parts of a commit -- the narrow top
+// levels of a tree and the transcript -- use halves, and what bounds them is
+// the dependency chain, so each step is arranged for the fewest dependent
+// operations (latencies measured: add 4.5 cycles, add and minimum 9, low
+// product 4.5, high or wide product 9.4, shuffle 24):
 //  - external layer: y_j = s_b + x_j + 2 x_{j+1} is M4 = circ(2,3,1,1) on the
 //    4-word block b (s_b = block sum, j + 1 mod 4), then y += the sum of y over
-//    the lane class (xor 4, xor 8);
-//  - partial round: the sum of lanes 1..15 is reduced while lane 0 runs its
-//    S-box, and lane 0's new word is broadcast and added afterwards.
+//    the lane class (l mod 4). The block's and the class's other three words
+//    come by three independent shuffles each: two shuffle latencies per layer,
+//    not four (a butterfly's);
+//  - partial rounds: half_partials.
+// 3,725 cycles for the built-in instance (9 external layers of 118, 8 S-boxes of
+// 102, 1,912 for the partial rounds); 4,900 with butterfly sums throughout.
 // Constants come from a P2Params in shared memory. Every lane of the warp must
 // make the call (full-warp shuffles), active half or not.
 constexpr unsigned kFullMask = 0xffffffffu;
 
 template <class F>
-__device__ __forceinline__ uint32_t half_sum16(uint32_t v) {
-  v = madd<F>(v, __shfl_xor_sync(kFullMask, v, 1));
-  v = madd<F>(v, __shfl_xor_sync(kFullMask, v, 2));
-  v = madd<F>(v, __shfl_xor_sync(kFullMask, v, 4));
-  return madd<F>(v, __shfl_xor_sync(kFullMask, v, 8));
+__device__ __forceinline__ uint32_t half_ext_linear(uint32_t x) {
+  const uint32_t a = __shfl_xor_sync(kFullMask, x, 1), b = __shfl_xor_sync(kFullMask, x, 2),
+                 c = __shfl_xor_sync(kFullMask, x, 3);
+  // x_{j+1}: lane j ^ 1 for an even j, j ^ 3 for an odd one
+  const uint32_t nxt = (threadIdx.x & 1) ? c : a;
+  const uint32_t u = madd<F>(x, madd<F>(nxt, nxt));
+  const uint32_t y = madd<F>(madd<F>(madd<F>(x, a), madd<F>(b, c)), u);
+  const uint32_t y2 = madd<F>(y, y);
+  const uint32_t d = __shfl_xor_sync(kFullMask, y, 4), e = __shfl_xor_sync(kFullMask, y, 8),
+                 f = __shfl_xor_sync(kFullMask, y, 12);
+  return madd<F>(madd<F>(y2, d), madd<F>(e, f));
 }
 
+// Montgomery reduction of c, |c| <= p^2, into (-p, p).
 template <class F>
-__device__ __forceinline__ uint32_t half_ext_linear(uint32_t x) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t nxt = __shfl_sync(kFullMask, x, (lane & ~3) | ((lane + 1) & 3));
-  uint32_t s = madd<F>(x, __shfl_xor_sync(kFullMask, x, 1));
-  s = madd<F>(s, __shfl_xor_sync(kFullMask, s, 2));
-  const uint32_t y = madd<F>(madd<F>(s, x), madd<F>(nxt, nxt));
-  uint32_t c = madd<F>(y, __shfl_xor_sync(kFullMask, y, 4));
-  c = madd<F>(c, __shfl_xor_sync(kFullMask, c, 8));
-  return madd<F>(y, c);
+__device__ __forceinline__ int32_t sredc(int64_t c) {
+  const uint32_t m = (uint32_t)c * F::MU;
+  return (int32_t)(c >> 32) - __mulhi((int32_t)m, (int32_t)F::P);
+}
+
+// n <= 16 partial rounds. Words 1..15 evolve linearly given the rounds' sums, so
+// with s_i the words at the start, y_r round r's S-box output and
+//   B_r = j * (sum of words 1..15 before round r)
+//       = sum_i j d_i^r s_i + sum_{m < r} j T_{r-1-m} sigma_m,  T_k = sum_{i>=1} d_i^k,
+// a round is sigma_r = j y_r + B_r and word 0 becomes (j + d_0) y_r + B_r: the chain
+// from one S-box to the next is one addition (a product more for j != 1), where
+// summing the fifteen words takes four shuffles and additions. Lane k
+// holds B_k: its first sum is a 15-term dot product (15 independent shuffles,
+// four terms to a reduction), and each round adds j T_{k-1-r} sigma_r to it
+// while the next S-box runs. Each lane l > 0 keeps its own word, x_l = sigma_r
+// + d_l x_l, off the chain too. Every lane runs the S-box of word 0. (Keeping x_l
+// as one wide accumulation, or B and x on the two halves of a warp in one
+// product, measured 10 % and 30 % slower: 2,107 and 2,504 cycles.)
+// MODE: 0: any j and d_0; 1: d_0 = -2 j, so word 0 becomes B_r - j y_r; 2: j = 1 too.
+// step(r, s0) = the S-box of round r on s0. Returns this lane's word.
+template <class F, int MODE, bool UNROLL, class Step>
+__device__ __forceinline__ uint32_t half_partials(uint32_t x, int n, uint32_t dg, uint32_t j,
+                                                  uint32_t e, uint32_t w, const int32_t (&m)[16],
+                                                  const Step& step) {
+  const int base = threadIdx.x & 16;
+  const int32_t xc = (int32_t)(x > F::P / 2 ? x - F::P : x);  // |xc| <= p/2
+  int32_t part[4];
+#pragma unroll
+  for (int g = 0; g < 4; g++) {
+    int64_t acc = 0;
+#pragma unroll
+    for (int i = 4 * g; i < 4 * g + 4; i++)
+      if (i) acc += (int64_t)m[i] * __shfl_sync(kFullMask, xc, base + i);  // |term| <= p^2 / 4
+    part[g] = sredc<F>(acc);
+  }
+  uint32_t B = madd<F>(madd<F>(snorm<F>(part[0]), snorm<F>(part[1])),
+                       madd<F>(snorm<F>(part[2]), snorm<F>(part[3])));
+  uint32_t s0 = __shfl_sync(kFullMask, x, base), b = __shfl_sync(kFullMask, B, base);
+  auto round = [&](int r) {
+    const uint32_t y = step(r, s0);
+    const uint32_t jy = MODE == 2 ? y : mmul<F>(y, j);
+    const uint32_t sigma = madd<F>(jy, b);
+    s0 = MODE > 0 ? msub<F>(b, jy) : madd<F>(mmul<F>(y, e), b);
+    x = madd<F>(sigma, mmul<F>(dg, x));
+    B = madd<F>(B, mmul<F>(w, sigma));
+    b = __shfl_sync(kFullMask, B, base + ((r + 1) & 15));
+    w = __shfl_up_sync(kFullMask, w, 1, 16);  // T_{k-1-r} for the next round
+  };
+  if constexpr (UNROLL) {
+#pragma unroll
+    for (int r = 0; r < ZC_BB16_ROUNDS_P; r++) round(r);
+  } else {
+#pragma unroll 1
+    for (int r = 0; r < n; r++) round(r);
+  }
+  return (threadIdx.x & 15) == 0 ? s0 : x;
 }
 
 // The rounds are rolled loops (constants read from shared memory one round
@@ -421,28 +511,42 @@ template <class F, int ALPHA>
 __device__ __forceinline__ uint32_t half_permute_a(uint32_t x, const P2Params* p) {
   const int l = threadIdx.x & 15;
   const int rfh = (int)p->rounds_f_half, rp = (int)p->rounds_p;
-  const uint32_t alpha = p->alpha, dg = p->diag[l], js = p->j_scale;
-  const bool jone = p->j_is_one != 0;
+  const uint32_t alpha = p->alpha, dg = p->diag[l], js = p->j_scale, e = p->chain_e;
   x = half_ext_linear<F>(x);
-  uint32_t c = rfh > 0 ? p->ext_init[0][l] : p->int_rc[0];
+  uint32_t c = rfh > 0 ? p->ext_init[0][l] : 0u;
 #pragma unroll 1
   for (int r = 0; r < rfh; r++) {
-    const uint32_t c_next = r + 1 < rfh ? p->ext_init[r + 1][l] : p->int_rc[0];
+    const uint32_t c_next = r + 1 < rfh ? p->ext_init[r + 1][l] : 0u;
     x = half_ext_linear<F>(ark_sbox_a<F, ALPHA>(x, c, alpha));
     c = c_next;
   }
+  if (rp > 0) {
+    int32_t m[16];
+    const int4* row = reinterpret_cast<const int4*>(p->chain_m[l]);
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      const int4 v = row[g];
+      m[4 * g] = v.x, m[4 * g + 1] = v.y, m[4 * g + 2] = v.z, m[4 * g + 3] = v.w;
+    }
+    const uint32_t w = l ? p->chain_t[l - 1] : 0u;
+    const int run = (int)p->chain;
 #pragma unroll 1
-  for (int r = 0; r < rp; r++) {
-    const uint32_t c_next = r + 1 < rp ? p->int_rc[r + 1] : p->ext_term[0][l];
-    const uint32_t s0 = ark_sbox_a<F, ALPHA>(x, c, alpha);  // lane 0's is used
-    const uint32_t rest = half_sum16<F>(l == 0 ? 0u : x);   // lanes 1..15
-    const uint32_t dx = mmul<F>(dg, l == 0 ? s0 : x);
-    uint32_t sum = madd<F>(rest, __shfl_sync(kFullMask, s0, threadIdx.x & 16));
-    if (!jone) sum = mmul<F>(sum, js);
-    x = madd<F>(sum, dx);
-    c = c_next;
+    for (int r0 = 0; r0 < rp; r0 += run) {
+      const int n = rp - r0 < run ? rp - r0 : run;
+      uint32_t rc = p->int_rc[r0];
+      const auto step = [&](int r, uint32_t s0) {
+        const uint32_t cur = rc;
+        rc = p->int_rc[r0 + r + 1 < rp ? r0 + r + 1 : 0];
+        return ark_sbox_a<F, ALPHA>(s0, cur, alpha);
+      };
+      switch (p->chain_mode) {
+        case 2: x = half_partials<F, 2, false>(x, n, dg, js, e, w, m, step); break;
+        case 1: x = half_partials<F, 1, false>(x, n, dg, js, e, w, m, step); break;
+        default: x = half_partials<F, 0, false>(x, n, dg, js, e, w, m, step); break;
+      }
+    }
   }
-  if (rp == 0) c = p->ext_term[0][l];
+  c = rfh > 0 ? p->ext_term[0][l] : 0u;
 #pragma unroll 1
   for (int r = 0; r < rfh; r++) {
     const uint32_t c_next = p->ext_term[r + 1 < rfh ? r + 1 : r][l];
@@ -543,37 +647,57 @@ __device__ __forceinline__ void p2_permute_quarter(uint32_t (&x)[4], const P2Par
   }
 }
 
-// The built-in BabyBear-16 instance on a half-warp, for permutations that run
-// alone (the transcript's one-warp chains): the same rounds as half_permute_a,
-// unrolled, with this lane's external-round constants and diagonal entry
-// passed in registers (ei, et, dg: loaded once per kernel) and the
-// partial-round constants read as constant-bank operands, so no round loads
-// a constant or runs loop control.
+// The built-in BabyBear-16 instance on a half-warp: the same rounds as
+// half_permute_a, unrolled, this lane's constants in registers (loaded once per
+// kernel where permutations follow one another) and the partial-round
+// constants read as constant-bank operands, so no round loads a constant or
+// runs loop control.
 static_assert(ZC_BB16_ROUNDS_F_HALF == 4, "built-in instance: 4 + 4 full rounds");
-__device__ __forceinline__ uint32_t half_permute_bb16(uint32_t x, const uint32_t (&ei)[4],
-                                                      const uint32_t (&et)[4], uint32_t dg) {
-  using F = BabyBear;
-  const int l = threadIdx.x & 15;
-  x = half_ext_linear<F>(x);
+static_assert(ZC_BB16_ROUNDS_P <= kChainMax, "built-in instance: one run of partial rounds");
+struct HalfBb16 {
+  uint32_t ei[4], et[4], dg, w;
+  int32_t m[16];
+  // p: the instance's parameters, in shared or global memory
+  __device__ __forceinline__ explicit HalfBb16(const P2Params* p) {
+    const int l = threadIdx.x & 15;
 #pragma unroll
-  for (int r = 0; r < 4; r++) x = half_ext_linear<F>(ark_sbox_a<F, 7>(x, ei[r], 7));
+    for (int r = 0; r < 4; r++) {
+      ei[r] = p->ext_init[r][l];
+      et[r] = p->ext_term[r][l];
+    }
+    dg = p->diag[l];
+    w = l ? p->chain_t[l - 1] : 0u;
+    const int4* row = reinterpret_cast<const int4*>(p->chain_m[l]);
 #pragma unroll
-  for (int r = 0; r < ZC_BB16_ROUNDS_P; r++) {
-    const uint32_t s0 = ark_sbox_a<F, 7>(x, c_bb16_int_rc[r], 7);  // lane 0's is used
-    const uint32_t rest = half_sum16<F>(l == 0 ? 0u : x);           // lanes 1..15
-    const uint32_t dx = mmul<F>(dg, l == 0 ? s0 : x);
-    x = madd<F>(madd<F>(rest, __shfl_sync(kFullMask, s0, threadIdx.x & 16)), dx);
+    for (int g = 0; g < 4; g++) {
+      const int4 v = row[g];
+      m[4 * g] = v.x, m[4 * g + 1] = v.y, m[4 * g + 2] = v.z, m[4 * g + 3] = v.w;
+    }
   }
+  __device__ __forceinline__ uint32_t permute(uint32_t x) const {
+    using F = BabyBear;
+    x = half_ext_linear<F>(x);
 #pragma unroll
-  for (int r = 0; r < 4; r++) x = half_ext_linear<F>(ark_sbox_a<F, 7>(x, et[r], 7));
-  return x;
-}
+    for (int r = 0; r < 4; r++) x = half_ext_linear<F>(ark_sbox_a<F, 7>(x, ei[r], 7));
+    x = half_partials<F, 2, true>(x, ZC_BB16_ROUNDS_P, dg, 0u, 0u, w, m, [](int r, uint32_t s0) {
+      return ark_sbox_a<F, 7>(s0, c_bb16_int_rc[r], 7);
+    });
+#pragma unroll
+    for (int r = 0; r < 4; r++) x = half_ext_linear<F>(ark_sbox_a<F, 7>(x, et[r], 7));
+    return x;
+  }
+};
 
-// Stage run-time params into shared memory (whole block participates).
+// Stage run-time params into shared memory (whole block participates): the
+// words [FROM, TO) of the block, by default what one thread's permutation
+// reads (kP2ThreadWords); the half-warp tables follow.
+constexpr int kP2Words = (int)(sizeof(P2Params) / 4);
+constexpr int kP2ThreadWords = (int)(offsetof(P2Params, chain) / 4);
+template <int FROM = 0, int TO = kP2Words>
 __device__ __forceinline__ void stage_params(P2Params* dst, const P2Params* src) {
   const uint32_t* s = reinterpret_cast<const uint32_t*>(src);
   uint32_t* d = reinterpret_cast<uint32_t*>(dst);
-  for (int i = threadIdx.x; i < (int)(sizeof(P2Params) / 4); i += blockDim.x) d[i] = s[i];
+  for (int i = FROM + threadIdx.x; i < TO; i += blockDim.x) d[i] = s[i];
   __syncthreads();
 }
 

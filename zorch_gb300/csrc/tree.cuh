@@ -39,16 +39,14 @@ struct RootHop {
 template <class F>
 __device__ __noinline__ void root_hop(const RootHop hop, const uint32_t* root, const P2Params* hp) {
   const HalfPerm<F> perm{hp};
-  Duplex t;
-  memcpy(&t, hop.state, sizeof(Duplex));
-  duplex_observe(t, root, 8, perm);
+  LaneDuplex t;
+  t.load(hop.state);
+  t.observe(root, 8, perm);
   for (int i = 0; i < hop.n; i++) {
-    uint32_t w;
-    duplex_sample(t, 1, &w, perm);
+    const uint32_t w = t.sample(perm);
     if (threadIdx.x == 0) hop.chal[i] = w;
   }
-  __syncwarp();
-  if (threadIdx.x == 0) memcpy(hop.state, &t, sizeof(Duplex));
+  t.store(hop.state);
 }
 
 // Leaf p = concat over q < G of base[q*gs + p*g .. +g] (zc_leaves).
@@ -275,22 +273,14 @@ template <class F>
 __device__ __forceinline__ uint32_t half_perm(uint32_t x, const P2Params* hp) {
   return p2_permute_half<F>(x, hp);
 }
-// The same for the provider K: the built-in instance runs unrolled
-// (half_permute_bb16), its lane constants read from the staged copy.
+// The same for the provider K: the built-in instance runs unrolled, its lane
+// constants read from the staged copy.
 template <class K>
 __device__ __forceinline__ uint32_t half_perm_k(uint32_t x, const P2Params* hp) {
-  if constexpr (std::is_same<K, Bb16Builtin>::value) {
-    const int l = threadIdx.x & 15;
-    uint32_t ei[4], et[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      ei[r] = hp->ext_init[r][l];
-      et[r] = hp->ext_term[r][l];
-    }
-    return half_permute_bb16(x, ei, et, hp->diag[l]);
-  } else {
+  if constexpr (std::is_same<K, Bb16Builtin>::value)
+    return HalfBb16(hp).permute(x);
+  else
     return p2_permute_half<typename K::F>(x, hp);
-  }
 }
 
 // One level of a subtree: parent i (< width) = compress(children 2i, 2i+1)
@@ -376,12 +366,7 @@ __global__ void __launch_bounds__(1024) k_subtree(Leaf leaf, uint32_t* layers, i
   }
   if (hop.state) {  // passed only to a one-CTA launch that ends at the root
     __syncthreads();
-    if (threadIdx.x < 32) {
-      uint32_t root[8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) root[i] = sm[cur][i];
-      root_hop<F>(hop, root, hp);
-    }
+    if (threadIdx.x < 32) root_hop<F>(hop, sm[cur], hp);
   }
 }
 

@@ -57,7 +57,7 @@ zc_status ensure_init() {
 template <class K, class Fn>
 __device__ __forceinline__ void with_half_perm(const P2Params* rt, P2Params* s_rt, Fn&& fn) {
   if constexpr (std::is_same<K, Bb16Builtin>::value) {
-    const HalfPermBb16 perm;
+    const HalfPermBb16 perm(rt);
     fn(perm);
   } else {
     KIn<K>::make(rt, s_rt);
@@ -66,28 +66,26 @@ __device__ __forceinline__ void with_half_perm(const P2Params* rt, P2Params* s_r
   }
 }
 
-// One warp; lane 0 writes the results.
+// One warp; lane 0 writes the challenges.
 template <class K>
 __global__ void __launch_bounds__(32) k_duplex_step(const P2Params* rt, uint32_t* state,
                                                     const uint32_t* values, int64_t m, int n,
                                                     uint32_t* out, int32_t* positions,
                                                     int64_t block_len) {
   __shared__ P2Params s_rt;
+  LaneDuplex t;
+  t.load(state);
   with_half_perm<K>(rt, &s_rt, [&](const auto& perm) {
-    Duplex t;
-    memcpy(&t, state, sizeof(Duplex));
-    duplex_observe(t, values, m, perm);
+    t.observe(values, m, perm);
     for (int i = 0; i < n; i++) {
-      uint32_t w;
-      duplex_sample(t, 1, &w, perm);
+      const uint32_t w = t.sample(perm);
       if (threadIdx.x == 0) {
         if (out) out[i] = w;
         if (positions) positions[i] = (int32_t)(w % (uint32_t)block_len);
       }
     }
-    __syncwarp();
-    if (threadIdx.x == 0) memcpy(state, &t, sizeof(Duplex));
   });
+  t.store(state);
 }
 
 template <class K>
@@ -97,32 +95,16 @@ __global__ void __launch_bounds__(32) k_duplex_hop(
     uint32_t* in_buf_o, uint32_t* out_buf_o, uint32_t* sponge_o, uint32_t* in_pos_o,
     uint32_t* out_pos_o, uint32_t* chal) {
   __shared__ P2Params s_rt;
+  LaneDuplex t;
+  t.load(in_buf, out_buf, sponge, in_pos, out_pos);
   with_half_perm<K>(rt, &s_rt, [&](const auto& perm) {
-    Duplex t;
-    for (int j = 0; j < 8; j++) {
-      t.in_buf[j] = in_buf[j];
-      t.out_buf[j] = out_buf[j];
-    }
-    for (int j = 0; j < 16; j++) t.sponge[j] = sponge[j];
-    t.in_pos = (int32_t)in_pos[0];
-    t.out_pos = (int32_t)out_pos[0];
-    duplex_observe(t, values, m, perm);
+    t.observe(values, m, perm);
     for (int i = 0; i < n; i++) {
-      uint32_t w;
-      duplex_sample(t, 1, &w, perm);
+      const uint32_t w = t.sample(perm);
       if (threadIdx.x == 0) chal[i] = w;
     }
-    // inputs may alias outputs: every lane has read them by now
-    __syncwarp();
-    if (threadIdx.x != 0) return;
-    for (int j = 0; j < 8; j++) {
-      in_buf_o[j] = t.in_buf[j];
-      out_buf_o[j] = t.out_buf[j];
-    }
-    for (int j = 0; j < 16; j++) sponge_o[j] = t.sponge[j];
-    in_pos_o[0] = (uint32_t)t.in_pos;
-    out_pos_o[0] = (uint32_t)t.out_pos;
   });
+  t.store(in_buf_o, out_buf_o, sponge_o, in_pos_o, out_pos_o);
 }
 
 template <class F>
@@ -295,6 +277,7 @@ zc_status zc_poseidon2_builtin(zc_field field, const zc_poseidon2** out) {
     memcpy(h->host.diag, dg, sizeof(dg));
     h->host.j_scale = BabyBear::ONE;
     h->host.j_is_one = 1;
+    p2_chain_tables<BabyBear>(&h->host);
     zc_status s = upload_params(h);
     if (s != ZC_OK) {
       delete h;
@@ -336,6 +319,10 @@ zc_status zc_poseidon2_create(zc_field field, int alpha, int rounds_f_half, int 
   for (int i = 0; i < 16; i++) h->host.diag[i] = conv(diag[i]);
   h->host.j_scale = conv(j_scale);
   h->host.j_is_one = (j_scale == 1);
+  if (field == ZC_FIELD_BABYBEAR)
+    p2_chain_tables<BabyBear>(&h->host);
+  else
+    p2_chain_tables<KoalaBear>(&h->host);
   zc_status s = upload_params(h);
   if (s != ZC_OK) {
     delete h;
