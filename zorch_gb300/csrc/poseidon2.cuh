@@ -83,6 +83,9 @@ ZC_HD uint32_t ark_sbox_a(uint32_t x, uint32_t c, uint32_t alpha) {
     const int32_t a2 = smul<F>(a, a);
     return snorm<F>(smul<F>(smul<F>(a2, a), smul<F>(a2, a2)));
   }
+  if (alpha == 3) return ark_sbox_a<F, 3>(x, c, alpha);
+  if (alpha == 5) return ark_sbox_a<F, 5>(x, c, alpha);
+  if (alpha == 7) return ark_sbox_a<F, 7>(x, c, alpha);
   return mpow<F>(madd<F>(x, c), alpha);
 }
 
@@ -576,9 +579,13 @@ __device__ __forceinline__ uint32_t p2_permute_half(uint32_t x, const P2Params* 
 // word 0 itself and runs its S-box redundantly, so the round needs no
 // broadcast: the sum over words 1..15 (local, then two shuffle levels) runs
 // while the S-box does, and every lane derives the new word 0 from the sum.
-// Per permutation this is about 2.3x fewer thread instructions than the
-// half-warp form, at no longer a dependency chain; it is the form used where
-// many latency-bound permutations run side by side (tree tops, transcript).
+// The form for widths between the other two. Cycles of one SM by the number
+// of permutations it runs at once (built-in instance; the multiplier pipe binds
+// from 64 up, the dependency chain below):
+//   permutations      8      16      32      64     128
+//   half-warps     3,718   4,617   7,240  13,230
+//   quarter-warps          5,500   5,930   7,950  13,130
+//   threads                                       18,100
 // Every lane of the warp must make the call (full-warp shuffles).
 template <class F>
 __device__ __forceinline__ void quarter_ext_linear(uint32_t (&x)[4]) {
@@ -592,59 +599,88 @@ __device__ __forceinline__ void quarter_ext_linear(uint32_t (&x)[4]) {
   for (int k = 0; k < 4; k++) x[k] = madd<F>(x[k], s[k]);
 }
 
+// One full round; c: the round's sixteen constants (16-byte aligned).
 template <class F, int ALPHA>
+__device__ __forceinline__ void quarter_full_round(uint32_t (&x)[4], const uint32_t* c,
+                                                   uint32_t alpha) {
+  const uint4 v = *reinterpret_cast<const uint4*>(c + 4 * (threadIdx.x & 3));
+  x[0] = ark_sbox_a<F, ALPHA>(x[0], v.x, alpha);
+  x[1] = ark_sbox_a<F, ALPHA>(x[1], v.y, alpha);
+  x[2] = ark_sbox_a<F, ALPHA>(x[2], v.z, alpha);
+  x[3] = ark_sbox_a<F, ALPHA>(x[3], v.w, alpha);
+  quarter_ext_linear<F>(x);
+}
+
+// One partial round; w0: word 0, on every lane (lane 0's x[0] is not kept).
+// MODE as in half_partials (chain_mode).
+template <class F, int ALPHA, int MODE>
+__device__ __forceinline__ void quarter_partial_round(uint32_t (&x)[4], uint32_t& w0, uint32_t c,
+                                                      uint32_t alpha, const uint32_t (&dg)[4],
+                                                      uint32_t j, uint32_t d0) {
+  const uint32_t y = ark_sbox_a<F, ALPHA>(w0, c, alpha);
+  // words 1..15 of this round's input
+  uint32_t part = madd<F>(madd<F>((threadIdx.x & 3) ? x[0] : 0u, x[1]), madd<F>(x[2], x[3]));
+  part = madd<F>(part, __shfl_xor_sync(kFullMask, part, 1));
+  part = madd<F>(part, __shfl_xor_sync(kFullMask, part, 2));
+  uint32_t dx[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) dx[k] = snorm<F>(smul3<F>((int32_t)x[k], (int32_t)dg[k]));
+  uint32_t sum = madd<F>(part, y);
+  if (MODE != 2) sum = mmul<F>(sum, j);
+  // word 0: j (part + y) + d_0 y, j (part - y) for d_0 = -2 j
+  if (MODE == 2) w0 = msub<F>(part, y);
+  if (MODE == 1) w0 = mmul<F>(msub<F>(part, y), j);
+  if (MODE == 0) w0 = madd<F>(sum, mmul<F>(d0, y));
+#pragma unroll
+  for (int k = 0; k < 4; k++) x[k] = madd<F>(sum, dx[k]);
+}
+
+template <class F, int ALPHA, int MODE>
 __device__ __forceinline__ void quarter_permute_a(uint32_t (&x)[4], const P2Params* p) {
   const int q = threadIdx.x & 3;
   const int rfh = (int)p->rounds_f_half, rp = (int)p->rounds_p;
-  const uint32_t alpha = p->alpha, js = p->j_scale, d0 = p->diag[0];
-  const bool jone = p->j_is_one != 0;
-  uint32_t dg[4];
-#pragma unroll
-  for (int k = 0; k < 4; k++) dg[k] = p->diag[4 * q + k];
+  const uint32_t alpha = p->alpha;
+  const uint4 d = *reinterpret_cast<const uint4*>(p->diag + 4 * q);
+  const uint32_t dg[4] = {d.x, d.y, d.z, d.w};
   quarter_ext_linear<F>(x);
 #pragma unroll 1
-  for (int r = 0; r < rfh; r++) {
-#pragma unroll
-    for (int k = 0; k < 4; k++) x[k] = ark_sbox_a<F, ALPHA>(x[k], p->ext_init[r][4 * q + k], alpha);
-    quarter_ext_linear<F>(x);
-  }
-  // word 0 on every lane of the quarter
+  for (int r = 0; r < rfh; r++) quarter_full_round<F, ALPHA>(x, p->ext_init[r], alpha);
   uint32_t w0 = __shfl_sync(kFullMask, x[0], threadIdx.x & ~3);
 #pragma unroll 1
-  for (int r = 0; r < rp; r++) {
-    const uint32_t s0 = ark_sbox_a<F, ALPHA>(w0, p->int_rc[r], alpha);
-    // words 1..15 of this round's input (lane 0's x[0] is word 0: left out)
-    uint32_t part = madd<F>(madd<F>(q ? x[0] : 0u, x[1]), madd<F>(x[2], x[3]));
-    part = madd<F>(part, __shfl_xor_sync(kFullMask, part, 1));
-    part = madd<F>(part, __shfl_xor_sync(kFullMask, part, 2));
-    uint32_t dx[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) dx[k] = mmul<F>(dg[k], x[k]);
-    uint32_t sum = madd<F>(part, s0);
-    if (!jone) sum = mmul<F>(sum, js);
-#pragma unroll
-    for (int k = 0; k < 4; k++) x[k] = madd<F>(sum, dx[k]);
-    w0 = madd<F>(sum, mmul<F>(d0, s0));
-    if (q == 0) x[0] = w0;
-  }
+  for (int r = 0; r < rp; r++)
+    quarter_partial_round<F, ALPHA, MODE>(x, w0, p->int_rc[r], alpha, dg, p->j_scale, p->diag[0]);
+  if (q == 0) x[0] = w0;
 #pragma unroll 1
-  for (int r = 0; r < rfh; r++) {
-#pragma unroll
-    for (int k = 0; k < 4; k++) x[k] = ark_sbox_a<F, ALPHA>(x[k], p->ext_term[r][4 * q + k], alpha);
-    quarter_ext_linear<F>(x);
-  }
+  for (int r = 0; r < rfh; r++) quarter_full_round<F, ALPHA>(x, p->ext_term[r], alpha);
 }
 
 // Lane q (of the caller's quarter-warp) passes state words 4q .. 4q+3 and gets
 // them back permuted. `p` points to shared memory.
 template <class F>
 __device__ __forceinline__ void p2_permute_quarter(uint32_t (&x)[4], const P2Params* p) {
-  switch (p->alpha) {
-    case 3: quarter_permute_a<F, 3>(x, p); break;
-    case 5: quarter_permute_a<F, 5>(x, p); break;
-    case 7: quarter_permute_a<F, 7>(x, p); break;
-    default: quarter_permute_a<F, 0>(x, p); break;
-  }
+  if (p->alpha == 3 && p->chain_mode == 2) return quarter_permute_a<F, 3, 2>(x, p);
+  if (p->alpha == 3 && p->chain_mode == 1) return quarter_permute_a<F, 3, 1>(x, p);
+  if (p->alpha == 7 && p->chain_mode == 2) return quarter_permute_a<F, 7, 2>(x, p);
+  quarter_permute_a<F, 0, 0>(x, p);
+}
+
+// The built-in instance on a quarter-warp: the partial rounds unrolled, their
+// constants constant-bank operands (fully unrolled saves 7 % more of a lone
+// permutation and 2 % of 128, for 1.5x the code).
+__device__ __forceinline__ void quarter_permute_bb16(uint32_t (&x)[4], const P2Params* p) {
+  using F = BabyBear;
+  const uint4 d = *reinterpret_cast<const uint4*>(p->diag + 4 * (threadIdx.x & 3));
+  const uint32_t dg[4] = {d.x, d.y, d.z, d.w};
+  quarter_ext_linear<F>(x);
+#pragma unroll 1
+  for (int r = 0; r < ZC_BB16_ROUNDS_F_HALF; r++) quarter_full_round<F, 7>(x, p->ext_init[r], 7);
+  uint32_t w0 = __shfl_sync(kFullMask, x[0], threadIdx.x & ~3);
+#pragma unroll
+  for (int r = 0; r < ZC_BB16_ROUNDS_P; r++)
+    quarter_partial_round<F, 7, 2>(x, w0, c_bb16_int_rc[r], 7, dg, 0u, 0u);
+  if ((threadIdx.x & 3) == 0) x[0] = w0;
+#pragma unroll 1
+  for (int r = 0; r < ZC_BB16_ROUNDS_F_HALF; r++) quarter_full_round<F, 7>(x, p->ext_term[r], 7);
 }
 
 // The built-in BabyBear-16 instance on a half-warp: the same rounds as

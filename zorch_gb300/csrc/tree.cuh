@@ -79,6 +79,31 @@ struct LayoutLeaf {
 #pragma unroll
     for (int j = 0; j < 8; j++) d[j] = s[j];
   }
+  // The same on a quarter-warp (lane q holds state words 4q .. 4q+3): lanes 0
+  // and 1 end with the digest. Every lane of the warp makes the call; `on`: the
+  // quarter has a leaf.
+  template <class Perm>
+  __device__ __forceinline__ void quarter_digest(int64_t p, bool on, uint32_t (&x)[4],
+                                                 const Perm& perm) const {
+    const int q4 = 4 * (threadIdx.x & 3);
+    const int w = G * g;
+    const uint32_t* src = base + p * (int64_t)g;
+#pragma unroll
+    for (int k = 0; k < 4; k++) x[k] = 0;
+    for (int e = 0; e < w; e += 8) {
+      if (on && q4 < 8) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const int i = e + q4 + k;
+          if (i < w) {
+            const int gi = i / g;
+            x[k] = __ldg(src + (int64_t)gi * gs + (i - gi * g));
+          }
+        }
+      }
+      perm(x);
+    }
+  }
 };
 
 // Node p of level l0 from children 2p, 2p+1 of the stored level l0-1.
@@ -90,39 +115,6 @@ struct NodeLeaf {
     load_digest(in + 16 * p, a);
     load_digest(in + 16 * p + 8, b);
     p2_compress(a, b, d, k);
-  }
-};
-
-// Query-layer node y of a query-strided tree (StridedMerkleTree,
-// zorch/commit/strided_merkle.py:100-152): the binary tree, adjacent pairs in
-// coset order, over the sponge-hashed rows y, y + s, ..., y + (rpq-1) s -- what
-// the reference's strided levels compute for residue y. One thread folds the
-// coset with a binary-counter stack (row r merges while bit b of r is set).
-constexpr int kMaxStridedLog = 8;
-struct StridedLeaf {
-  LayoutLeaf rows;
-  int64_t s;
-  int log_rpq;
-  template <class K>
-  __device__ __forceinline__ void digest(int64_t p, uint32_t* d, const K& k) const {
-    uint32_t stack[kMaxStridedLog][8];
-    const int rpq = 1 << log_rpq;
-    uint32_t cur[8];
-    for (int r = 0; r < rpq; r++) {
-      rows.digest(p + (int64_t)r * s, cur, k);
-      int b = 0;
-      for (; (r >> b) & 1; b++) {
-        uint32_t out[8];
-        p2_compress(stack[b], cur, out, k);
-#pragma unroll
-        for (int i = 0; i < 8; i++) cur[i] = out[i];
-      }
-      if (b < kMaxStridedLog)
-#pragma unroll
-        for (int i = 0; i < 8; i++) stack[b][i] = cur[i];
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++) d[i] = cur[i];
   }
 };
 
@@ -224,6 +216,44 @@ struct FoldLeaf {
 #pragma unroll
     for (int j = 0; j < 8; j++) d[j] = s[j];
   }
+  // On a quarter-warp: lanes 0 and 1 fold one element each.
+  template <class Perm>
+  __device__ __forceinline__ void quarter_digest(int64_t p, bool on, uint32_t (&x)[4],
+                                                 const Perm& perm) const {
+    const int q = threadIdx.x & 3;
+#pragma unroll
+    for (int e = 0; e < 4; e++) x[e] = 0;
+    if (on && q < 2) {
+      const int64_t quarter = n >> 2, half = n >> 1;
+      uint32_t bt[4];
+#pragma unroll
+      for (int e = 0; e < LB; e++) bt[e] = __ldg(beta + e);
+      uint32_t o[4];
+      int64_t i;
+      if (BR) {
+        uint32_t xi = mmul<F>(inv2s, mpow<F>(winv, (uint64_t)brev64(2 * p, ilog2_dev(half))));
+        if (q) xi = mmul<F>(xi, w4inv);
+        i = 2 * p + q;
+        M::fold(f + 2 * i * LI, 1, 0, xi, bt, o);
+      } else {
+        uint32_t xi = mmul<F>(inv2s, mpow<F>(winv, (uint64_t)p));
+        if (q) xi = mmul<F>(xi, w4inv);
+        i = p + q * quarter;
+        M::fold(f, half, i, xi, bt, o);
+      }
+#pragma unroll
+      for (int e = 0; e < LO; e++) {
+        g[i * LO + e] = o[e];
+        x[e] = o[e];
+      }
+    }
+    if (LO == 1) {  // both elements are words of lane 0's block
+      const uint32_t second = __shfl_down_sync(kFullMask, x[0], 1);
+      if (q == 0) x[1] = second;
+      if (q == 1) x[0] = 0;
+    }
+    perm(x);
+  }
 };
 
 // Nodes per tree-top CTA of the batched commit (k_tree_top) at its first
@@ -283,31 +313,40 @@ __device__ __forceinline__ uint32_t half_perm_k(uint32_t x, const P2Params* hp) 
     return p2_permute_half<typename K::F>(x, hp);
 }
 
+// Quarter-warp permutation for the provider K.
+template <class K>
+__device__ __forceinline__ void quarter_perm_k(uint32_t (&x)[4], const P2Params* hp) {
+  if constexpr (std::is_same<K, Bb16Builtin>::value)
+    quarter_permute_bb16(x, hp);
+  else
+    p2_permute_quarter<typename K::F>(x, hp);
+}
+
+// Levels of at most this many parents run on half-warps, wider ones on
+// quarter-warps (the table at the quarters in poseidon2.cuh: 4,617 against 5,500
+// cycles for 16, 7,240 against 5,930 for 32).
+constexpr int kHalfMaxWidth = 16;
+
 // One level of a subtree: parent i (< width) = compress(children 2i, 2i+1)
 // read from the digest slots `src` ([node][8 words], 16-byte aligned),
-// written to the `dst` slots and to the tree's level at `lay`. A level with
-// more parents than the CTA has half-warps runs on quarter-warps (one round of
-// up to blockDim/4 parents; a quarter's permutation costs ~2.3x fewer thread
-// instructions, which is what counts when every warp is busy); a narrower
-// level runs on half-warps, whose permutation has the shorter dependency
-// chain (each lane issues a quarter of the instructions), which is what
-// counts when the level is a latency chain. Parents are taken round-robin by
-// quarter (half) g = g, g + Q, ...; a warp with no parent in a round skips it
-// (a warp-uniform branch: the shuffles need every lane of a running warp).
+// written to the `dst` slots and to the tree's level at `lay`. Wider levels run
+// on quarter-warps, Q = blockDim/4 parents a round; narrow ones on half-warps,
+// whose permutation has the shorter dependency chain. A warp with no parent in
+// a round skips it (a warp-uniform branch: the shuffles need every lane of a
+// running warp).
 template <class K>
 __device__ __forceinline__ void subtree_level(const uint32_t* src, uint32_t* dst, uint32_t* lay,
                                               int width, const P2Params* hp) {
-  using F = typename K::F;
   const int t = threadIdx.x;
-  if (width > (int)(blockDim.x >> 4)) {  // quarter-warps: lane q holds words 4q .. 4q+3
-    const int q = t & 3, Q = blockDim.x >> 2;
+  if (width > kHalfMaxWidth || width > (int)(blockDim.x >> 4)) {
+    const int q = t & 3, Q = blockDim.x >> 2;  // lane q holds words 4q .. 4q+3
     for (int r = 0; r < width; r += Q) {
       if (r + 8 * (t >> 5) >= width) continue;
       const int node = r + (t >> 2);
       const bool on = node < width;
       uint4 v = on ? reinterpret_cast<const uint4*>(src)[4 * node + q] : make_uint4(0, 0, 0, 0);
       uint32_t x[4] = {v.x, v.y, v.z, v.w};
-      p2_permute_quarter<F>(x, hp);
+      quarter_perm_k<K>(x, hp);
       if (on && q < 2) {
         const uint4 o = make_uint4(x[0], x[1], x[2], x[3]);
         reinterpret_cast<uint4*>(lay)[2 * node + q] = o;
@@ -329,10 +368,11 @@ __device__ __forceinline__ void subtree_level(const uint32_t* src, uint32_t* dst
 }
 
 // One subtree of T first-level nodes per CTA (blockDim = subtree_threads(T)):
-// the first level is T leaf digests (one thread each; for NodeLeaf, quarter-
-// or half-warps compressing stored children), then every level up to the
-// subtree root is compressed out of ping-pong shared-memory slots
-// (subtree_level), each level written to `layers`.
+// the first level is T leaf digests (a quarter-warp each: the chain of a
+// thread's permutation is 3x as long; for NodeLeaf, stored children
+// compressed), then every level up to the subtree root is compressed out of
+// ping-pong shared-memory slots (subtree_level), each level written to
+// `layers`.
 template <class K, class Leaf>
 __global__ void __launch_bounds__(1024) k_subtree(Leaf leaf, uint32_t* layers, int64_t L,
                                                        int l0, int T, const P2Params* rt,
@@ -340,7 +380,7 @@ __global__ void __launch_bounds__(1024) k_subtree(Leaf leaf, uint32_t* layers, i
   using F = typename K::F;
   __shared__ P2Params s_rt;
   __shared__ __align__(16) uint32_t sm[2][8 * kSubCap];  // [node][word] digest slots
-  K k = KIn<K>::make(rt, &s_rt);
+  KIn<K>::make(rt, &s_rt);
   const P2Params* hp = KIn<K>::half(rt, &s_rt);
   const int t = threadIdx.x;
   const int64_t base = (int64_t)blockIdx.x * T;
@@ -348,11 +388,19 @@ __global__ void __launch_bounds__(1024) k_subtree(Leaf leaf, uint32_t* layers, i
   if constexpr (std::is_same<Leaf, NodeLeaf>::value) {
     subtree_level<K>(leaf.in + 16 * base, sm[0], lay0, T, hp);
   } else {
-    if (t < T) {
-      uint32_t d[8];
-      leaf.digest(base + t, d, k);
-      store_digest(lay0 + 8 * t, d);
-      store_digest(sm[0] + 8 * t, d);
+    const int q = t & 3, Q = blockDim.x >> 2;
+    const auto perm = [&](uint32_t (&x)[4]) { quarter_perm_k<K>(x, hp); };
+    for (int r = 0; r < T; r += Q) {
+      if (r + 8 * (t >> 5) >= T) continue;  // warp-uniform
+      const int node = r + (t >> 2);
+      const bool on = node < T;
+      uint32_t x[4];
+      leaf.quarter_digest(base + node, on, x, perm);
+      if (on && q < 2) {
+        const uint4 o = make_uint4(x[0], x[1], x[2], x[3]);
+        reinterpret_cast<uint4*>(lay0)[2 * node + q] = o;
+        reinterpret_cast<uint4*>(sm[0])[2 * node + q] = o;
+      }
     }
   }
   int cur = 0, lvl = l0, width = T;
@@ -400,6 +448,50 @@ __global__ void __launch_bounds__(kLeafT, HashOcc<K>::v) k_leaf(Leaf leaf, uint3
   uint32_t d[8];
   leaf.digest(p, d, k);
   store_digest(out + 8 * p, d);
+}
+
+// The query layer of a query-strided tree (StridedMerkleTree,
+// zorch/commit/strided_merkle.py:100-152): node y is the root of the binary
+// tree, adjacent pairs in coset order, over the sponge-hashed rows y, y + s, ...,
+// y + (rpq-1) s -- what the reference's strided levels compute for residue y.
+// A CTA takes `np` nodes, one thread per row, then one per compression of each
+// level out of shared memory (row r of node y in slot r * np + y). Against one
+// thread folding a whole coset, rpq times the threads: 2^20 rows in cosets of
+// 16 are 2^16 threads of 31 permutations each, 3.4 warps where a
+// sub-partition needs ten, or 2^20 of one and 2^19, 2^18, ... of the others.
+constexpr int kMaxStridedLog = 8;
+constexpr int kStridedT = 256;
+template <class K>
+__global__ void __launch_bounds__(kStridedT, 4) k_strided(LayoutLeaf rows, int64_t s, int log_rpq,
+                                                         int np, uint32_t* out,
+                                                         const P2Params* rt) {
+  __shared__ P2Params s_rt;
+  __shared__ __align__(16) uint32_t sm[8 * kStridedT];
+  K k = KIn<K>::make(rt, &s_rt);
+  const int t = threadIdx.x;
+  const int64_t y0 = (int64_t)blockIdx.x * np;
+  int width = np << log_rpq;  // digests of the current level
+  const int r = t / np, y = t - r * np;
+  uint32_t d[8];
+  if (t < width) {
+    rows.digest(y0 + y + (int64_t)r * s, d, k);
+    if (log_rpq) store_digest(sm + 8 * t, d);
+  }
+  for (int l = 0; l < log_rpq; l++) {
+    __syncthreads();
+    width >>= 1;
+    uint32_t a[8], b[8];
+    if (t < width) {  // children (2r, y), (2r + 1, y)
+      load_digest(sm + 8 * (2 * r * np + y), a);
+      load_digest(sm + 8 * ((2 * r + 1) * np + y), b);
+    }
+    __syncthreads();  // read before anyone overwrites
+    if (t < width) {
+      p2_compress(a, b, d, k);
+      store_digest(sm + 8 * t, d);
+    }
+  }
+  if (t < width) store_digest(out + 8 * (y0 + t), d);
 }
 
 // Levels with more than tree_shape().levelwise_min nodes run one thread per

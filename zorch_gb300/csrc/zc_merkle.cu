@@ -326,11 +326,15 @@ zc_status zc_strided_merkle_commit(const zc_poseidon2* p, zc_leaves lv, int32_t 
   if ((int64_t)lv.groups * lv.group_len > (1 << 20)) return ZC_BAD_SHAPE;
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t s = lv.num_leaves / rows_per_query;
-  StridedLeaf leaf{LayoutLeaf{lv.base, lv.groups, lv.group_len, lv.group_stride}, s,
-                   ilog2(rows_per_query)};
-  return with_perm(p, [&](auto k, const P2Params* rt) {
+  const LayoutLeaf rows{lv.base, lv.groups, lv.group_len, lv.group_stride};
+  const int log_rpq = ilog2(rows_per_query);
+  const int np = (int)(s < (kStridedT >> log_rpq) ? s : kStridedT >> log_rpq);
+  return with_perm(p, [&](auto k, const P2Params* rt) -> zc_status {
     using K = decltype(k);
-    return commit_tree<K>(leaf, layers, s, rt, st);
+    const int threads = (np << log_rpq) < 32 ? 32 : np << log_rpq;
+    k_strided<K><<<(unsigned)(s / np), threads, 0, st>>>(rows, s, log_rpq, np, layers, rt);
+    ZC_TRY(launch_check());
+    return finish_tree<K>(layers, s, 0, rt, st);
   });
 }
 
