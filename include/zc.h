@@ -382,6 +382,57 @@ zc_status zc_sumcheck_fold(zc_field field, const uint32_t* mle, int64_t M, const
                            int32_t beta_limbs, const uint32_t* msg, uint32_t* mle_out,
                            const uint32_t* eq, uint32_t* eq_out, uint32_t* claim, void* stream);
 
+/* The commit-and-fold rounds of an open in one call, as FriProver's commit
+ * phase (zorch/pcs/fold.py:90-115), the Basefold open (zorch/pcs/basefold/
+ * prover.py:419-480) and the SP1 stacked open (zorch/pcs/jagged/open.py:237-330)
+ * run them: per round commit the layer's pair leaves, observe the sumcheck
+ * message (if any) and the root, squeeze beta, fold. No host synchronisation,
+ * no allocation. */
+typedef struct {
+  int32_t rounds;        /* >= 1 */
+  int32_t log_n;         /* layer 0 has 2^log_n points, log_n >= rounds */
+  int32_t ef_in;         /* layer 0 is EF4 */
+  int32_t beta_limbs;    /* 1 or 4 */
+  int32_t bit_reversed;
+  int32_t bind;          /* observe SP1's bound root (zc_smcs_bind_root) */
+  uint32_t generator;
+  int32_t first_committed; /* first_tree already holds layer 0's digests */
+  const uint32_t* shifts;  /* host, [rounds]: each level's coset shift, Montgomery, 0 = none */
+  const uint32_t* codeword;  /* layer 0 */
+  uint32_t* first_tree;    /* layer 0's digest layers */
+  uint32_t* layers;        /* layers 1 .. rounds-1, one after the other */
+  uint32_t* trees;         /* their digest layers, one after the other */
+  uint32_t* final_layer;   /* layer `rounds` */
+  uint32_t* state;         /* the 34-word duplex state, advanced in place */
+  uint32_t* betas;         /* [rounds][beta_limbs] */
+  uint32_t* roots;         /* [rounds][8], as observed */
+  uint32_t* raw_roots;     /* [rounds][8] before binding, or NULL */
+  /* the interleaved sumcheck over 2^rounds EF4 entries (mle == NULL: none) */
+  const uint32_t* mle;
+  const uint32_t* eq;      /* 2^(rounds-1) entries */
+  uint32_t* claim;         /* advanced in place */
+  const uint32_t* zinv;    /* [rounds] EF4: 1/z per coordinate */
+  uint32_t* msgs;          /* [rounds][8] */
+  void* workspace;         /* zc_fold_rounds_workspace_bytes, with mle only */
+  size_t workspace_bytes;
+} zc_fold_rounds_desc;
+
+size_t zc_fold_rounds_workspace_bytes(int32_t rounds);
+zc_status zc_fold_rounds(const zc_poseidon2* p, const zc_fold_rounds_desc* d, void* stream);
+
+/* zc_merkle_open_reduced of the same positions in several trees, one launch
+ * for up to 32 of them. */
+typedef struct {
+  zc_leaves leaves;
+  const uint32_t* layers;
+  uint32_t* rows;   /* [q][groups*group_len] */
+  uint32_t* paths;  /* [depth][q][8] */
+  int32_t shift;
+} zc_open_job;
+
+zc_status zc_open_layers(const zc_open_job* jobs, int32_t count, const int32_t* idx, int32_t q,
+                         void* stream);
+
 /* Staggered partial-Lagrange batching of a committed matrix's w base columns
  * (n words each) into one EF4 codeword [n, 4] (16-byte aligned): weights =
  * eq(., r) over nbv = ceil(log2 w) EF4 challenges (challenges: nbv x 4 words,

@@ -44,6 +44,23 @@ class MerkleJob(C.Structure):
                 ("count", C.c_int32), ("leaf_stride", C.c_int64), ("layer_stride", C.c_int64)]
 
 
+class FoldRoundsDesc(C.Structure):
+    _fields_ = [("rounds", C.c_int32), ("log_n", C.c_int32), ("ef_in", C.c_int32),
+                ("beta_limbs", C.c_int32), ("bit_reversed", C.c_int32), ("bind", C.c_int32),
+                ("generator", C.c_uint32), ("first_committed", C.c_int32),
+                ("shifts", C.c_void_p), ("codeword", C.c_void_p), ("first_tree", C.c_void_p),
+                ("layers", C.c_void_p), ("trees", C.c_void_p), ("final_layer", C.c_void_p),
+                ("state", C.c_void_p), ("betas", C.c_void_p), ("roots", C.c_void_p),
+                ("raw_roots", C.c_void_p), ("mle", C.c_void_p), ("eq", C.c_void_p),
+                ("claim", C.c_void_p), ("zinv", C.c_void_p), ("msgs", C.c_void_p),
+                ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t)]
+
+
+class OpenJob(C.Structure):
+    _fields_ = [("leaves", Leaves), ("layers", C.c_void_p), ("rows", C.c_void_p),
+                ("paths", C.c_void_p), ("shift", C.c_int32)]
+
+
 _lock = threading.Lock()
 _lib: C.CDLL | None = None
 
@@ -107,6 +124,9 @@ def _declare(lib: C.CDLL) -> None:
         "zc_rs_encode_batch_workspace_bytes": (sz, [vp, i32]),
         "zc_rs_encode_batch": (st, [st, vp, i32, u32, vp, sz, vp]),
         "zc_merkle_commit_batch": (st, [vp, vp, i32, vp, sz, vp]),
+        "zc_fold_rounds_workspace_bytes": (sz, [i32]),
+        "zc_fold_rounds": (st, [vp, C.POINTER(FoldRoundsDesc), vp]),
+        "zc_open_layers": (st, [C.POINTER(OpenJob), i32, vp, i32, vp]),
         "zc_eval_poly_workspace_bytes": (sz, [i64]),
         "zc_eval_poly": (st, [st, vp, i64, vp, i32, vp, vp, sz, vp]),
         "zc_deep_quotient": (st, [st, vp, i64, vp, i32, vp, u32, u32, i32, vp, vp]),

@@ -2,6 +2,8 @@
 // zorch/transcript.py:239-481) shared by the transcript kernels and the
 // tree-top kernels that run a round's transcript hop in the same launch.
 #pragma once
+#include <type_traits>
+
 #include "internal.cuh"
 
 namespace zc {
@@ -88,6 +90,21 @@ struct HalfPermBb16 {
   __device__ explicit HalfPermBb16(const P2Params* p) : h(p) {}
   __device__ uint32_t half(uint32_t x) const { return h.permute(x); }
 };
+
+// Calls fn(perm) with the transcript's half-warp permutation: the unrolled
+// built-in form for the built-in instance, the run-time form (constants
+// staged to shared memory) otherwise.
+template <class K, class Fn>
+__device__ __forceinline__ void with_half_perm(const P2Params* rt, P2Params* s_rt, Fn&& fn) {
+  if constexpr (std::is_same<K, Bb16Builtin>::value) {
+    const HalfPermBb16 perm(rt);
+    fn(perm);
+  } else {
+    KIn<K>::make(rt, s_rt);
+    const HalfPerm<typename K::F> perm{KIn<K>::half(rt, s_rt)};
+    fn(perm);
+  }
+}
 
 // The duplex on one warp: lane l of each half (both run the same) holds sponge
 // word l and, for l < 8, words l of the input and output buffers. The same

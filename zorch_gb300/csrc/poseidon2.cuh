@@ -560,9 +560,10 @@ __device__ __forceinline__ uint32_t half_permute_a(uint32_t x, const P2Params* p
 }
 
 // Lane l (of the caller's half-warp) passes state word l and gets word l of
-// the permuted state back. `p` points to shared memory.
+// the permuted state back. `p` points to shared memory. Not inlined: one copy
+// of its forms in a translation unit.
 template <class F>
-__device__ __forceinline__ uint32_t p2_permute_half(uint32_t x, const P2Params* p) {
+__device__ __noinline__ uint32_t p2_permute_half(uint32_t x, const P2Params* p) {
   switch (p->alpha) {
     case 3: return half_permute_a<F, 3>(x, p);
     case 5: return half_permute_a<F, 5>(x, p);

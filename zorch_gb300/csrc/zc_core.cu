@@ -51,21 +51,6 @@ zc_status ensure_init() {
   return ZC_OK;
 }
 
-// Calls fn(perm) with the transcript's half-warp permutation: the unrolled
-// built-in form for the built-in instance, the run-time form (constants
-// staged to shared memory) otherwise.
-template <class K, class Fn>
-__device__ __forceinline__ void with_half_perm(const P2Params* rt, P2Params* s_rt, Fn&& fn) {
-  if constexpr (std::is_same<K, Bb16Builtin>::value) {
-    const HalfPermBb16 perm(rt);
-    fn(perm);
-  } else {
-    KIn<K>::make(rt, s_rt);
-    const HalfPerm<typename K::F> perm{KIn<K>::half(rt, s_rt)};
-    fn(perm);
-  }
-}
-
 // One warp; lane 0 writes the challenges.
 template <class K>
 __global__ void __launch_bounds__(32) k_duplex_step(const P2Params* rt, uint32_t* state,

@@ -8,49 +8,11 @@
 // per-block partial sums whatever the order.
 #include <algorithm>
 
+#include "ef4.cuh"
 #include "internal.cuh"
+#include "rounds.cuh"
 
 namespace zc {
-
-__device__ __forceinline__ ef4 ld4(const uint32_t* p) {
-  const uint4 v = *reinterpret_cast<const uint4*>(p);
-  return ef4{{v.x, v.y, v.z, v.w}};
-}
-__device__ __forceinline__ void st4(uint32_t* p, const ef4& a) {
-  *reinterpret_cast<uint4*>(p) = make_uint4(a.c[0], a.c[1], a.c[2], a.c[3]);
-}
-template <class F>
-__device__ __forceinline__ ef4 ef_base(const ef4& a, uint32_t b) {  // EF4 * base
-  return ef_scale<F>(a, b);
-}
-
-// Block-wide EF4 sum (blockDim a multiple of 32, <= 1024); the result is
-// valid in thread 0.
-template <class F>
-__device__ ef4 block_sum(ef4 v) {
-  __shared__ uint32_t red[4][32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int e = 0; e < 4; e++) v.c[e] = madd<F>(v.c[e], __shfl_xor_sync(0xffffffffu, v.c[e], o));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();  // red reused across calls
-  if (lane == 0)
-#pragma unroll
-    for (int e = 0; e < 4; e++) red[e][warp] = v.c[e];
-  __syncthreads();
-  ef4 r{{0, 0, 0, 0}};
-  if (warp == 0) {
-    const int nw = blockDim.x >> 5;
-#pragma unroll
-    for (int e = 0; e < 4; e++) r.c[e] = lane < nw ? red[e][lane] : 0u;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int e = 0; e < 4; e++) r.c[e] = madd<F>(r.c[e], __shfl_xor_sync(0xffffffffu, r.c[e], o));
-  }
-  return r;
-}
 
 // expand_eq_to_hypercube(z, 1) for m <= kEqSmall variables on one block:
 // out[2i] = s - s z_j, out[2i+1] = s z_j per step (z[0] ends on the top bit).
@@ -231,6 +193,38 @@ __global__ void k_sc_fold(const uint32_t* mle, int64_t M, const uint32_t* beta, 
   }
 }
 
+// The fold of a round and the next round's s0 partials in one pass: thread k <
+// M/2 folds outputs 2k and 2k+1 and contracts eq entry k, which are the terms
+// eq'[k] mle'[2k] of the next message (k_sc_reduce's sum), so the folded table
+// is not read back and the round has one launch fewer.
+template <class F>
+__global__ void __launch_bounds__(256) k_sc_fold_reduce(const uint32_t* mle, int64_t M,
+                                                        const uint32_t* beta, int beta_limbs,
+                                                        const uint32_t* msg, uint32_t* mle_out,
+                                                        const uint32_t* eq, uint32_t* eq_out,
+                                                        uint32_t* claim, uint32_t* partial) {
+  ef4 b{{__ldg(beta), 0, 0, 0}};
+  if (beta_limbs == 4) b = ld4(beta);
+  const auto mul = [&](const ef4& x) { return beta_limbs == 4 ? ef_mul<F>(b, x) : ef_base<F>(x, b.c[0]); };
+  ef4 acc{{0, 0, 0, 0}};
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < M / 2;
+       k += (int64_t)gridDim.x * blockDim.x) {
+    const ef4 f0 = ef_add<F>(ld4(mle + 16 * k), mul(ld4(mle + 16 * k + 4)));
+    const ef4 f1 = ef_add<F>(ld4(mle + 16 * k + 8), mul(ld4(mle + 16 * k + 12)));
+    const ef4 e = ef_add<F>(ld4(eq + 8 * k), ld4(eq + 8 * k + 4));
+    st4(mle_out + 8 * k, f0);
+    st4(mle_out + 8 * k + 4, f1);
+    st4(eq_out + 4 * k, e);
+    acc = ef_add<F>(acc, ef_mul<F>(e, f0));
+  }
+  acc = block_sum<F>(acc);
+  if (threadIdx.x == 0) st4(partial + 4 * blockIdx.x, acc);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const ef4 s0 = ld4(msg), s1 = ld4(msg + 4);
+    st4(claim, ef_add<F>(s0, mul(s1)));
+  }
+}
+
 // Staggered batching with an offset into the weight table and accumulation
 // (batch_staggered, zorch/pcs/basefold/batching.py:66-80).
 template <class F>
@@ -297,6 +291,37 @@ __global__ void k_ef4_inv(const uint32_t* in, uint32_t* out, int64_t count) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
        i += (int64_t)gridDim.x * blockDim.x)
     st4(out + 4 * i, ef_inv<F>(ld4(in + 4 * i)));
+}
+
+// ------------------------------------------------- rounds.cuh's two steps --
+// One CTA of 256 per 256 items, at most four per SM (the partials are summed by
+// one warp, the round's hop).
+static int sc_blocks(int64_t items) {
+  const int64_t b = (items + 255) / 256;
+  return (int)(b < kRoundPartials ? b : kRoundPartials);
+}
+
+zc_status sc_first_partials(zc_field field, const uint32_t* mle, int64_t M, const uint32_t* eq,
+                            uint32_t* partial, int* np, cudaStream_t st) {
+  return with_field(field, [&](auto f) {
+    using F = decltype(f);
+    *np = sc_blocks(M);
+    k_sc_reduce<F><<<*np, 256, 0, st>>>(mle, eq, M, partial);
+    return launch_check();
+  });
+}
+
+zc_status sc_fold_partials(zc_field field, const uint32_t* mle, int64_t M, const uint32_t* beta,
+                           int beta_limbs, const uint32_t* msg, uint32_t* mle_out,
+                           const uint32_t* eq, uint32_t* eq_out, uint32_t* claim,
+                           uint32_t* partial, int* np, cudaStream_t st) {
+  return with_field(field, [&](auto f) {
+    using F = decltype(f);
+    *np = sc_blocks(M / 2);
+    k_sc_fold_reduce<F><<<*np, 256, 0, st>>>(mle, M, beta, beta_limbs, msg, mle_out, eq, eq_out,
+                                             claim, partial);
+    return launch_check();
+  });
 }
 
 }  // namespace zc

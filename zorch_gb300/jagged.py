@@ -26,6 +26,7 @@ from . import _lib
 from .coding import BitReversedReedSolomon
 from .commit import DigestLayers, SingleMatrixCommitmentScheme, leaves_layout
 from .field import from_mont, ptr, stream_handle, to_host
+from .pcs import layer_spec, open_layers, run_fold_rounds
 from .transcript import DuplexTranscript
 
 
@@ -244,46 +245,27 @@ def stacked_basefold_open(smcs: SingleMatrixCommitmentScheme, code: BitReversedR
     nb = L.zc_eq_expand_workspace_bytes(v - 1)
     ews = torch.empty(max((nb + 15) // 4, 4), dtype=torch.int32, device=dev)
     _lib.check(L.zc_eq_expand(f.id, ptr(zs), v - 1, ptr(eq), ptr(ews), nb, st), "eq_expand")
-    scb = L.zc_sumcheck_workspace_bytes()
-    scws = torch.empty(scb // 4, dtype=torch.int32, device=dev)
-    msgs = torch.empty((v, 8), dtype=torch.int32, device=dev)
-    fold = StackedFoldCommit(smcs, code)
-    layers: list[StackedFoldLayer] = []
-    pending = None
-    for i in range(v):
-        M = S >> (i + 1)
-        _lib.check(L.zc_sumcheck_message(f.id, ptr(mle), M, ptr(eq), ptr(claim),
-                                         ptr(zinv[v - 1 - i]), ptr(msgs[i]), ptr(scws), scb, st),
-                   "sumcheck_message")
-        layer = pending if pending is not None else fold.commit_layer(cw)
-        t.observe_(msgs[i])
-        beta = t.observe_and_sample_(layer.bound_root, 4)
-        cw_next, pending = fold.fold_commit(cw, beta, code.level_of(cw.shape[0]))
-        mle_next = torch.empty((M, 4), dtype=torch.int32, device=dev)
-        eq_next = torch.empty((M // 2, 4), dtype=torch.int32, device=dev) if M >= 2 else None
-        _lib.check(L.zc_sumcheck_fold(f.id, ptr(mle), M, ptr(beta), 4, ptr(msgs[i]),
-                                      ptr(mle_next), ptr(eq) if eq_next is not None else None,
-                                      ptr(eq_next) if eq_next is not None else None, ptr(claim),
-                                      st), "sumcheck_fold")
-        layers.append(layer)
-        mle, eq, cw = mle_next, eq_next, cw_next
+    fr = run_fold_rounds(smcs.perm, code, cw, v, 4, t, bind=True,
+                         sumcheck=(mle, eq, claim, zinv))
+    cw = fr.final_layer
     final_poly = cw[0].contiguous()
     t.observe_(final_poly)
     t, witness = t.grind(pow_bits)  # the query-phase proof of work (:304-307)
     witness = witness.reshape(1)
     t, positions = sample_query_positions(t, n, num_queries)
     positions = positions.to(torch.int32)
-    query_openings = fold.open_layers(layers, positions, check=False)  # masked below n
-    component_openings = []
+    # the rounds' matrices, then every fold layer at a_i = q >> (i+1)
+    # (BitReversedReedSolomon.layer_positions); positions are masked below n
+    specs = []
     for rd in rounds:
         K = rd.codeword.shape[0]
-        op = smcs._tree.open_layout(leaves_layout(rd.codeword, n, K, 1, n), rd.digest_layers,
-                                    positions, K, check=False)
-        component_openings.append((op.row, op.path))
+        specs.append((leaves_layout(rd.codeword, n, K, 1, n), rd.digest_layers, K, 0))
+    opened = [(op.row, op.path) for op in
+              open_layers(specs + [layer_spec(ly, i, True) for i, ly in enumerate(fr.layers)],
+                          positions)]
     proof = StackedOpenProof(
-        [rd.commitment for rd in rounds], torch.stack([ly.raw_root for ly in layers]),
-        torch.stack([ly.bound_root for ly in layers]), msgs.reshape(v, 2, 4), final_poly,
-        witness, batch_evals, component_openings, query_openings, positions)
+        [rd.commitment for rd in rounds], fr.raw_roots, fr.roots, fr.msgs.view(v, 2, 4),
+        final_poly, witness, batch_evals, opened[:len(specs)], opened[len(specs):], positions)
     return proof, t
 
 

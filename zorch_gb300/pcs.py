@@ -11,6 +11,7 @@ zorch/pcs/fold.py:42-52). A layer's pair leaves (zorch/coding/reed_solomon.py:
 
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass, field as dc_field
 from typing import Sequence
 
@@ -267,6 +268,104 @@ def open_layer(tree: MerkleTree, layer: CommittedLayer, positions: torch.Tensor,
 
 
 @dataclass
+class FoldRounds:
+    """What run_fold_rounds leaves: the committed layers, the observed and raw
+    roots [R, 8], the challenges [R, limbs], the final layer and, with a
+    sumcheck, its messages [R, 8]."""
+
+    layers: list[CommittedLayer]
+    roots: torch.Tensor
+    raw_roots: torch.Tensor | None
+    betas: torch.Tensor
+    final_layer: torch.Tensor
+    msgs: torch.Tensor | None = None
+
+
+def run_fold_rounds(perm, code, codeword: torch.Tensor, rounds: int, limbs: int,
+                    t: DuplexTranscript, first_layer: CommittedLayer | None = None,
+                    bind: bool = False, sumcheck: tuple | None = None) -> FoldRounds:
+    """`rounds` (1 .. log2 n) rounds of commit pair leaves -> observe -> sample
+    beta -> fold from `codeword`, as PreFoldPairCommitRound runs them
+    (zorch/pcs/fold.py:90-115), launched by one call (zc_fold_rounds). `t`
+    advances in place. `bind` observes SP1's bound roots; `sumcheck` = (mle
+    [2^rounds, 4], eq, claim, zinv) interleaves the sumcheck of the Basefold
+    opens, advancing `claim`."""
+    dev = codeword.device
+    n = codeword.shape[0]
+    log_n = n.bit_length() - 1
+    ef = codeword.dim() == 2
+    lo = 4 if (ef or limbs == 4) else 1
+    L = _lib.lib()
+    words = lambda k: torch.empty(k, dtype=torch.int32, device=dev)  # noqa: E731
+    lens = [n >> i for i in range(1, rounds)]
+    leaves = [n >> (i + 1) for i in range(1, rounds)]
+    if first_layer is None:
+        first_layer = CommittedLayer(codeword, DigestLayers(words((n - 1, 8)), n // 2))
+        committed = 0
+    else:
+        committed = 1
+    cws = words((sum(lens) * lo,))
+    trees = words((sum(2 * m - 1 for m in leaves), 8))
+    final = words((n >> rounds, 4) if lo == 4 else (n >> rounds,))
+    roots, betas = words((rounds, 8)), words((rounds, limbs))
+    raw = words((rounds, 8)) if bind else None
+    # the fused folds count levels from the codeword, the last one is code.fold
+    shifts = (ctypes.c_uint32 * rounds)(
+        *[code.level_shift_mont(i) for i in range(rounds - 1)],
+        code.level_shift_mont(code.level_of(n >> (rounds - 1))))
+    d = _lib.FoldRoundsDesc(
+        rounds, log_n, int(ef), limbs, int(code.bit_reversed), int(bind),
+        code.generator or 0, committed, ctypes.addressof(shifts), ptr(codeword),
+        ptr(first_layer.digest_layers.flat), ptr(cws), ptr(trees), ptr(final), ptr(t.state),
+        ptr(betas), ptr(roots), ptr(raw))
+    msgs = ws = None
+    if sumcheck is not None:
+        mle, eq, claim, zinv = sumcheck
+        msgs = words((rounds, 8))
+        nb = L.zc_fold_rounds_workspace_bytes(rounds)
+        ws = words(((nb + 3) // 4,))
+        d.mle, d.eq, d.claim, d.zinv, d.msgs = (ptr(mle), ptr(eq), ptr(claim), ptr(zinv),
+                                                ptr(msgs))
+        d.workspace, d.workspace_bytes = ptr(ws), nb
+    _lib.check(L.zc_fold_rounds(perm.handle, ctypes.byref(d), stream_handle()), "fold_rounds")
+    layers = [first_layer]
+    if rounds > 1:
+        cw_parts = cws.split_with_sizes([k * lo for k in lens])
+        tree_parts = trees.split_with_sizes([2 * m - 1 for m in leaves])
+        layers += [CommittedLayer(c.view(-1, 4) if lo == 4 else c, DigestLayers(tr, m))
+                   for c, tr, m in zip(cw_parts, tree_parts, leaves)]
+    return FoldRounds(layers, roots, raw, betas, final, msgs)
+
+
+def open_layers(specs: Sequence[tuple], positions: torch.Tensor) -> list[Opening]:
+    """Openings of the same positions in several trees, one launch
+    (zc_open_layers): specs are (leaf layout, digest layers, leaf width, shift),
+    each opened at leaf (position >> shift) mod num_leaves."""
+    idx = positions.to(torch.int32).contiguous()
+    q = idx.numel()
+    sizes = []
+    for lv, dl, width, _ in specs:
+        sizes += [q * width, dl.depth * q * 8]
+    parts = torch.empty(sum(sizes), dtype=torch.int32, device=idx.device).split_with_sizes(sizes)
+    jobs = (_lib.OpenJob * len(specs))()
+    out = []
+    for i, (lv, dl, width, shift) in enumerate(specs):
+        row, path = parts[2 * i], parts[2 * i + 1]
+        jobs[i] = _lib.OpenJob(lv, ptr(dl.flat), row.data_ptr(), path.data_ptr(), shift)
+        out.append(Opening(row.view(q, width), path.view(dl.depth, q, 8)))
+    _lib.check(_lib.lib().zc_open_layers(jobs, len(specs), ptr(idx), q, stream_handle()),
+               "open_layers")
+    return out
+
+
+def layer_spec(layer: CommittedLayer, level: int, bit_reversed: bool) -> tuple:
+    """open_layers' spec of fold layer `level`'s pair leaves at its layer
+    positions (see open_layer)."""
+    return (pair_layout(layer.codeword, bit_reversed), layer.digest_layers, 2 * layer.limbs,
+            level + 1 if bit_reversed else 0)
+
+
+@dataclass
 class CommitPhaseProof:
     """Commit-phase proof: per-round roots, the cleartext final layer, the
     query positions and each layer's opened pair leaf with its path."""
@@ -339,27 +438,37 @@ class FriProver:
         """Fold rounds down to block_len >> num_rounds, observe the final layer,
         sample the query positions and open every layer (the commit/query phase
         of _open_one, zorch/pcs/fri/prover.py:151-187, on `codeword` itself)."""
-        p = self.params
-        # fuse_hop stays off: on the 2^22, 15-round commit phase replayed from
-        # a CUDA graph the separate hop launch measured 0.05 ms faster per
-        # proof (6.26 vs 6.31 ms) than the hop inside the root launch
-        rnd = PreFoldPairCommitRound(p.code, p.tree, p.challenge_limbs,
-                                     last_round=p.num_rounds - 1)
-        state = FoldState(codeword, (), first_layer)
         t = transcript._copy()
-        roots = []
-        for _ in range(p.num_rounds):
-            state, t, root = rnd(state, t)
-            roots.append(root)
-        final = state.codeword
-        n0 = codeword.shape[0]
-        positions = t.sample_positions_(n0, p.num_queries, values=final)
-        br = p.code.bit_reversed
-        openings = [open_layer(p.tree, layer, positions, i, br)
-                    for i, layer in enumerate(state.layers)]
-        roots_t = stack_rows(roots, (8,), codeword.device)
-        return CommitPhaseProof(roots_t, list(state.betas), final, positions, openings), t, state
+        phase, state, _ = self._rounds_and_openings(codeword, t, first_layer)
+        return phase, t, state
 
+    def _rounds_and_openings(self, codeword: torch.Tensor, t: DuplexTranscript,
+                             first_layer: CommittedLayer | None = None,
+                             extra: Sequence[tuple] = ()):
+        """commit_phase on `t` in place; `extra` trees (open_layers' specs) are
+        opened at the same positions in the same launch. Returns (proof, fold
+        state, extra openings)."""
+        p = self.params
+        n0 = codeword.shape[0]
+        br = p.code.bit_reversed
+        if 1 <= p.num_rounds <= n0.bit_length() - 1 and n0 & (n0 - 1) == 0:
+            fr = run_fold_rounds(p.tree.perm, p.code, codeword, p.num_rounds, p.challenge_limbs,
+                                 t, first_layer)
+            betas, roots = fr.betas.unbind(0), fr.roots
+            state = FoldState(fr.final_layer, tuple(fr.layers), None, betas)
+        else:  # no round, or more rounds than halvings (refused by the rounds)
+            rnd = PreFoldPairCommitRound(p.code, p.tree, p.challenge_limbs,
+                                         last_round=p.num_rounds - 1)
+            state, moved, msgs = fold_rounds(rnd, FoldState(codeword, (), first_layer), t,
+                                             p.num_rounds)
+            t.state = moved.state
+            betas, roots = state.betas, stack_rows(msgs, (8,), codeword.device)
+        final = state.codeword
+        positions = t.sample_positions_(n0, p.num_queries, values=final)
+        specs = [layer_spec(layer, i, br) for i, layer in enumerate(state.layers)]
+        ops = open_layers([*specs, *extra], positions) if specs or extra else []
+        proof = CommitPhaseProof(roots, list(betas), final, positions, ops[:len(specs)])
+        return proof, state, ops[len(specs):]
 
     # -- the open: ProverStage.prove (zorch/pcs/fri/prover.py:101-187) --------
     def prove(self, claim: OpeningClaim, witness: OpeningWitness,
@@ -413,11 +522,9 @@ class FriProver:
                                       int(code.bit_reversed), ptr(q), st), "deep_quotient")
         t = t._copy()
         t.observe_(committed.root)
-        phase, t, _ = self.commit_phase(q, t)
         br = code.bit_reversed
-        f_open = tree.open_layout_reduced(pair_layout(committed.codeword, br),
-                                          committed.digest_layers, phase.positions, 2,
-                                          1 if br else 0)
+        f_spec = (pair_layout(committed.codeword, br), committed.digest_layers, 2, 1 if br else 0)
+        phase, _, (f_open,) = self._rounds_and_openings(q, t, None, [f_spec])
         proof = FriProof(v.reshape(()) if zl == 1 else v, phase.roots, phase.final_layer,
                          f_open, phase.openings, phase.positions)
         return proof, t
@@ -769,38 +876,17 @@ class BasefoldProver:
         nb = L.zc_eq_expand_workspace_bytes(v - 1)
         ews = torch.empty(max((nb + 15) // 4, 4), dtype=torch.int32, device=dev)
         _lib.check(L.zc_eq_expand(f.id, ptr(zc), v - 1, ptr(eq), ptr(ews), nb, st), "eq_expand")
-        scb = L.zc_sumcheck_workspace_bytes()
-        scws = torch.empty(scb // 4, dtype=torch.int32, device=dev)
-        msgs = torch.empty((v, 8), dtype=torch.int32, device=dev)
-        rnd = PreFoldPairCommitRound(code, tree, 1)
-        layers: list[CommittedLayer] = []
-        pending = None
-        for i in range(v):
-            M = S >> (i + 1)
-            _lib.check(L.zc_sumcheck_message(f.id, ptr(mle), M, ptr(eq), ptr(claim),
-                                             ptr(zinv[v - 1 - i]), ptr(msgs[i]), ptr(scws), scb,
-                                             st), "sumcheck_message")
-            t.observe_(msgs[i])
-            layer = pending if pending is not None else rnd.commit_layer(cw)
-            beta = t.observe_and_sample_(layer.root, 1)
-            if i < v - 1 and cw.shape[0] >= 4:
-                cw_next, pending = rnd.fold_commit(cw, beta, i)
-            else:
-                cw_next, pending = code.fold(cw, beta), None
-            mle_next = torch.empty((M, 4), dtype=torch.int32, device=dev)
-            eq_next = torch.empty((M // 2, 4), dtype=torch.int32, device=dev) if M >= 2 else None
-            _lib.check(L.zc_sumcheck_fold(f.id, ptr(mle), M, ptr(beta), 1, ptr(msgs[i]),
-                                          ptr(mle_next), ptr(eq) if eq_next is not None else None,
-                                          ptr(eq_next) if eq_next is not None else None,
-                                          ptr(claim), st), "sumcheck_fold")
-            layers.append(layer)
-            mle, eq, cw = mle_next, eq_next, cw_next
-        final = cw
+        fr = run_fold_rounds(tree.perm, code, cw, v, 1, t, sumcheck=(mle, eq, claim, zinv))
+        final = fr.final_layer
         positions = t.sample_positions_(n, self.num_queries, values=final)
-        comp = [self.open_rows(pd, positions, check=False) for pd in rounds]
-        queries = [open_layer(tree, layer, positions) for layer in layers]
-        proof = BasefoldProof(msgs, torch.stack([ly.root for ly in layers]), final, comp,
-                              queries, positions)
+        specs = []
+        for pd in rounds:
+            K, nc = pd.codeword.shape
+            specs.append((leaves_layout(pd.codeword, nc, K, 1, nc), pd.digest_layers, K, 0))
+        ops = open_layers(specs + [layer_spec(ly, i, code.bit_reversed)
+                                   for i, ly in enumerate(fr.layers)], positions)
+        proof = BasefoldProof(fr.msgs, fr.roots, final, ops[:len(specs)], ops[len(specs):],
+                              positions)
         return values, proof, t
 
     def commit(self, polys: Sequence[torch.Tensor]):
