@@ -46,6 +46,18 @@ def _instance(orc, name):
                 orc.Poseidon2.koalabear16_golden())
     if name == "sp1":
         return koalabear16_params(orc.load_sp1_fixture()), orc.sp1_koalabear16()
+    if name[0] in ("plonky3", "sp1"):  # the two diagonals with other rounds and scales
+        _, rp, j = name
+        p, rng = KOALABEAR.p, np.random.default_rng(rp)
+        h = lambda k: pow(2, -k, p)  # noqa: E731
+        d = ([-2, 1, 2, h(1), 3, 4, -h(1), -3, -4, h(8), h(3), h(24), -h(8), -h(3), -h(4), -h(24)]
+             if name[0] == "plonky3" else [-2] + [1 << i for i in range(14)] + [1 << 15])
+        ei, et = (rng.integers(0, p, size=(4, 16), dtype=np.uint64).astype(np.uint32)
+                  for _ in range(2))
+        ir = rng.integers(0, p, size=rp, dtype=np.uint64).astype(np.uint32)
+        dg = np.asarray([x * j % p for x in d], np.uint32)
+        return (Poseidon2.from_params(1, 3, ei, et, ir, dg, j),
+                orc.Poseidon2.from_canonical(1, 3, ei, et, ir, dg, j))
     field, alpha, rfh, rp, j = name
     return _random_instance(orc, field, alpha, rfh, rp, j, 7 * rp + alpha)
 
@@ -55,7 +67,9 @@ INSTANCES = ["bb16", "kb16", "sp1",
              (0, 7, 4, 13, 1), (0, 7, 4, 13, 5), (0, 5, 3, 1, 1), (0, 3, 1, 2, 2013265920),
              (0, 11, 4, 14, 1), (1, 3, 4, 20, 1), (1, 3, 4, 20, 1057030144), (1, 3, 4, 12, 2),
              (1, 5, 8, 15, 1), (1, 7, 2, 16, 3), (1, 3, 4, 17, 1), (0, 7, 4, 26, 1),
-             (1, 3, 1, 64, 9), (0, 7, 8, 29, 1)]
+             (1, 3, 1, 64, 9), (0, 7, 8, 29, 1),
+             *[("plonky3", rp, j) for rp, j in [(1, 1), (2, 1), (3, 1), (20, 1), (33, 1), (20, 7)]],
+             *[("sp1", rp, j) for rp, j in [(1, 5), (2, 1), (21, 1057030144), (64, 2130706432)]]]
 IDS = [i if isinstance(i, str) else "-".join(map(str, i)) for i in INSTANCES]
 
 

@@ -21,19 +21,23 @@ struct KIn<Bb16Builtin> {
   __device__ static Bb16Builtin make(const P2Params*, P2Params*) { return {}; }
   // The half-warp permutation reads P2Params from shared memory: stage them.
   __device__ static const P2Params* half(const P2Params* g, P2Params* s) {
-    stage_params(s, g);
+    stage_words<0, kP2Sp1At>(s, g);
+    __syncthreads();
     return s;
   }
 };
 template <class F>
 struct KIn<RtParams<F>> {
   __device__ static RtParams<F> make(const P2Params* g, P2Params* s) {
-    stage_params<0, kP2ThreadWords>(s, g);
+    stage_words<0, kP2ChainAt>(s, g);
+    if (g->kind == kP2Sp1Kb) stage_words<kP2Sp1At, kP2Words>(s, g);
+    __syncthreads();
     return RtParams<F>{s};
   }
   // make has staged the front of the same shared copy.
   __device__ static const P2Params* half(const P2Params* g, P2Params* s) {
-    stage_params<kP2ThreadWords, kP2Words>(s, g);
+    stage_words<kP2ChainAt, kP2Sp1At>(s, g);
+    __syncthreads();
     return s;
   }
 };

@@ -31,6 +31,12 @@ struct P2Params {
   uint32_t diag[16];
   uint32_t j_scale;
   uint32_t j_is_one;
+  // diag and j_scale as int32 of least magnitude (RtParams' partial rounds).
+  int32_t j_c;
+  // Partial rounds of their own (KoalaBear, x^3): kP2Plonky3Kb for Plonky3's
+  // diagonal with j = 1, kP2Sp1Kb for SP1's with any j; 0: none.
+  int32_t kind;
+  alignas(16) int32_t diag_c[16];
   // Derived tables of the half-warp partial rounds (half_partials), for runs of
   // up to `chain` rounds: chain_m[k][i] = j d_i^k as an int32 of least
   // magnitude (0 for word 0), chain_t[k] = j sum_{i>=1} d_i^k, chain_e = j + d_0,
@@ -40,12 +46,68 @@ struct P2Params {
   uint32_t chain_e;
   uint32_t chain_t[16];
   alignas(16) int32_t chain_m[16][20];  // rows of 16, padded to spread 16-byte reads over the banks
+  // kP2Sp1Kb: round r's constant times mu^-r and its S-box's factor mu^2r, and
+  // mu^rounds_p, mu = 2^24 j (kb_sp1_partials).
+  uint32_t sp1_rc[64];
+  uint32_t sp1_mul[64];
+  uint32_t sp1_out;
 };
 constexpr int kChainMax = 16;
 
-// Fills the derived tables from diag, j_scale and rounds_p.
+// The representative of least magnitude of a word in [0, p).
+template <class F>
+ZC_HD int32_t centred(uint32_t x) {
+  return x > F::P / 2 ? (int32_t)(x - F::P) : (int32_t)x;
+}
+
+constexpr int kP2Plonky3Kb = 1, kP2Sp1Kb = 2;
+
+// Which of the two KoalaBear-16 internal diagonals (over j) this is:
+// [-2, 1, 2, 1/2, 3, 4, -1/2, -3, -4, 2^-8, 2^-3, 2^-24, -2^-8, -2^-3, -2^-4,
+// -2^-24] (Plonky3) or [-2, 1, 2, 4, 8, ..., 2^13, 2^15] (SP1).
+template <class F>
+inline int p2_kind(const P2Params* p) {
+  if (F::ID != KoalaBear::ID || p->alpha != 3) return 0;
+  const auto mul = [&](uint32_t c) { return mmul<F>(p->j_scale, c); };
+  const auto inv2k = [&](int k) { return mpow<F>(F::INV2, (uint64_t)k); };
+  uint32_t plonky3[16], sp1[16];
+  const uint32_t three = madd<F>(F::TWO, F::ONE), four = madd<F>(F::TWO, F::TWO);
+  const uint32_t d[16] = {mneg<F>(F::TWO), F::ONE,         F::TWO,          F::INV2,
+                          three,           four,           mneg<F>(F::INV2), mneg<F>(three),
+                          mneg<F>(four),   inv2k(8),       inv2k(3),        inv2k(24),
+                          mneg<F>(inv2k(8)), mneg<F>(inv2k(3)), mneg<F>(inv2k(4)),
+                          mneg<F>(inv2k(24))};
+  for (int i = 0; i < 16; i++) {
+    plonky3[i] = d[i];
+    sp1[i] = i == 0 ? d[0] : mpow<F>(F::TWO, (uint64_t)(i == 15 ? 15 : i - 1));
+  }
+  int kind = kP2Plonky3Kb;
+  for (int i = 0; i < 16; i++)
+    if (p->j_scale != F::ONE || p->diag[i] != plonky3[i]) kind = 0;
+  if (kind) return kind;
+  kind = kP2Sp1Kb;
+  for (int i = 0; i < 16; i++)
+    if (p->j_scale == 0 || p->diag[i] != mul(sp1[i])) kind = 0;
+  return kind;
+}
+
+// Fills the derived constants from diag, j_scale and rounds_p.
 template <class F>
 inline void p2_chain_tables(P2Params* p) {
+  p->j_c = centred<F>(p->j_scale);
+  for (int i = 0; i < 16; i++) p->diag_c[i] = centred<F>(p->diag[i]);
+  p->kind = p2_kind<F>(p);
+  if (p->kind == kP2Sp1Kb) {
+    const uint32_t mu = mmul<F>(p->j_scale, mpow<F>(F::TWO, 24)), mu_inv = minv<F>(mu);
+    uint32_t up = F::ONE, down = F::ONE;
+    for (uint32_t r = 0; r < p->rounds_p; r++) {
+      p->sp1_rc[r] = mmul<F>(p->int_rc[r], down);
+      p->sp1_mul[r] = mmul<F>(up, up);
+      up = mmul<F>(up, mu);
+      down = mmul<F>(down, mu_inv);
+    }
+    p->sp1_out = up;
+  }
   const uint32_t runs = (p->rounds_p + kChainMax - 1) / kChainMax;
   p->chain = runs ? (p->rounds_p + runs - 1) / runs : 0;
   p->chain_e = madd<F>(p->j_scale, p->diag[0]);
@@ -57,8 +119,7 @@ inline void p2_chain_tables(P2Params* p) {
     for (int i = 0; i < 20; i++) p->chain_m[k][i] = 0;
     for (int i = 1; i < 16; i++) {
       t = madd<F>(t, pw[i]);
-      const uint32_t m = mmul<F>(p->j_scale, pw[i]);
-      p->chain_m[k][i] = m > F::P / 2 ? (int32_t)(m - F::P) : (int32_t)m;
+      p->chain_m[k][i] = centred<F>(mmul<F>(p->j_scale, pw[i]));
       pw[i] = mmul<F>(pw[i], p->diag[i]);
     }
     p->chain_t[k] = mmul<F>(p->j_scale, t);
@@ -122,6 +183,13 @@ __device__ __forceinline__ int32_t smul3(int32_t a, int32_t b) {
   return (int32_t)((uint32_t)(c >> 32) - (uint32_t)mp + c_zero);
 }
 
+// Montgomery reduction of c, |c| <= p^2, into (-p, p).
+template <class F>
+__device__ __forceinline__ int32_t sredc(int64_t c) {
+  const uint32_t m = (uint32_t)c * F::MU;
+  return (int32_t)(c >> 32) - __mulhi((int32_t)m, (int32_t)F::P);
+}
+
 // The built-in BabyBear-16 instance (x^7, 4 + 4 full and 13 partial rounds),
 // one state per thread.
 //
@@ -141,9 +209,14 @@ __device__ __forceinline__ int32_t smul3(int32_t a, int32_t b) {
 //    low k bits of x, x 2^-k = (x >> k) - q * 15 * 2^(27-k), in (-p, p).
 // 87 instructions per partial round, 5,190 per permutation (5,880 before):
 // 1.654 against 1.911 ms for 2^20 threads x 8 permutations at the same clock.
-struct Bb {
-  using F = BabyBear;
+// Products by small constants and powers of two in a field p = A 2^T + 1 with
+// 2^31 = p + 2^T - 1 (BabyBear: 15, 27; KoalaBear: 127, 24).
+template <class F>
+struct Pow2 {
   static constexpr uint32_t P = F::P;
+  static constexpr int T = F::TWO_ADICITY;
+  static constexpr uint32_t A = (P - 1) >> T;
+  static_assert((A << T) + 1 == P && P + (1u << T) - 1 == 0x80000000u, "p = A 2^T + 1");
   __device__ __forceinline__ static uint32_t add(uint32_t a, uint32_t b) { return madd<F>(a, b); }
   __device__ __forceinline__ static uint32_t dbl(uint32_t x) { return madd<F>(x, x); }
   __device__ __forceinline__ static uint32_t half(uint32_t x) {
@@ -152,8 +225,8 @@ struct Bb {
   // x 2^-K in (-p, p / 2^K] for x in [0, p).
   template <int K>
   __device__ __forceinline__ static int32_t shr(uint32_t x) {
-    static_assert(K >= 1 && K <= 27, "k out of range");
-    return (int32_t)((x >> K) - (x & ((1u << K) - 1u)) * (15u << (27 - K)));
+    static_assert(K >= 1 && K <= T, "k out of range");
+    return (int32_t)((x >> K) - (x & ((1u << K) - 1u)) * (A << (T - K)));
   }
   template <int K>
   __device__ __forceinline__ static uint32_t div2exp(uint32_t x) {
@@ -161,23 +234,33 @@ struct Bb {
   }
   // sum + x 2^-K in [0, p): the sum of the three terms lies in (-p, p + p/2^K],
   // so one correction from below and one from above (an instruction less than
-  // normalising x 2^-K first).
+  // normalising x 2^-K first). The first takes its largest value plus p in 32
+  // bits: K >= 3 for BabyBear, 6 for KoalaBear.
   template <int K>
   __device__ __forceinline__ static uint32_t add_div2exp(uint32_t sum, uint32_t x) {
-    static_assert(K >= 1 && K <= 27, "k out of range");
+    static_assert(K <= T && 2 * (uint64_t)P + (P >> K) < (1ull << 32), "k out of range");
     const uint32_t r =
-        snorm<F>((int32_t)((sum + (x >> K)) - (x & ((1u << K) - 1u)) * (15u << (27 - K))));
+        snorm<F>((int32_t)((sum + (x >> K)) - (x & ((1u << K) - 1u)) * (A << (T - K))));
     const uint32_t t = r - P;
     return t < r ? t : r;
   }
-  // 2^K x: the bits above 2^31 come back as 2^31 = 2^27 - 1 (mod p); below 2p
+  // 2^K x: the bits above 2^31 come back as 2^31 = 2^T - 1 (mod p); below 2p
   // for x in [0, p) and K <= 4.
   template <int K>
   __device__ __forceinline__ static uint32_t mul2exp(uint32_t x) {
     static_assert(K >= 1 && K <= 4, "k out of range");
-    const uint32_t r = ((x << K) & 0x7fffffffu) + (x >> (31 - K)) * ((1u << 27) - 1u);
+    const uint32_t r = ((x << K) & 0x7fffffffu) + (x >> (31 - K)) * ((1u << T) - 1u);
     const uint32_t t = r - P;
     return t < r ? t : r;
+  }
+  // The pair of d = 2^-T, carried as h and g = 2^-T h_{r-1} in (-p, 2^(31-T)):
+  // h' = sum + 2^-T g, g' = 2^-T h. g > -p, so its shift is in [-A, 0] and the
+  // sum of the terms in (-p, p): one correction.
+  __device__ __forceinline__ static void lowest_pair(uint32_t sum, uint32_t& h, uint32_t& g) {
+    const uint32_t hn = snorm<F>((int32_t)((sum + (uint32_t)((int32_t)g >> T)) -
+                                           (g & ((1u << T) - 1u)) * A));
+    g = (uint32_t)shr<T>(h);
+    h = hn;
   }
 };
 
@@ -200,7 +283,7 @@ struct Bb16Builtin {
   template <bool FIRST>
   __device__ __forceinline__ static void partial_round(uint32_t* s, uint32_t (&h)[5],
                                                        uint32_t (&hp)[5], uint32_t c) {
-    using B = Bb;
+    using B = Pow2<F>;
     const uint32_t y = sbox(s[0], c - F::P);
     const uint32_t H = B::add(B::add(B::add(h[0], h[1]), B::add(h[2], h[3])), h[4]);
     const uint32_t part = B::add(B::add(B::add(s[1], s[2]), B::add(s[10], s[11])),
@@ -226,17 +309,11 @@ struct Bb16Builtin {
       hp[1] = B::add(B::add(sum, hp[1]), B::mul2exp<3>(hp[1]));
       hp[2] = B::add(sum, B::mul2exp<4>(hp[2]));
       hp[3] = B::add_div2exp<16>(sum, hp[3]);
-      // d = 2^-27: h' = sum + d g, g' = d h. For g in (-p, 16) the shift is in
-      // [-15, 0], so the sum of the terms is in (-p, p): one correction.
-      const int32_t g = (int32_t)hp[4];
-      const uint32_t hn =
-          snorm<F>((int32_t)((sum + (uint32_t)(g >> 27)) - (hp[4] & 0x7ffffffu) * 15u));
-      hp[4] = (uint32_t)B::shr<27>(h[4]);
-      h[4] = hn;
+      B::lowest_pair(sum, h[4], hp[4]);
     }
   }
   __device__ __forceinline__ static void partial_rounds(uint32_t* s) {
-    using B = Bb;
+    using B = Pow2<F>;
     constexpr int ia[5] = {3, 4, 5, 9, 12}, ib[5] = {6, 7, 8, 13, 15};
     uint32_t h[5], hp[5];
 #pragma unroll
@@ -279,7 +356,11 @@ struct Bb16Builtin {
 template <class F_>
 struct RtParams {
   using F = F_;
+#ifdef __CUDA_ARCH__
+  static constexpr bool kOwnPermute = true;
+#else
   static constexpr bool kOwnPermute = false;
+#endif
   const P2Params* p;  // shared memory on the device, plain memory on the host
   ZC_HD int rf_half() const { return (int)p->rounds_f_half; }
   ZC_HD int rp() const { return (int)p->rounds_p; }
@@ -306,6 +387,8 @@ struct RtParams {
 #pragma unroll
     for (int i = 0; i < 16; i++) s[i] = madd<F>(sum, mmul<F>(dg(i), s[i]));
   }
+  // One thread's permutation on the device (below).
+  __device__ __forceinline__ void permute(uint32_t* s) const;
 };
 
 // M4 = circ(2, 3, 1, 1) on one 4-word block.
@@ -365,6 +448,219 @@ __device__ __forceinline__ void Bb16Builtin::permute(uint32_t* s) const {
   partial_rounds(s);
 #pragma unroll 1
   for (int r = 0; r < ZC_BB16_ROUNDS_F_HALF; r++) full_round(s, c_bb16_term_lp.v + 16 * r);
+}
+
+// A run-time instance, one state per thread, constants from shared memory (rows of
+// four words a load). The exponent is chosen once a permutation. A partial
+// round's word is d_i s_i + j sum as one 64-bit value, j sum formed once, and
+// one reduction: with d_i and j of least magnitude |d_i s_i + j sum| <= p^2,
+// which sredc takes. 18 pipe cycles a word where a product, its correction and
+// a modular addition take 24.
+template <class F, int ALPHA>
+__device__ __forceinline__ uint32_t rt_sbox(uint32_t x, uint32_t c, uint32_t alpha) {
+  const int32_t a = (int32_t)(x + c - F::P);
+  if (ALPHA == 3) return snorm<F>(smul3<F>(smul3<F>(a, a), a));
+  if (ALPHA == 7) {
+    const int32_t a2 = smul3<F>(a, a);
+    return snorm<F>(smul3<F>(smul3<F>(a2, a), smul3<F>(a2, a2)));
+  }
+  return ark_sbox_a<F, 0>(x, c, alpha);
+}
+
+template <class F, int ALPHA>
+__device__ __forceinline__ void rt_full_round(uint32_t* s, const uint32_t* c, uint32_t alpha) {
+  uint32_t col[4];
+#pragma unroll
+  for (int b = 0; b < 16; b += 4) {
+    const uint4 v = *reinterpret_cast<const uint4*>(c + b);
+    uint32_t x[4] = {rt_sbox<F, ALPHA>(s[b], v.x, alpha), rt_sbox<F, ALPHA>(s[b + 1], v.y, alpha),
+                     rt_sbox<F, ALPHA>(s[b + 2], v.z, alpha),
+                     rt_sbox<F, ALPHA>(s[b + 3], v.w, alpha)};
+    m4_block<F>(x);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      s[b + k] = x[k];
+      col[k] = b ? madd<F>(col[k], x[k]) : x[k];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 16; i++) s[i] = madd<F>(s[i], col[i & 3]);
+}
+
+// Partial rounds of the KoalaBear-16 instance of Plonky3: its diagonal holds six
+// pairs (d, -d), at words (3, 6), (4, 7), (5, 8), (9, 12), (10, 13), (11, 15),
+// carried as sums and differences as the built-in BabyBear instance carries its
+// five. 70 instructions a round, against 16 products of the general form.
+template <bool FIRST>
+__device__ __forceinline__ void kb_plonky3_round(uint32_t* s, uint32_t (&h)[6], uint32_t (&hp)[6],
+                                                 uint32_t c) {
+  using F = KoalaBear;
+  using B = Pow2<F>;
+  const uint32_t y = rt_sbox<F, 3>(s[0], c, 3);
+  const uint32_t H = B::add(B::add(B::add(h[0], h[1]), B::add(h[2], h[3])), B::add(h[4], h[5]));
+  const uint32_t part = B::add(B::add(s[1], s[2]), B::add(s[14], B::dbl(H)));
+  const uint32_t sum = B::add(part, y);
+  s[0] = msub<F>(part, y);  // sum - 2 y
+  s[1] = B::add(sum, s[1]);
+  s[2] = B::add(sum, B::dbl(s[2]));
+  s[14] = msub<F>(sum, B::div2exp<4>(s[14]));
+  if (FIRST) {  // hp = a - b: times d / 2
+    hp[0] = B::add(sum, B::div2exp<2>(hp[0]));
+    hp[1] = B::add(B::add(sum, hp[1]), B::half(hp[1]));
+    hp[2] = B::add(sum, B::dbl(hp[2]));
+    hp[3] = B::add_div2exp<9>(sum, hp[3]);
+    hp[4] = B::add(sum, B::div2exp<4>(hp[4]));
+    const uint32_t hn = B::add_div2exp<24>(sum, B::half(hp[5]));
+    hp[5] = (uint32_t)B::shr<24>(h[5]);
+    h[5] = hn;
+  } else {  // hp = h_{r-1}: times d^2
+    hp[0] = B::add(sum, B::div2exp<2>(hp[0]));
+    hp[1] = B::add(B::add(sum, hp[1]), B::mul2exp<3>(hp[1]));
+    hp[2] = B::add(sum, B::mul2exp<4>(hp[2]));
+    hp[3] = B::add_div2exp<16>(sum, hp[3]);
+    hp[4] = B::add_div2exp<6>(sum, hp[4]);
+    B::lowest_pair(sum, h[5], hp[5]);
+  }
+}
+
+__device__ __forceinline__ void kb_plonky3_partials(uint32_t* s, const P2Params* p) {
+  using F = KoalaBear;
+  using B = Pow2<F>;
+  constexpr int ia[6] = {3, 4, 5, 9, 10, 11}, ib[6] = {6, 7, 8, 12, 13, 15};
+  const int rp = (int)p->rounds_p;
+  if (rp == 0) return;
+  uint32_t h[6], hp[6];
+#pragma unroll
+  for (int i = 0; i < 6; i++) {
+    h[i] = B::half(B::add(s[ia[i]], s[ib[i]]));
+    hp[i] = msub<F>(s[ia[i]], s[ib[i]]);
+  }
+  kb_plonky3_round<true>(s, h, hp, p->int_rc[0]);
+  // hp = h_{r+1} and h = h_r of the first five pairs after a round: they change
+  // places, two rounds a turn
+  int r = 1;
+#pragma unroll 1
+  for (; r + 1 < rp; r += 2) {
+    uint32_t cur[6] = {hp[0], hp[1], hp[2], hp[3], hp[4], h[5]};
+    uint32_t old[6] = {h[0], h[1], h[2], h[3], h[4], hp[5]};
+    kb_plonky3_round<false>(s, cur, old, p->int_rc[r]);
+    uint32_t cur2[6] = {old[0], old[1], old[2], old[3], old[4], cur[5]};
+    uint32_t old2[6] = {cur[0], cur[1], cur[2], cur[3], cur[4], old[5]};
+    kb_plonky3_round<false>(s, cur2, old2, p->int_rc[r + 1]);
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+      h[i] = cur2[i];
+      hp[i] = old2[i];
+    }
+    h[5] = cur2[5];
+    hp[5] = old2[5];
+  }
+  if (r < rp) {
+    uint32_t cur[6] = {hp[0], hp[1], hp[2], hp[3], hp[4], h[5]};
+    uint32_t old[6] = {h[0], h[1], h[2], h[3], h[4], hp[5]};
+    kb_plonky3_round<false>(s, cur, old, p->int_rc[r]);
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+      h[i] = cur[i];
+      hp[i] = old[i];
+    }
+    h[5] = cur[5];
+    hp[5] = old[5];
+  }
+  const uint32_t g[6] = {B::half(h[0]),       B::add(B::dbl(h[1]), h[1]), B::dbl(B::dbl(h[2])),
+                         B::div2exp<8>(h[3]), B::div2exp<3>(h[4]),        snorm<F>((int32_t)hp[5])};
+  const uint32_t hh[6] = {hp[0], hp[1], hp[2], hp[3], hp[4], h[5]};
+#pragma unroll
+  for (int i = 0; i < 6; i++) {
+    s[ia[i]] = B::add(hh[i], g[i]);
+    s[ib[i]] = msub<F>(hh[i], g[i]);
+  }
+}
+
+// Partial rounds of SP1's KoalaBear-16 instance, s_i' = j (sum + 2^k_i s_i) with
+// k = 0, 1, 2, ..., 13, 15 (and -2 for word 0). With t = s / mu^r, mu = 2^24 j,
+// they are t_i' = 2^-24 (sum + 2^k_i t_i): every factor 2^(k_i - 24) is a shift
+// and one low product. Word 0's S-box takes (t_0 mu^r + c)^3 = mu^3r (t_0 +
+// c mu^-r)^3, so a round costs one product more (mu^2r), and the sixteen words
+// are scaled by mu^rounds_p at the end.
+// Words may exceed p here: t_i' = sum + 2^-e t_i, e = 24 - k_i >= 9, is corrected
+// from below only and stays below p + (p + p/512) 2^-e. The excesses of the
+// fifteen words sum to less than 0.003 p, so every partial sum of two stays
+// below 2.004 p < 2^32 = 2.015 p, and the sum itself is reduced below p (its
+// factor 2^-24) before it is used: the bounds hold from round to round.
+template <int I>
+__device__ __forceinline__ void kb_sp1_words(uint32_t* s, uint32_t sum) {
+  if constexpr (I < 16) {
+    using F = KoalaBear;
+    constexpr int e = 24 - (I == 15 ? 15 : I - 1);
+    s[I] = snorm<F>((int32_t)((sum + (s[I] >> e)) - (s[I] & ((1u << e) - 1u)) * (127u << (24 - e))));
+    kb_sp1_words<I + 1>(s, sum);
+  }
+}
+
+__device__ __forceinline__ void kb_sp1_partials(uint32_t* s, const P2Params* p) {
+  using F = KoalaBear;
+  using B = Pow2<F>;
+  const int rp = (int)p->rounds_p;
+#pragma unroll 1
+  for (int r = 0; r < rp; r++) {
+    const int32_t a = (int32_t)(s[0] + p->sp1_rc[r] - F::P);
+    const uint32_t y =
+        snorm<F>(smul3<F>(smul3<F>(smul3<F>(a, a), a), (int32_t)p->sp1_mul[r]));
+    uint32_t q[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      q[k] = B::add(k ? B::add(s[4 * k], s[4 * k + 1]) : s[1], B::add(s[4 * k + 2], s[4 * k + 3]));
+    const uint32_t part = B::add(B::add(q[0], q[1]), B::add(q[2], q[3]));
+    const uint32_t sum = B::div2exp<24>(B::add(part, y));
+    s[0] = B::div2exp<24>(msub<F>(part, y));  // 2^-24 (sum - 2 y)
+    kb_sp1_words<1>(s, sum);
+  }
+  const int32_t out = (int32_t)p->sp1_out;
+#pragma unroll
+  for (int i = 0; i < 16; i++) s[i] = snorm<F>(smul3<F>((int32_t)s[i], out));
+}
+
+template <class F, int ALPHA>
+__device__ __forceinline__ void rt_permute_a(uint32_t* s, const P2Params* p) {
+  const int rfh = (int)p->rounds_f_half, rp = (int)p->rounds_p;
+  const uint32_t alpha = p->alpha;
+  p2_ext_linear<F>(s);
+#pragma unroll 1
+  for (int r = 0; r < rfh; r++) rt_full_round<F, ALPHA>(s, p->ext_init[r], alpha);
+  const int kind = F::ID == KoalaBear::ID && ALPHA == 3 ? p->kind : 0;
+  if (kind == kP2Plonky3Kb) kb_plonky3_partials(s, p);
+  if (kind == kP2Sp1Kb) kb_sp1_partials(s, p);
+#pragma unroll 1
+  for (int r = 0; r < (kind ? 0 : rp); r++) {
+    s[0] = rt_sbox<F, ALPHA>(s[0], p->int_rc[r], alpha);
+    uint32_t a[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      a[k] = madd<F>(madd<F>(s[4 * k], s[4 * k + 1]), madd<F>(s[4 * k + 2], s[4 * k + 3]));
+    const uint32_t sum = madd<F>(madd<F>(a[0], a[1]), madd<F>(a[2], a[3]));
+    const int64_t js = (int64_t)p->j_c * (int32_t)sum;
+#pragma unroll
+    for (int b = 0; b < 16; b += 4) {
+      const int4 d = *reinterpret_cast<const int4*>(p->diag_c + b);
+      s[b] = snorm<F>(sredc<F>(js + (int64_t)d.x * (int32_t)s[b]));
+      s[b + 1] = snorm<F>(sredc<F>(js + (int64_t)d.y * (int32_t)s[b + 1]));
+      s[b + 2] = snorm<F>(sredc<F>(js + (int64_t)d.z * (int32_t)s[b + 2]));
+      s[b + 3] = snorm<F>(sredc<F>(js + (int64_t)d.w * (int32_t)s[b + 3]));
+    }
+  }
+#pragma unroll 1
+  for (int r = 0; r < rfh; r++) rt_full_round<F, ALPHA>(s, p->ext_term[r], alpha);
+}
+
+template <class F>
+__device__ __forceinline__ void RtParams<F>::permute(uint32_t* s) const {
+  if (p->alpha == 3)
+    rt_permute_a<F, 3>(s, p);
+  else if (p->alpha == 7)
+    rt_permute_a<F, 7>(s, p);
+  else
+    rt_permute_a<F, 0>(s, p);
 }
 
 #pragma nv_exec_check_disable
@@ -446,13 +742,6 @@ __device__ __forceinline__ uint32_t half_ext_linear(uint32_t x) {
   return madd<F>(madd<F>(y2, d), madd<F>(e, f));
 }
 
-// Montgomery reduction of c, |c| <= p^2, into (-p, p).
-template <class F>
-__device__ __forceinline__ int32_t sredc(int64_t c) {
-  const uint32_t m = (uint32_t)c * F::MU;
-  return (int32_t)(c >> 32) - __mulhi((int32_t)m, (int32_t)F::P);
-}
-
 // n <= 16 partial rounds. Words 1..15 evolve linearly given the rounds' sums, so
 // with s_i the words at the start, y_r round r's S-box output and
 //   B_r = j * (sum of words 1..15 before round r)
@@ -473,7 +762,7 @@ __device__ __forceinline__ uint32_t half_partials(uint32_t x, int n, uint32_t dg
                                                   uint32_t e, uint32_t w, const int32_t (&m)[16],
                                                   const Step& step) {
   const int base = threadIdx.x & 16;
-  const int32_t xc = (int32_t)(x > F::P / 2 ? x - F::P : x);  // |xc| <= p/2
+  const int32_t xc = centred<F>(x);  // |xc| <= p/2
   int32_t part[4];
 #pragma unroll
   for (int g = 0; g < 4; g++) {
@@ -560,16 +849,20 @@ __device__ __forceinline__ uint32_t half_permute_a(uint32_t x, const P2Params* p
 }
 
 // Lane l (of the caller's half-warp) passes state word l and gets word l of
-// the permuted state back. `p` points to shared memory. Not inlined: one copy
-// of its forms in a translation unit.
+// the permuted state back. `p` points to shared memory. Only KoalaBear's
+// exponent is inlined; one copy of the rest in a translation unit.
 template <class F>
-__device__ __noinline__ uint32_t p2_permute_half(uint32_t x, const P2Params* p) {
+__device__ __noinline__ uint32_t p2_permute_half_any(uint32_t x, const P2Params* p) {
   switch (p->alpha) {
     case 3: return half_permute_a<F, 3>(x, p);
-    case 5: return half_permute_a<F, 5>(x, p);
     case 7: return half_permute_a<F, 7>(x, p);
     default: return half_permute_a<F, 0>(x, p);
   }
+}
+template <class F>
+__device__ __forceinline__ uint32_t p2_permute_half(uint32_t x, const P2Params* p) {
+  if (F::ID == KoalaBear::ID && p->alpha == 3) return half_permute_a<F, 3>(x, p);
+  return p2_permute_half_any<F>(x, p);
 }
 
 // ----------------------------------------------------------- quarters ---
@@ -725,17 +1018,17 @@ struct HalfBb16 {
   }
 };
 
-// Stage run-time params into shared memory (whole block participates): the
-// words [FROM, TO) of the block, by default what one thread's permutation
-// reads (kP2ThreadWords); the half-warp tables follow.
+// Stage run-time params into shared memory (whole block participates), the
+// words [FROM, TO) of the block: what one thread's permutation reads lies in
+// front of the half-warp tables and, for one instance, behind them.
 constexpr int kP2Words = (int)(sizeof(P2Params) / 4);
-constexpr int kP2ThreadWords = (int)(offsetof(P2Params, chain) / 4);
-template <int FROM = 0, int TO = kP2Words>
-__device__ __forceinline__ void stage_params(P2Params* dst, const P2Params* src) {
+constexpr int kP2ChainAt = (int)(offsetof(P2Params, chain) / 4);
+constexpr int kP2Sp1At = (int)(offsetof(P2Params, sp1_rc) / 4);
+template <int FROM, int TO>
+__device__ __forceinline__ void stage_words(P2Params* dst, const P2Params* src) {
   const uint32_t* s = reinterpret_cast<const uint32_t*>(src);
   uint32_t* d = reinterpret_cast<uint32_t*>(dst);
   for (int i = FROM + threadIdx.x; i < TO; i += blockDim.x) d[i] = s[i];
-  __syncthreads();
 }
 
 }  // namespace zc
