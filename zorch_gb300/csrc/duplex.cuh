@@ -189,6 +189,16 @@ struct LaneDuplex {
     out_pos = pos == 0 ? 8 : 0;
   }
 
+  // After a whole block has been absorbed with nothing pending: y, the permuted
+  // sponge's word of this lane.
+  __device__ __forceinline__ void absorbed(uint32_t y) {
+    x = y;
+    in = 0u;
+    in_pos = 0;
+    out = (threadIdx.x & 15) < 8 ? y : 0u;
+    out_pos = 8;
+  }
+
   // The next challenge word, on every lane.
   template <class HP>
   __device__ __forceinline__ uint32_t sample(const HP& perm) {

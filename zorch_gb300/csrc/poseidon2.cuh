@@ -742,13 +742,28 @@ __device__ __forceinline__ uint32_t half_ext_linear(uint32_t x) {
   return madd<F>(madd<F>(y2, d), madd<F>(e, f));
 }
 
+// f (x + c)^alpha, the factor's product off the dependency chain: it multiplies
+// the first power, beside the square. FACTOR = false: f = 1.
+template <class F, int ALPHA, bool FACTOR>
+__device__ __forceinline__ uint32_t ark_sbox_times(uint32_t x, uint32_t c, uint32_t alpha,
+                                                   uint32_t f) {
+  if (!FACTOR) return ark_sbox_a<F, ALPHA>(x, c, alpha);
+  const int32_t a = (int32_t)(x + c - F::P);
+  if (ALPHA == 3) return snorm<F>(smul<F>(smul<F>(a, a), smul<F>(a, (int32_t)f)));
+  if (ALPHA == 7) {
+    const int32_t a2 = smul<F>(a, a);
+    return snorm<F>(smul<F>(smul<F>(a2, smul<F>(a, (int32_t)f)), smul<F>(a2, a2)));
+  }
+  return mmul<F>(ark_sbox_a<F, ALPHA>(x, c, alpha), f);
+}
+
 // n <= 16 partial rounds. Words 1..15 evolve linearly given the rounds' sums, so
 // with s_i the words at the start, y_r round r's S-box output and
 //   B_r = j * (sum of words 1..15 before round r)
 //       = sum_i j d_i^r s_i + sum_{m < r} j T_{r-1-m} sigma_m,  T_k = sum_{i>=1} d_i^k,
 // a round is sigma_r = j y_r + B_r and word 0 becomes (j + d_0) y_r + B_r: the chain
-// from one S-box to the next is one addition (a product more for j != 1), where
-// summing the fifteen words takes four shuffles and additions. Lane k
+// from one S-box to the next is one addition (two products more for a general
+// d_0), where summing the fifteen words takes four shuffles and additions. Lane k
 // holds B_k: its first sum is a 15-term dot product (15 independent shuffles,
 // four terms to a reduction), and each round adds j T_{k-1-r} sigma_r to it
 // while the next S-box runs. Each lane l > 0 keeps its own word, x_l = sigma_r
@@ -756,7 +771,8 @@ __device__ __forceinline__ uint32_t half_ext_linear(uint32_t x) {
 // as one wide accumulation, or B and x on the two halves of a warp in one
 // product, measured 10 % and 30 % slower: 2,107 and 2,504 cycles.)
 // MODE: 0: any j and d_0; 1: d_0 = -2 j, so word 0 becomes B_r - j y_r; 2: j = 1 too.
-// step(r, s0) = the S-box of round r on s0. Returns this lane's word.
+// step(r, s0) = the S-box of round r on s0, times j for MODE 1. Returns this
+// lane's word.
 template <class F, int MODE, bool UNROLL, class Step>
 __device__ __forceinline__ uint32_t half_partials(uint32_t x, int n, uint32_t dg, uint32_t j,
                                                   uint32_t e, uint32_t w, const int32_t (&m)[16],
@@ -777,7 +793,7 @@ __device__ __forceinline__ uint32_t half_partials(uint32_t x, int n, uint32_t dg
   uint32_t s0 = __shfl_sync(kFullMask, x, base), b = __shfl_sync(kFullMask, B, base);
   auto round = [&](int r) {
     const uint32_t y = step(r, s0);
-    const uint32_t jy = MODE == 2 ? y : mmul<F>(y, j);
+    const uint32_t jy = MODE > 0 ? y : mmul<F>(y, j);
     const uint32_t sigma = madd<F>(jy, b);
     s0 = MODE > 0 ? msub<F>(b, jy) : madd<F>(mmul<F>(y, e), b);
     x = madd<F>(sigma, mmul<F>(dg, x));
@@ -789,16 +805,13 @@ __device__ __forceinline__ uint32_t half_partials(uint32_t x, int n, uint32_t dg
 #pragma unroll
     for (int r = 0; r < ZC_BB16_ROUNDS_P; r++) round(r);
   } else {
-#pragma unroll 1
+#pragma unroll 5  // 1: 1,850 cycles for ten rounds of x^3, 5: 1,690
     for (int r = 0; r < n; r++) round(r);
   }
   return (threadIdx.x & 15) == 0 ? s0 : x;
 }
 
-// The rounds are rolled loops (constants read from shared memory one round
-// ahead): a permutation runs only a few times per launch here, so its code
-// is fetched cold, and a short loop body costs far fewer instruction-cache
-// misses than unrolled rounds.
+// Constants are read from shared memory one round ahead.
 template <class F, int ALPHA>
 __device__ __forceinline__ uint32_t half_permute_a(uint32_t x, const P2Params* p) {
   const int l = threadIdx.x & 15;
@@ -826,14 +839,20 @@ __device__ __forceinline__ uint32_t half_permute_a(uint32_t x, const P2Params* p
     for (int r0 = 0; r0 < rp; r0 += run) {
       const int n = rp - r0 < run ? rp - r0 : run;
       uint32_t rc = p->int_rc[r0];
-      const auto step = [&](int r, uint32_t s0) {
+      const auto next_rc = [&](int r) {
         const uint32_t cur = rc;
         rc = p->int_rc[r0 + r + 1 < rp ? r0 + r + 1 : 0];
-        return ark_sbox_a<F, ALPHA>(s0, cur, alpha);
+        return cur;
+      };
+      const auto step = [&](int r, uint32_t s0) {
+        return ark_sbox_a<F, ALPHA>(s0, next_rc(r), alpha);
+      };
+      const auto step_j = [&](int r, uint32_t s0) {
+        return ark_sbox_times<F, ALPHA, true>(s0, next_rc(r), alpha, js);
       };
       switch (p->chain_mode) {
         case 2: x = half_partials<F, 2, false>(x, n, dg, js, e, w, m, step); break;
-        case 1: x = half_partials<F, 1, false>(x, n, dg, js, e, w, m, step); break;
+        case 1: x = half_partials<F, 1, false>(x, n, dg, js, e, w, m, step_j); break;
         default: x = half_partials<F, 0, false>(x, n, dg, js, e, w, m, step); break;
       }
     }
@@ -906,12 +925,12 @@ __device__ __forceinline__ void quarter_full_round(uint32_t (&x)[4], const uint3
 }
 
 // One partial round; w0: word 0, on every lane (lane 0's x[0] is not kept).
-// MODE as in half_partials (chain_mode).
+// MODE as in half_partials (chain_mode): for 1, y below is j times the S-box.
 template <class F, int ALPHA, int MODE>
 __device__ __forceinline__ void quarter_partial_round(uint32_t (&x)[4], uint32_t& w0, uint32_t c,
                                                       uint32_t alpha, const uint32_t (&dg)[4],
                                                       uint32_t j, uint32_t d0) {
-  const uint32_t y = ark_sbox_a<F, ALPHA>(w0, c, alpha);
+  const uint32_t y = ark_sbox_times<F, ALPHA, MODE == 1>(w0, c, alpha, j);
   // words 1..15 of this round's input
   uint32_t part = madd<F>(madd<F>((threadIdx.x & 3) ? x[0] : 0u, x[1]), madd<F>(x[2], x[3]));
   part = madd<F>(part, __shfl_xor_sync(kFullMask, part, 1));
@@ -919,12 +938,10 @@ __device__ __forceinline__ void quarter_partial_round(uint32_t (&x)[4], uint32_t
   uint32_t dx[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) dx[k] = snorm<F>(smul3<F>((int32_t)x[k], (int32_t)dg[k]));
-  uint32_t sum = madd<F>(part, y);
-  if (MODE != 2) sum = mmul<F>(sum, j);
-  // word 0: j (part + y) + d_0 y, j (part - y) for d_0 = -2 j
-  if (MODE == 2) w0 = msub<F>(part, y);
-  if (MODE == 1) w0 = mmul<F>(msub<F>(part, y), j);
-  if (MODE == 0) w0 = madd<F>(sum, mmul<F>(d0, y));
+  if (MODE != 2) part = mmul<F>(part, j);
+  const uint32_t sum = madd<F>(part, MODE == 0 ? mmul<F>(y, j) : y);
+  // word 0: sum + d_0 y, j part - j y for d_0 = -2 j
+  w0 = MODE == 0 ? madd<F>(sum, mmul<F>(d0, y)) : msub<F>(part, y);
 #pragma unroll
   for (int k = 0; k < 4; k++) x[k] = madd<F>(sum, dx[k]);
 }
@@ -940,7 +957,7 @@ __device__ __forceinline__ void quarter_permute_a(uint32_t (&x)[4], const P2Para
 #pragma unroll 1
   for (int r = 0; r < rfh; r++) quarter_full_round<F, ALPHA>(x, p->ext_init[r], alpha);
   uint32_t w0 = __shfl_sync(kFullMask, x[0], threadIdx.x & ~3);
-#pragma unroll 1
+#pragma unroll 4  // 1: 6,570 cycles a permutation of x^3 (9,060 for j != 1), 4: 5,900 (6,990)
   for (int r = 0; r < rp; r++)
     quarter_partial_round<F, ALPHA, MODE>(x, w0, p->int_rc[r], alpha, dg, p->j_scale, p->diag[0]);
   if (q == 0) x[0] = w0;

@@ -64,11 +64,26 @@ __global__ void __launch_bounds__(32) k_round_hop(const P2Params* rt, const Roun
     __syncwarp();
   }
   with_half_perm<K>(rt, &s_rt, [&](const auto& perm) {
+    // SP1's separator: compress([root, sponge([log_height, width])]). Its first
+    // permutation runs on the upper half while the lower one observes the
+    // message, when that is one permutation (nothing pending).
+    uint32_t sep = l == 0 ? to_mont<F>(a.log_height) : (l == 1 ? to_mont<F>(a.width) : 0u);
+    bool sep_done = false;
+    if (a.msg) {
+      if (a.bind && (t.in_pos & 7) == 0) {
+        uint32_t x = lane < 16 ? (l < 8 ? vals[l] : t.x) : sep;
+        x = perm.half(x);
+        sep = __shfl_sync(kFullMask, x, 16 | l);
+        t.absorbed(__shfl_sync(kFullMask, x, l));
+        sep_done = true;
+      } else {
+        t.observe(vals, 8, perm);
+      }
+    }
     uint32_t root = raw;
     if (a.bind) {
-      uint32_t x = l == 0 ? to_mont<F>(a.log_height) : (l == 1 ? to_mont<F>(a.width) : 0u);
-      x = perm.half(x);
-      const uint32_t par = __shfl_sync(kFullMask, x, (lane & 16) | (l & 7));
+      if (!sep_done) sep = perm.half(sep);
+      const uint32_t par = __shfl_sync(kFullMask, sep, (lane & 16) | (l & 7));
       root = perm.half(l < 8 ? raw : par);
     }
     if (lane < 8) {
@@ -77,7 +92,6 @@ __global__ void __launch_bounds__(32) k_round_hop(const P2Params* rt, const Roun
       vals[8 + lane] = root;
     }
     __syncwarp();
-    if (a.msg) t.observe(vals, 8, perm);
     t.observe(vals + 8, 8, perm);
     for (int i = 0; i < a.n_chal; i++) {
       const uint32_t w = t.sample(perm);
