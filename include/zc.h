@@ -382,6 +382,11 @@ zc_status zc_sumcheck_fold(zc_field field, const uint32_t* mle, int64_t M, const
                            int32_t beta_limbs, const uint32_t* msg, uint32_t* mle_out,
                            const uint32_t* eq, uint32_t* eq_out, uint32_t* claim, void* stream);
 
+/* [n] EF4 words to [4][n] limbs (to_limbs != 0) or back: the layout of a
+ * transform that acts limb by limb (lax.ntt over an extension field). */
+zc_status zc_ef4_limbs(const uint32_t* in, int64_t n, int32_t to_limbs, uint32_t* out,
+                       void* stream);
+
 /* The commit-and-fold rounds of an open in one call, as FriProver's commit
  * phase (zorch/pcs/fold.py:90-115), the Basefold open (zorch/pcs/basefold/
  * prover.py:419-480) and the SP1 stacked open (zorch/pcs/jagged/open.py:237-330)

@@ -124,6 +124,7 @@ def _declare(lib: C.CDLL) -> None:
         "zc_rs_encode_batch_workspace_bytes": (sz, [vp, i32]),
         "zc_rs_encode_batch": (st, [st, vp, i32, u32, vp, sz, vp]),
         "zc_merkle_commit_batch": (st, [vp, vp, i32, vp, sz, vp]),
+        "zc_ef4_limbs": (st, [vp, i64, i32, vp, vp]),
         "zc_fold_rounds_workspace_bytes": (sz, [i32]),
         "zc_fold_rounds": (st, [vp, C.POINTER(FoldRoundsDesc), vp]),
         "zc_open_layers": (st, [C.POINTER(OpenJob), i32, vp, i32, vp]),

@@ -106,6 +106,14 @@ __device__ __forceinline__ void with_half_perm(const P2Params* rt, P2Params* s_r
   }
 }
 
+// The same out of line; p: the parameters, in shared memory or, for the built-in
+// instance, anywhere.
+template <class K>
+struct CallPerm {
+  const P2Params* p;
+  __device__ __forceinline__ uint32_t half(uint32_t x) const { return half_perm_call<K>(x, p); }
+};
+
 // The duplex on one warp: lane l of each half (both run the same) holds sponge
 // word l and, for l < 8, words l of the input and output buffers. The same
 // steps as duplex_observe and duplex_sample with no word-by-word state in

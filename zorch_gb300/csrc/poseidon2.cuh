@@ -267,6 +267,7 @@ struct Pow2 {
 struct Bb16Builtin {
   using F = BabyBear;
   static constexpr bool kOwnPermute = true;
+  static constexpr bool kOwnTables = true;  // the compile-time instance
   // x + c in (-p, p), c_lp = c - p; the power chain is unnormalised.
   __device__ __forceinline__ static uint32_t sbox(uint32_t x, uint32_t c_lp) {
     const int32_t a = (int32_t)(x + c_lp);
@@ -356,6 +357,7 @@ struct Bb16Builtin {
 template <class F_>
 struct RtParams {
   using F = F_;
+  static constexpr bool kOwnTables = false;
 #ifdef __CUDA_ARCH__
   static constexpr bool kOwnPermute = true;
 #else
@@ -1034,6 +1036,18 @@ struct HalfBb16 {
     return x;
   }
 };
+
+// The half-warp permutation out of line, for a round's hop, which has it at five
+// places and runs once between large kernels: its code comes from L2 (or, after
+// a layer of hundreds of MB, from HBM) each time, 15 KB instead of 75 (5.7 us a
+// hop inlined, 4.3 out of line).
+template <class K>
+__device__ __noinline__ uint32_t half_perm_call(uint32_t x, const P2Params* p) {
+  if constexpr (K::kOwnTables)
+    return HalfBb16(p).permute(x);
+  else
+    return p2_permute_half<typename K::F>(x, p);
+}
 
 // Stage run-time params into shared memory (whole block participates), the
 // words [FROM, TO) of the block: what one thread's permutation reads lies in

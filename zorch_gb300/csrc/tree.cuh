@@ -35,10 +35,10 @@ struct RootHop {
 };
 
 // One full warp (all 32 lanes: half-warp permutations shuffle across it).
-// Not inlined: compiled once per field, not into every subtree variant.
-template <class F>
-__device__ __noinline__ void root_hop(const RootHop hop, const uint32_t* root, const P2Params* hp) {
-  const HalfPerm<F> perm{hp};
+template <class K>
+__device__ __forceinline__ void root_hop(const RootHop hop, const uint32_t* root,
+                                         const P2Params* hp) {
+  const CallPerm<K> perm{hp};
   LaneDuplex t;
   t.load(hop.state);
   t.observe(root, 8, perm);
@@ -298,25 +298,19 @@ inline int subtree_threads(int T) {
   return t < 1024 ? t : 1024;
 }
 
-// Half-warp permutation of the caller's field (lane l passes state word l).
-template <class F>
-__device__ __forceinline__ uint32_t half_perm(uint32_t x, const P2Params* hp) {
-  return p2_permute_half<F>(x, hp);
-}
-// The same for the provider K: the built-in instance runs unrolled, its lane
-// constants read from the staged copy.
+// The tree kernels' permutations for the provider K, inlined (out of line, as
+// the hop's, measured 1 to 5 % slower on the opens: the constants are loaded per
+// call).
 template <class K>
 __device__ __forceinline__ uint32_t half_perm_k(uint32_t x, const P2Params* hp) {
-  if constexpr (std::is_same<K, Bb16Builtin>::value)
+  if constexpr (K::kOwnTables)
     return HalfBb16(hp).permute(x);
   else
     return p2_permute_half<typename K::F>(x, hp);
 }
-
-// Quarter-warp permutation for the provider K.
 template <class K>
 __device__ __forceinline__ void quarter_perm_k(uint32_t (&x)[4], const P2Params* hp) {
-  if constexpr (std::is_same<K, Bb16Builtin>::value)
+  if constexpr (K::kOwnTables)
     quarter_permute_bb16(x, hp);
   else
     p2_permute_quarter<typename K::F>(x, hp);
@@ -377,7 +371,6 @@ template <class K, class Leaf>
 __global__ void __launch_bounds__(1024) k_subtree(Leaf leaf, uint32_t* layers, int64_t L,
                                                        int l0, int T, const P2Params* rt,
                                                        RootHop hop) {
-  using F = typename K::F;
   __shared__ P2Params s_rt;
   __shared__ __align__(16) uint32_t sm[2][8 * kSubCap];  // [node][word] digest slots
   KIn<K>::make(rt, &s_rt);
@@ -414,7 +407,7 @@ __global__ void __launch_bounds__(1024) k_subtree(Leaf leaf, uint32_t* layers, i
   }
   if (hop.state) {  // passed only to a one-CTA launch that ends at the root
     __syncthreads();
-    if (threadIdx.x < 32) root_hop<F>(hop, sm[cur], hp);
+    if (threadIdx.x < 32) root_hop<K>(hop, sm[cur], hp);
   }
 }
 

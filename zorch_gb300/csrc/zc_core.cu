@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(32) k_duplex_step(const P2Params* rt, uint32_t
   with_half_perm<K>(rt, &s_rt, [&](const auto& perm) {
     t.observe(values, m, perm);
     for (int i = 0; i < n; i++) {
-      const uint32_t w = t.sample(perm);
+      const uint32_t w = t.sample(CallPerm<K>{K::kOwnTables ? rt : &s_rt});
       if (threadIdx.x == 0) {
         if (out) out[i] = w;
         if (positions) positions[i] = (int32_t)(w % (uint32_t)block_len);
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(32) k_duplex_hop(
   with_half_perm<K>(rt, &s_rt, [&](const auto& perm) {
     t.observe(values, m, perm);
     for (int i = 0; i < n; i++) {
-      const uint32_t w = t.sample(perm);
+      const uint32_t w = t.sample(CallPerm<K>{K::kOwnTables ? rt : &s_rt});
       if (threadIdx.x == 0) chal[i] = w;
     }
   });

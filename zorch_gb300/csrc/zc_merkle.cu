@@ -1,5 +1,5 @@
 // Merkle commits (single, strided, batched over many trees), openings, the
-// SP1 root binding, the partial-Lagrange column batching and device fills.
+// SP1 root binding and device fills.
 // The tree kernels themselves are in tree.cuh.
 #include <string.h>
 
@@ -50,11 +50,11 @@ __global__ void __launch_bounds__(32) k_bind_root(const P2Params* rt, const uint
   const int lane = threadIdx.x & 31, l = lane & 15;
   // sponge: state = [log_height, width, 0 ...] (one absorb block), permute
   uint32_t x = l == 0 ? to_mont<F>(log_height) : (l == 1 ? to_mont<F>(width) : 0u);
-  x = half_perm<F>(x, hp);
+  x = half_perm_call<K>(x, hp);
   // compress: state = raw_root || params (params = words 0..7 of the sponge)
   const uint32_t par = __shfl_sync(kFullMask, x, (lane & 16) | (l & 7));
   uint32_t y = l < 8 ? raw_root[l] : par;
-  y = half_perm<F>(y, hp);
+  y = half_perm_call<K>(y, hp);
   __syncwarp();  // raw_root may alias out: every lane has read it
   if (lane < 8) out[lane] = y;
 }
@@ -226,45 +226,6 @@ zc_status tree_batch_wave(const zc_merkle_job* jobs, int n, unsigned long long* 
   return launch_check();
 }
 
-// Staggered partial-Lagrange batching of one committed matrix's columns into
-// one EF4 codeword (sample_rlc_coeffs_bits + batch_staggered,
-// zorch/pcs/jagged/open.py:88-105, zorch/pcs/basefold/batching.py:66-80):
-// weights = eq(., r) over nbv = ceil(log2 w) EF4 challenges, table built by
-// the MSB-first interleaving step (zorch/poly/eq.py:55-62: high = s*r,
-// low = s - high), column c weighted by entry c; out[j] = sum_c wt_c cw[c][j].
-template <class F>
-__global__ void k_rlc(const uint32_t* cw, int64_t n, int w, const uint32_t* chal, int nbv,
-                      uint32_t* out) {
-  extern __shared__ uint32_t wt[];  // 2^nbv x 4 (EF4)
-  if (threadIdx.x == 0) {
-    wt[0] = F::ONE;
-    wt[1] = wt[2] = wt[3] = 0;
-    for (int j = 0; j < nbv; j++) {
-      const ef4 r{{chal[4 * j], chal[4 * j + 1], chal[4 * j + 2], chal[4 * j + 3]}};
-      for (int i = (1 << j) - 1; i >= 0; i--) {  // in place, from the top
-        const ef4 s{{wt[4 * i], wt[4 * i + 1], wt[4 * i + 2], wt[4 * i + 3]}};
-        const ef4 hi = ef_mul<F>(s, r);
-        const ef4 lo = ef_sub<F>(s, hi);
-        for (int e = 0; e < 4; e++) {
-          wt[4 * (2 * i) + e] = lo.c[e];
-          wt[4 * (2 * i + 1) + e] = hi.c[e];
-        }
-      }
-    }
-  }
-  __syncthreads();
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n;
-       j += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t r[4] = {0, 0, 0, 0};
-    for (int c = 0; c < w; c++) {
-      const uint32_t x = __ldg(cw + (int64_t)c * n + j);
-#pragma unroll
-      for (int e = 0; e < 4; e++) r[e] = madd<F>(r[e], mmul<F>(wt[4 * c + e], x));
-    }
-    reinterpret_cast<uint4*>(out)[j] = make_uint4(r[0], r[1], r[2], r[3]);
-  }
-}
-
 // Seeded synthetic field data: SplitMix64(seed, index) reduced mod p.
 __host__ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
   x += 0x9E3779B97F4A7C15ull;
@@ -429,23 +390,6 @@ zc_status zc_merkle_commit_batch(const zc_poseidon2* p, const zc_merkle_job* job
       ZC_TRY(tree_batch_wave<K>(jobs + i, n, ctr, rt, st));
     }
     return ZC_OK;
-  });
-}
-
-zc_status zc_rlc_columns(zc_field field, const uint32_t* cw, int64_t n, int32_t w,
-                         const uint32_t* challenges, uint32_t* out, void* stream) {
-  if (!cw || !out || n < 0 || w < 1 || w > 4096) return ZC_BAD_ARG;
-  const int nbv = ilog2(w);
-  if (nbv > 0 && !challenges) return ZC_BAD_ARG;
-  if ((uintptr_t)out % 16) return ZC_BAD_ARG;
-  if (n == 0) return ZC_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  return with_field(field, [&](auto f) {
-    using F = decltype(f);
-    int64_t blocks = (n + 255) / 256;
-    if (blocks > 152 * 8) blocks = 152 * 8;
-    k_rlc<F><<<(unsigned)blocks, 256, ((size_t)16) << nbv, st>>>(cw, n, w, challenges, nbv, out);
-    return launch_check();
   });
 }
 

@@ -29,30 +29,38 @@ struct RoundHop1 {
   uint32_t* chal;
 };
 
-// One warp: the round's message (s0 = the partials' sum, s1 = (claim - s0) /
+// Threads of a round's hop: the CTA sums the message's partials (608 of them took
+// one warp 20 us), then its first warp goes on alone.
+constexpr int kHopT = 256;
+
+// The round's message (s0 = the partials' sum, s1 = (claim - s0) /
 // z_last + s0, zorch/pcs/basefold/kernel.py:52-66), observed; the layer's root,
 // bound if asked (k_bind_root's two permutations), observed; n_chal challenge
 // words squeezed. A chain of 1 to 5 permutations; as separate launches it was
 // three to five of them with a launch gap between each.
 template <class K>
-__global__ void __launch_bounds__(32) k_round_hop(const P2Params* rt, const RoundHop1 a) {
+__global__ void __launch_bounds__(kHopT) k_round_hop(const P2Params* rt, const RoundHop1 a) {
   using F = typename K::F;
   __shared__ P2Params s_rt;
   __shared__ uint32_t vals[16];
   const int lane = threadIdx.x & 31, l = lane & 15;
   LaneDuplex t;
-  t.load(a.state);
-  const uint32_t raw = a.root[l & 7];
+  uint32_t raw = 0;
+  if (threadIdx.x < 32) {
+    t.load(a.state);
+    raw = a.root[l & 7];
+  }
+  if constexpr (!K::kOwnTables) {
+    KIn<K>::make(rt, &s_rt);  // staged by the whole CTA
+    KIn<K>::half(rt, &s_rt);
+  }
   if (a.msg) {
     ef4 s0{{0, 0, 0, 0}};
-    for (int i = lane; i < a.np; i += 32) s0 = ef_add<F>(s0, ld4(a.partial + 4 * i));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int e = 0; e < 4; e++)
-        s0.c[e] = madd<F>(s0.c[e], __shfl_xor_sync(kFullMask, s0.c[e], o));
-    const ef4 s1 = ef_add<F>(ef_mul<F>(ef_sub<F>(ld4(a.claim), s0), ld4(a.zinv)), s0);
-    if (lane == 0) {
+    for (int i = threadIdx.x; i < a.np; i += blockDim.x)
+      s0 = ef_add<F>(s0, ld4(a.partial + 4 * i));
+    s0 = block_sum<F>(s0);
+    if (threadIdx.x == 0) {
+      const ef4 s1 = ef_add<F>(ef_mul<F>(ef_sub<F>(ld4(a.claim), s0), ld4(a.zinv)), s0);
       st4(a.msg, s0);
       st4(a.msg + 4, s1);
 #pragma unroll
@@ -61,9 +69,10 @@ __global__ void __launch_bounds__(32) k_round_hop(const P2Params* rt, const Roun
         vals[4 + e] = s1.c[e];
       }
     }
-    __syncwarp();
+    __syncthreads();
   }
-  with_half_perm<K>(rt, &s_rt, [&](const auto& perm) {
+  if (threadIdx.x >= 32) return;
+  const auto body = [&](const auto& perm) {
     // SP1's separator: compress([root, sponge([log_height, width])]). Its first
     // permutation runs on the upper half while the lower one observes the
     // message, when that is one permutation (nothing pending).
@@ -97,7 +106,8 @@ __global__ void __launch_bounds__(32) k_round_hop(const P2Params* rt, const Roun
       const uint32_t w = t.sample(perm);
       if (lane == 0) a.chal[i] = w;
     }
-  });
+  };
+  body(CallPerm<K>{K::kOwnTables ? rt : &s_rt});
   t.store(a.state);
 }
 
@@ -214,7 +224,7 @@ zc_status zc_fold_rounds(const zc_poseidon2* p, const zc_fold_rounds_desc* d, vo
     h.n_chal = d->beta_limbs;
     h.chal = beta;
     ZC_TRY(with_perm(p, [&](auto k, const P2Params* rt) {
-      k_round_hop<decltype(k)><<<1, 32, 0, st>>>(rt, h);
+      k_round_hop<decltype(k)><<<1, kHopT, 0, st>>>(rt, h);
       return launch_check();
     }));
     const bool last = r == d->rounds - 1;

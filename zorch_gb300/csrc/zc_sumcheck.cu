@@ -14,32 +14,42 @@
 
 namespace zc {
 
-// expand_eq_to_hypercube(z, 1) for m <= kEqSmall variables on one block:
-// out[2i] = s - s z_j, out[2i+1] = s z_j per step (z[0] ends on the top bit).
+// expand_eq_to_hypercube(z, 1) for m <= kEqSmall variables, one CTA a table
+// (z[0] ends on the top bit): the tables of the upper and the lower half of the
+// variables are doubled up side by side in shared memory (out[2i] = s - s z_j,
+// out[2i+1] = s z_j), at most six dependent products, and the table is their
+// outer product. Twelve variables took 14.5 us doubled through global memory,
+// one step after another.
 constexpr int kEqSmall = 12;
+struct EqTable {
+  const uint32_t* z;
+  int m;
+  uint32_t* out;
+};
 template <class F>
-__global__ void __launch_bounds__(1024) k_eq_small(const uint32_t* z, int m, uint32_t* out) {
-  if (threadIdx.x == 0) st4(out, ef4{{F::ONE, 0, 0, 0}});
-  __syncthreads();
-  for (int j = 0; j < m; j++) {
-    const ef4 zj = ld4(z + 4 * j);
-    const int half = 1 << j;
-    // read all of level j before anyone writes level j+1 (in place)
-    ef4 lo[4], hi[4];
-    int cnt = 0;
-    for (int i = threadIdx.x; i < half && cnt < 4; i += blockDim.x, cnt++) {
-      const ef4 s = ld4(out + 4 * i);
-      hi[cnt] = ef_mul<F>(s, zj);
-      lo[cnt] = ef_sub<F>(s, hi[cnt]);
-    }
+__global__ void __launch_bounds__(512) k_eq_small(const EqTable t0, const EqTable t1) {
+  constexpr int H = kEqSmall / 2;
+  __shared__ __align__(16) uint32_t tab[2][2][4 << H];  // [parity of the step][half][entry]
+  const EqTable t = blockIdx.x ? t1 : t0;
+  const int m1 = t.m / 2, m2 = t.m - m1;
+  const int half = threadIdx.x >> H, i = threadIdx.x & ((1 << H) - 1);  // halves 0 and 1 work
+  const int mh = half == 0 ? m1 : m2;
+  const uint32_t* zh = half == 0 ? t.z : t.z + 4 * m1;
+  if (half < 2 && i == 0) st4(tab[0][half], ef4{{F::ONE, 0, 0, 0}});
+  for (int j = 0; j < H; j++) {
     __syncthreads();
-    cnt = 0;
-    for (int i = threadIdx.x; i < half && cnt < 4; i += blockDim.x, cnt++) {
-      st4(out + 4 * (2 * i), lo[cnt]);
-      st4(out + 4 * (2 * i + 1), hi[cnt]);
+    if (half < 2 && j < mh && i < (1 << j)) {
+      const ef4 s = ld4(tab[j & 1][half] + 4 * i);
+      const ef4 hi = ef_mul<F>(s, ld4(zh + 4 * j));
+      st4(tab[(j & 1) ^ 1][half] + 8 * i, ef_sub<F>(s, hi));
+      st4(tab[(j & 1) ^ 1][half] + 8 * i + 4, hi);
     }
-    __syncthreads();
   }
+  __syncthreads();
+  const uint32_t *hi = tab[m1 & 1][0], *lo = tab[m2 & 1][1];  // after m1 and m2 steps
+  for (int k = threadIdx.x; k < (1 << t.m); k += blockDim.x)
+    st4(t.out + 4 * k,
+        ef_mul<F>(ld4(hi + 4 * (k >> m2)), ld4(lo + 4 * (k & ((1 << m2) - 1)))));
 }
 
 // out[i] = hi[i >> m2] * lo[i & (2^m2 - 1)]: the table of z = (z_hi, z_lo) as
@@ -68,35 +78,65 @@ inline size_t eq_ws_bytes(int m) {
 template <class F>
 zc_status eq_expand(const uint32_t* z, int m, uint32_t* out, uint32_t* ws, cudaStream_t st) {
   if (m <= kEqSmall) {
-    k_eq_small<F><<<1, 1024, 0, st>>>(z, m, out);
+    k_eq_small<F><<<1, 512, 0, st>>>(EqTable{z, m, out}, EqTable{});
     return launch_check();
   }
   const int m1 = m / 2, m2 = m - m1;
   uint32_t* th = ws;
   uint32_t* tl = ws + ((size_t)4 << m1);
-  k_eq_small<F><<<1, 1024, 0, st>>>(z, m1, th);
-  ZC_TRY(launch_check());
-  k_eq_small<F><<<1, 1024, 0, st>>>(z + 4 * m1, m2, tl);
+  k_eq_small<F><<<2, 512, 0, st>>>(EqTable{z, m1, th}, EqTable{z + 4 * m1, m2, tl});
   ZC_TRY(launch_check());
   const int64_t total = (int64_t)1 << m;
   k_eq_outer<F><<<grid_for(total, 256), 256, 0, st>>>(th, tl, m2, total, out);
   return launch_check();
 }
 
-// eval_mle of base columns with eq = hi (x) lo: partial[c][h] =
-// sum_l lo[l] cols[c][h 2^m2 + l], one block per (h, c).
+// acc[c] += w[c] x for EF4 weights w and base words x, two terms to a reduction:
+// |w_e x| <= p * p/2 with x of least magnitude, so two products sum to at most
+// p^2, which sredc takes.
 template <class F>
-__global__ void __launch_bounds__(256) k_eval_inner(const uint32_t* cols, int64_t S, int m2,
+__device__ __forceinline__ void ef_dot2(ef4& acc, const ef4& w0, uint32_t x0, const ef4& w1,
+                                        uint32_t x1) {
+  const int32_t a = centred<F>(x0), b = centred<F>(x1);
+#pragma unroll
+  for (int e = 0; e < 4; e++)
+    acc.c[e] = madd<F>(acc.c[e], snorm<F>(sredc<F>((int64_t)(int32_t)w0.c[e] * a +
+                                                   (int64_t)(int32_t)w1.c[e] * b)));
+}
+
+// eval_mle of base columns with eq = hi (x) lo: partial[c][h] =
+// sum_l lo[l] cols[c][h 2^m2 + l], one CTA per h and kEvalCols columns: a table
+// entry (16 bytes) is read once for four column words (4 bytes each), where
+// reading it for every word made the table the larger traffic (24 us for 2^20 x
+// 8; the columns are 5 us of HBM).
+constexpr int kEvalCols = 4;
+template <class F>
+__global__ void __launch_bounds__(256) k_eval_inner(const uint32_t* cols, int w, int64_t S, int m2,
                                                     const uint32_t* lo, uint32_t* partial,
                                                     int64_t H) {
-  const int64_t h = blockIdx.x, c = blockIdx.y;
+  const int64_t h = blockIdx.x;
+  const int c0 = blockIdx.y * kEvalCols;
   const int64_t L = (int64_t)1 << m2;
-  const uint32_t* col = cols + c * S + h * L;
-  ef4 acc{{0, 0, 0, 0}};
-  for (int64_t l = threadIdx.x; l < L; l += blockDim.x)
-    acc = ef_add<F>(acc, ef_base<F>(ld4(lo + 4 * l), __ldg(col + l)));
-  acc = block_sum<F>(acc);
-  if (threadIdx.x == 0) st4(partial + 4 * (c * H + h), acc);
+  ef4 acc[kEvalCols];
+#pragma unroll
+  for (int c = 0; c < kEvalCols; c++) acc[c] = ef4{{0, 0, 0, 0}};
+  for (int64_t l = threadIdx.x; l < L; l += 2 * blockDim.x) {
+    const bool two = l + blockDim.x < L;
+    const ef4 w0 = ld4(lo + 4 * l);
+    const ef4 w1 = two ? ld4(lo + 4 * (l + blockDim.x)) : ef4{{0, 0, 0, 0}};
+#pragma unroll
+    for (int c = 0; c < kEvalCols; c++) {
+      if (c0 + c >= w) break;
+      const uint32_t* col = cols + (c0 + c) * S + h * L + l;
+      ef_dot2<F>(acc[c], w0, __ldg(col), w1, two ? __ldg(col + blockDim.x) : 0u);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < kEvalCols; c++) {
+    if (c0 + c >= w) break;  // the same for the whole CTA
+    const ef4 r = block_sum<F>(acc[c]);
+    if (threadIdx.x == 0) st4(partial + 4 * ((c0 + c) * H + h), r);
+  }
 }
 
 // out[c] = sum_h hi[h] partial[c][h], one block per column.
@@ -133,9 +173,16 @@ zc_status eval_mle(const uint32_t* cols, int w, int m, const uint32_t* z, uint32
   uint32_t* lo = hi + 4 * H;
   uint32_t* partial = lo + ((size_t)4 << m2);
   uint32_t* eqws = partial + 4 * (size_t)w * H;
-  ZC_TRY(eq_expand<F>(z, m1, hi, eqws, st));           // z[0 .. m1): high index bits
-  ZC_TRY(eq_expand<F>(z + 4 * m1, m2, lo, eqws, st));  // z[m1 .. m): low index bits
-  k_eval_inner<F><<<dim3((unsigned)H, (unsigned)w), 256, 0, st>>>(cols, S, m2, lo, partial, H);
+  // z[0 .. m1): high index bits, z[m1 .. m): low ones (m2 <= kEqSmall)
+  if (m1 <= kEqSmall) {
+    k_eq_small<F><<<2, 512, 0, st>>>(EqTable{z, m1, hi}, EqTable{z + 4 * m1, m2, lo});
+    ZC_TRY(launch_check());
+  } else {
+    ZC_TRY(eq_expand<F>(z, m1, hi, eqws, st));
+    ZC_TRY(eq_expand<F>(z + 4 * m1, m2, lo, eqws, st));
+  }
+  k_eval_inner<F><<<dim3((unsigned)H, (unsigned)((w + kEvalCols - 1) / kEvalCols)), 256, 0, st>>>(
+      cols, w, S, m2, lo, partial, H);
   ZC_TRY(launch_check());
   k_eval_outer<F><<<(unsigned)w, 256, 0, st>>>(partial, hi, H, out);
   return launch_check();
@@ -225,63 +272,94 @@ __global__ void __launch_bounds__(256) k_sc_fold_reduce(const uint32_t* mle, int
   }
 }
 
-// Staggered batching with an offset into the weight table and accumulation
-// (batch_staggered, zorch/pcs/basefold/batching.py:66-80).
+// The partial-Lagrange weight of entry `idx` over nbv EF4 challenges: the product
+// over the bits of idx, from the top, of r_j or 1 - r_j (zorch/poly/eq.py:55-62).
 template <class F>
-__global__ void k_rlc_ex(const uint32_t* cw, int64_t n, int w, const uint32_t* chal, int nbv,
-                         int offset, int accumulate, uint32_t* out) {
-  extern __shared__ uint32_t wt[];  // 2^nbv x 4
-  if (threadIdx.x == 0) {
-    wt[0] = F::ONE;
-    wt[1] = wt[2] = wt[3] = 0;
-    for (int j = 0; j < nbv; j++) {
-      const ef4 r{{chal[4 * j], chal[4 * j + 1], chal[4 * j + 2], chal[4 * j + 3]}};
-      for (int i = (1 << j) - 1; i >= 0; i--) {
-        const ef4 s{{wt[4 * i], wt[4 * i + 1], wt[4 * i + 2], wt[4 * i + 3]}};
-        const ef4 hi = ef_mul<F>(s, r);
-        const ef4 lo = ef_sub<F>(s, hi);
-        for (int e = 0; e < 4; e++) {
-          wt[4 * (2 * i) + e] = lo.c[e];
-          wt[4 * (2 * i + 1) + e] = hi.c[e];
-        }
-      }
-    }
+__device__ __forceinline__ ef4 rlc_weight(const uint32_t* chal, int nbv, int idx) {
+  ef4 w{{F::ONE, 0, 0, 0}};
+  for (int j = 0; j < nbv; j++) {
+    const ef4 wr = ef_mul<F>(w, ef4{{__ldg(chal + 4 * j), __ldg(chal + 4 * j + 1),
+                                     __ldg(chal + 4 * j + 2), __ldg(chal + 4 * j + 3)}});
+    w = (idx >> (nbv - 1 - j)) & 1 ? wr : ef_sub<F>(w, wr);
   }
+  return w;
+}
+
+// Staggered batching with an offset into the weight table and accumulation
+// (batch_staggered, zorch/pcs/basefold/batching.py:66-80): out[j] (+)= sum_c
+// weights[offset + c] cw[c][j]. A CTA forms its w weights one per thread (one
+// thread doubling up the whole table took 10 us and more before the first
+// word), then two columns go to a reduction (ef_dot2). Bound by the columns'
+// bytes: 2^21 x 8 words in 45 us before.
+template <class F>
+__global__ void __launch_bounds__(256) k_rlc_ex(const uint32_t* cw, int64_t n, int w,
+                                                const uint32_t* chal, int nbv, int offset,
+                                                int accumulate, uint32_t* out) {
+  extern __shared__ __align__(16) uint32_t wt[];  // w x 4
+  for (int c = threadIdx.x; c < w; c += blockDim.x)
+    st4(wt + 4 * c, rlc_weight<F>(chal, nbv, offset + c));
   __syncthreads();
   for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n;
        j += (int64_t)gridDim.x * blockDim.x) {
     ef4 r{{0, 0, 0, 0}};
     if (accumulate) r = ld4(out + 4 * j);
-    for (int c = 0; c < w; c++) {
-      const uint32_t x = __ldg(cw + (int64_t)c * n + j);
-      const uint32_t* wc = wt + 4 * (offset + c);
-#pragma unroll
-      for (int e = 0; e < 4; e++) r.c[e] = madd<F>(r.c[e], mmul<F>(wc[e], x));
+    const uint32_t* x = cw + j;
+    int c = 0;
+    for (; c + 4 <= w; c += 4) {
+      const uint32_t x0 = __ldg(x + c * n), x1 = __ldg(x + (c + 1) * n),
+                     x2 = __ldg(x + (c + 2) * n), x3 = __ldg(x + (c + 3) * n);
+      ef_dot2<F>(r, ld4(wt + 4 * c), x0, ld4(wt + 4 * c + 4), x1);
+      ef_dot2<F>(r, ld4(wt + 4 * c + 8), x2, ld4(wt + 4 * c + 12), x3);
+    }
+    for (; c < w; c += 2) {
+      const bool two = c + 1 < w;
+      ef_dot2<F>(r, ld4(wt + 4 * c), __ldg(x + c * n),
+                 two ? ld4(wt + 4 * c + 4) : ef4{{0, 0, 0, 0}}, two ? __ldg(x + (c + 1) * n) : 0u);
     }
     st4(out + 4 * j, r);
   }
 }
 
-// out = sum_c weights[offset + c] values[c] (EF4 x EF4), accumulated; one
-// thread (the claim of the batch, a handful of columns).
+// out (+)= sum_c weights[offset + c] values[c] (EF4 x EF4): the claim of the
+// batch, one column a thread.
 template <class F>
-__global__ void k_rlc_values(const uint32_t* values, int w, const uint32_t* chal, int nbv,
-                             int offset, int accumulate, uint32_t* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__global__ void __launch_bounds__(256) k_rlc_values(const uint32_t* values, int w,
+                                                    const uint32_t* chal, int nbv, int offset,
+                                                    int accumulate, uint32_t* out) {
   ef4 acc{{0, 0, 0, 0}};
-  if (accumulate) acc = ld4(out);
-  for (int c = 0; c < w; c++) {
-    // weight offset+c = prod_j (bit j of (offset+c) from the top ? r_j : 1 - r_j)
-    ef4 wgt{{F::ONE, 0, 0, 0}};
-    const int idx = offset + c;
-    for (int j = 0; j < nbv; j++) {
-      const ef4 r = ld4(chal + 4 * j);
-      const bool bit = (idx >> (nbv - 1 - j)) & 1;
-      wgt = bit ? ef_mul<F>(wgt, r) : ef_sub<F>(wgt, ef_mul<F>(wgt, r));
+  for (int c = threadIdx.x; c < w; c += blockDim.x)
+    acc = ef_add<F>(acc, ef_mul<F>(rlc_weight<F>(chal, nbv, offset + c), ld4(values + 4 * c)));
+  acc = block_sum<F>(acc);
+  if (threadIdx.x == 0) st4(out, accumulate ? ef_add<F>(acc, ld4(out)) : acc);
+}
+
+// [4][n] limbs <-> [n] EF4 words, for a transform that acts limb by limb.
+__global__ void __launch_bounds__(256) k_ef4_limbs(const uint32_t* in, int64_t n, int to_limbs,
+                                                   uint32_t* out) {
+  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n;
+       j += (int64_t)gridDim.x * blockDim.x) {
+    if (to_limbs) {
+      const ef4 v = ld4(in + 4 * j);
+#pragma unroll
+      for (int e = 0; e < 4; e++) out[e * n + j] = v.c[e];
+    } else {
+      st4(out + 4 * j, ef4{{in[j], in[n + j], in[2 * n + j], in[3 * n + j]}});
     }
-    acc = ef_add<F>(acc, ef_mul<F>(wgt, ld4(values + 4 * c)));
   }
-  st4(out, acc);
+}
+
+// Up to eight CTAs per SM (each forms the weights once). w <= 4096: 64 KB of them.
+template <class F>
+zc_status rlc_launch(const uint32_t* cw, int64_t n, int w, const uint32_t* chal, int nbv,
+                     int offset, int accumulate, uint32_t* out, cudaStream_t st) {
+  const size_t smem = (size_t)16 * w;
+  if (smem > 48 * 1024)
+    ZC_CUDA(cudaFuncSetAttribute(k_rlc_ex<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem));
+  int64_t blocks = (n + 255) / 256;
+  if (blocks > 152 * 8) blocks = 152 * 8;
+  k_rlc_ex<F><<<(unsigned)blocks, 256, smem, st>>>(cw, n, w, chal, nbv, offset, accumulate, out);
+  return launch_check();
 }
 
 constexpr int kReduceBlocks = 256;
@@ -373,10 +451,30 @@ zc_status zc_rlc_columns_ex(zc_field field, const uint32_t* cw, int64_t n, int32
   cudaStream_t st = (cudaStream_t)stream;
   return with_field(field, [&](auto f) {
     using F = decltype(f);
-    k_rlc_ex<F><<<grid_for(n, 256), 256, ((size_t)16) << nbv, st>>>(cw, n, w, challenges, nbv,
-                                                                    offset, accumulate, out);
-    return launch_check();
+    return rlc_launch<F>(cw, n, w, challenges, nbv, offset, accumulate, out, st);
   });
+}
+
+zc_status zc_rlc_columns(zc_field field, const uint32_t* cw, int64_t n, int32_t w,
+                         const uint32_t* challenges, uint32_t* out, void* stream) {
+  if (!cw || !out || n < 0 || w < 1 || w > 4096) return ZC_BAD_ARG;
+  const int nbv = ilog2(w);
+  if (nbv > 0 && !challenges) return ZC_BAD_ARG;
+  if ((uintptr_t)out % 16) return ZC_BAD_ARG;
+  if (n == 0) return ZC_OK;
+  return with_field(field, [&](auto f) {
+    using F = decltype(f);
+    return rlc_launch<F>(cw, n, w, challenges, nbv, 0, 0, out, (cudaStream_t)stream);
+  });
+}
+
+zc_status zc_ef4_limbs(const uint32_t* in, int64_t n, int32_t to_limbs, uint32_t* out,
+                       void* stream) {
+  if (n < 0 || (n > 0 && (!in || !out))) return ZC_BAD_ARG;
+  if ((uintptr_t)(to_limbs ? in : out) % 16) return ZC_BAD_ARG;
+  if (n == 0) return ZC_OK;
+  k_ef4_limbs<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(in, n, to_limbs, out);
+  return launch_check();
 }
 
 zc_status zc_rlc_values(zc_field field, const uint32_t* values, int32_t w,
@@ -388,7 +486,7 @@ zc_status zc_rlc_values(zc_field field, const uint32_t* values, int32_t w,
   cudaStream_t st = (cudaStream_t)stream;
   return with_field(field, [&](auto f) {
     using F = decltype(f);
-    k_rlc_values<F><<<1, 32, 0, st>>>(values, w, challenges, nbv, offset, accumulate, out);
+    k_rlc_values<F><<<1, 256, 0, st>>>(values, w, challenges, nbv, offset, accumulate, out);
     return launch_check();
   });
 }

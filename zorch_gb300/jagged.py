@@ -25,7 +25,7 @@ import torch
 from . import _lib
 from .coding import BitReversedReedSolomon
 from .commit import DigestLayers, SingleMatrixCommitmentScheme, leaves_layout
-from .field import from_mont, ptr, stream_handle, to_host
+from .field import from_mont, full_u32, ptr, stream_handle, to_host
 from .pcs import layer_spec, open_layers, run_fold_rounds
 from .transcript import DuplexTranscript
 
@@ -169,8 +169,14 @@ class StackedOpenProof:
 def _ef4_encode(code: BitReversedReedSolomon, mle: torch.Tensor) -> torch.Tensor:
     """Bit-reversed encode of an EF4 message [S, 4] limb by limb (the base-field
     roots act on each coefficient) -> [n, 4]."""
-    limbs = mle.movedim(-1, 0).contiguous()  # [4, S]
-    return code.encode(limbs).movedim(0, -1).contiguous()
+    L, st = _lib.lib(), stream_handle()
+    S = mle.shape[0]
+    limbs = torch.empty((4, S), dtype=torch.int32, device=mle.device)
+    _lib.check(L.zc_ef4_limbs(ptr(mle), S, 1, ptr(limbs), st), "ef4_limbs")
+    cw = code.encode(limbs)
+    out = torch.empty((cw.shape[1], 4), dtype=torch.int32, device=mle.device)
+    _lib.check(L.zc_ef4_limbs(ptr(cw), cw.shape[1], 0, ptr(out), st), "ef4_limbs")
+    return out
 
 
 def stacked_basefold_open(smcs: SingleMatrixCommitmentScheme, code: BitReversedReedSolomon,
@@ -220,9 +226,7 @@ def stacked_basefold_open(smcs: SingleMatrixCommitmentScheme, code: BitReversedR
         t.observe_(e.reshape(-1))
     total = sum(int(rd.block.shape[0]) for rd in rounds)
     nbv = (total - 1).bit_length() if total > 1 else 0
-    chal = torch.zeros((max(nbv, 1), 4), dtype=torch.int32, device=dev)
-    if nbv:
-        chal[:nbv] = t.sample_(4 * nbv).reshape(nbv, 4)
+    chal = t.sample_(4 * nbv) if nbv else torch.empty(4, dtype=torch.int32, device=dev)
     mle = torch.empty((S, 4), dtype=torch.int32, device=dev)
     claim = torch.empty(4, dtype=torch.int32, device=dev)
     off = 0
@@ -236,9 +240,7 @@ def stacked_basefold_open(smcs: SingleMatrixCommitmentScheme, code: BitReversedR
         off += K
     # fold zone
     cw = _ef4_encode(code, mle)
-    nv = torch.zeros(1, dtype=torch.int32, device=dev)
-    nv.fill_(f.mont(v))  # a fill kernel: no host copy
-    t.observe_(nv)
+    t.observe_(full_u32(1, f.mont(v), dev))  # a fill kernel: no host copy
     zinv = torch.empty_like(zs)  # 1/z per stacking coordinate, on the device
     _lib.check(L.zc_ef4_inv(f.id, ptr(zs), ptr(zinv), v, st), "ef4_inv")
     eq = torch.empty((max(S // 2, 1), 4), dtype=torch.int32, device=dev)
