@@ -140,6 +140,13 @@ zc_status zc_rs_encode_bitrev(zc_field field, const uint32_t* coeffs, int64_t ba
                               uint32_t* out, void* workspace, size_t workspace_bytes,
                               void* stream);
 
+/* Inverse NTT (lax.ntt INTT) of `batch` rows of 2^log_k, natural order in and
+ * out: the forward transform of the row read at -i mod k, its outputs scaled
+ * by 1/k in the last pass. Workspace as zc_rs_encode with log_blowup 0. */
+zc_status zc_intt(zc_field field, const uint32_t* evals, int64_t batch, int log_k,
+                  uint32_t generator, uint32_t* out, void* workspace, size_t workspace_bytes,
+                  void* stream);
+
 /* The LDE of zc_rs_encode without any device allocation and without a
  * caller workspace: no counterpart in the reference. For callers that cannot
  * allocate device memory at call time -- a handler inside an XLA/FRX custom

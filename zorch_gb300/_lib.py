@@ -87,6 +87,7 @@ def _declare(lib: C.CDLL) -> None:
         "zc_poseidon2_permute_host": (st, [vp, vp, i64]),
         "zc_rs_encode_workspace_bytes": (sz, [i64, C.c_int, C.c_int]),
         "zc_rs_encode": (st, [st, vp, i64, C.c_int, C.c_int, u32, u32, vp, vp, sz, vp]),
+        "zc_intt": (st, [st, vp, i64, C.c_int, u32, vp, vp, sz, vp]),
         "zc_rs_encode_noalloc": (st, [st, vp, i64, C.c_int, C.c_int, u32, u32, vp, vp]),
         "zc_rs_encode_bitrev": (st, [st, vp, i64, C.c_int, C.c_int, u32, u32, vp, vp, sz, vp]),
         "zc_merkle_commit": (st, [vp, Leaves, vp, vp]),

@@ -53,15 +53,20 @@ def ntt(field, x: torch.Tensor, generator: int = 0) -> torch.Tensor:
 
 
 def intt(field, x: torch.Tensor, generator: int = 0) -> torch.Tensor:
-    """Inverse NTT over the last axis (lax.ntt INTT): (1/k) * NTT(x)[-i mod k]."""
+    """Inverse NTT over the last axis (lax.ntt INTT): (1/k) * NTT(x)[-i mod k], by
+    the forward transform of the row read in that order (zc_intt)."""
     f = field_of(field)
     k = x.shape[-1]
-    y = ntt(f, x, generator)
-    rev = torch.remainder(-torch.arange(k, device=x.device), k)
-    y = y.index_select(-1, rev).contiguous()
-    out = torch.empty_like(y)
-    _lib.check(_lib.lib().zc_scale(f.id, ptr(y), ptr(out), y.numel(), f.inv_mont(f.mont(k)),
-                                   stream_handle()), "scale")
+    if not _is_pow2(k):
+        raise ValueError(f"message_len must be a power of two, got {k}")
+    batch = x.numel() // k
+    out = torch.empty(x.shape, dtype=torch.int32, device=x.device)
+    L = _lib.lib()
+    nb = L.zc_rs_encode_workspace_bytes(batch, _log2(k), 0)
+    ws = torch.empty(max(nb // 4, 1), dtype=torch.int32, device=x.device)
+    x = x.contiguous()
+    _lib.check(L.zc_intt(f.id, ptr(x), batch, _log2(k), generator, ptr(out), ptr(ws), nb,
+                         stream_handle()), "intt")
     return out
 
 

@@ -119,7 +119,10 @@ __device__ void root_table(uint32_t* tab, int count, int log_m) {
 // The R stages of one radix-2^R group held in registers: members j at
 // positions base + j S (S = 2^lS, off = base mod S); stage r's twiddle is
 // tw[pos << (sh0 + r)] with pos = off + (j mod 2^hb) S.
-template <class F, int R>
+// LAST: the last pass of a row (S = 1, off = 0), where the butterflies with
+// jm = 0 have twiddle 1: 31 of a radix-2^5 group's 80, which then need no product
+// (2^20 x 64 at blowup 4: 1.98 -> 1.91 ms).
+template <class F, int R, bool LAST = false>
 __device__ __forceinline__ void dif_group(uint32_t (&v)[1 << R], const uint32_t* tw, int off,
                                           int lS, int sh0) {
   constexpr int G = 1 << R;
@@ -133,9 +136,13 @@ __device__ __forceinline__ void dif_group(uint32_t (&v)[1 << R], const uint32_t*
     for (int j = 0; j < G; j++) {
       if (!(j & (1 << hb))) {
         const int j2 = j | (1 << hb);
-        const uint32_t w = tw[tb + (j & ((1 << hb) - 1)) * ts];
         const uint32_t u = v[j], t = v[j2];
         v[j] = madd<F>(u, t);
+        if (LAST && (j & ((1 << hb) - 1)) == 0) {
+          v[j2] = msub<F>(u, t);
+          continue;
+        }
+        const uint32_t w = tw[tb + (j & ((1 << hb) - 1)) * ts];
         // u - t in (-p, p) feeds the signed product directly
         v[j2] = snorm<F>(smul<F>((int32_t)(u - t), (int32_t)w));
       }
@@ -165,7 +172,10 @@ __device__ __forceinline__ void dif_pass(uint32_t* a, int log_rows, int logm, in
     uint32_t v[G];
 #pragma unroll
     for (int j = 0; j < G; j++) v[j] = ar[pad(j << lS)];
-    dif_group<F, R>(v, tw, off, lS, sh0);
+    if (lS == 0)
+      dif_group<F, R, true>(v, tw, 0, 0, sh0);
+    else
+      dif_group<F, R>(v, tw, off, lS, sh0);
 #pragma unroll
     for (int j = 0; j < G; j++) ar[pad(j << lS)] = v[j];
   }
@@ -212,7 +222,6 @@ __device__ void smem_ntt_dif(uint32_t* a, int log_rows, int logm, int rs, const 
 }
 
 constexpr int kThreads = 512;
-[[maybe_unused]] constexpr int kLogThreads = 9;
 // Threads and resident CTAs per SM of the four-step passes with largest radix
 // 2^MR: the wide build's 128 registers allow 512 threads per SM.
 template <int MR>
@@ -240,7 +249,7 @@ __device__ __forceinline__ void cp_async_wait_all() {
 template <class F>
 __device__ void lde_small_body(const uint32_t* x, uint32_t* out, int log_k, int log_b,
                                uint32_t h, int64_t c, uint32_t* sm, int brev_out,
-                               int max_r = kMaxRadixLog) {
+                               int max_r = kMaxRadixLog, int rev = 0, uint32_t post = F::ONE) {
   const int k = 1 << log_k, b = 1 << log_b, log_n = log_k + log_b;
   const int rs = row_stride(k);
   uint32_t* work = sm;
@@ -250,7 +259,8 @@ __device__ void lde_small_body(const uint32_t* x, uint32_t* out, int log_k, int 
   uint32_t* wh = wl + 128;  // w_n^(128 e), e < 128
   const uint32_t* xc = x + (c << log_k);
   for (int idx = threadIdx.x; idx < (b << log_k); idx += blockDim.x)
-    cp_async4(work + (idx >> log_k) * rs + pad(idx & (k - 1)), xc + (idx & (k - 1)));
+    cp_async4(work + (idx >> log_k) * rs + pad(idx & (k - 1)),
+              xc + ((rev ? -idx : idx) & (k - 1)));
   root_table<F>(tw, k > 1 ? k / 2 : 1, log_k);
   const uint32_t nmask = (1u << log_n) - 1;  // w_n^e depends on e mod n
   for (int e = threadIdx.x; e < 128; e += blockDim.x) {
@@ -267,6 +277,7 @@ __device__ void lde_small_body(const uint32_t* x, uint32_t* out, int log_k, int 
       const int e = s * i;  // < n <= 2^14
       v = smul<F>(v, smul<F>((int32_t)wl[e & 127], (int32_t)wh[e >> 7]));
     }
+    if (post != F::ONE) v = smul<F>(v, (int32_t)post);
     *slot = snorm<F>(v);
   }
   __syncthreads();
@@ -288,59 +299,14 @@ __device__ void lde_small_body(const uint32_t* x, uint32_t* out, int log_k, int 
 template <class F>
 __global__ void __launch_bounds__(kThreads, 2) k_lde_small(const uint32_t* x, uint32_t* out,
                                                         int log_k, int log_b, uint32_t h,
-                                                        int brev_out) {
+                                                        int brev_out, int rev, uint32_t post) {
   extern __shared__ uint32_t sm[];
-  lde_small_body<F>(x, out, log_k, log_b, h, blockIdx.x, sm, brev_out);
+  lde_small_body<F>(x, out, log_k, log_b, h, blockIdx.x, sm, brev_out, kMaxRadixLog, rev, post);
 }
 
 // Pass 1 item (coset s, i1 tile, column c): the k2-point DIF NTTs down the
 // strided columns i1 of the message scaled by g_s^(i1 + k1 i2); writes the
 // untwiddled intermediate z[c][s][t2][i1] (t2 = bit-reversed position).
-// Layout: work[TI][rs] | tw[k2/2] | gi[TI].
-template <class F>
-__device__ void lde_pass1_body(const uint32_t* x, uint32_t* z, int log_k1, int log_k2, int log_b,
-                               int log_ti, uint32_t h, int s, int tile, int64_t c,
-                               uint32_t* sm, int max_r = kMaxRadixLog) {
-  const int k1 = 1 << log_k1, k2 = 1 << log_k2, TI = 1 << log_ti;
-  const int log_k = log_k1 + log_k2, log_n = log_k + log_b;
-  const int rs = row_stride(k2);
-  uint32_t* work = sm;
-  uint32_t* tw = work + TI * rs;
-  uint32_t* gi = tw + (k2 > 1 ? k2 / 2 : 1);
-  const int i1_0 = tile * TI;
-  // Thread t always owns column d = t mod TI (TI <= kThreads, both powers of
-  // two) and walks i2 = t / TI, + kThreads / TI, ...: the column offsets are
-  // loop-invariant and the row offsets step by constants.
-  const int d = threadIdx.x & (TI - 1), i2_0 = threadIdx.x >> log_ti;
-  const int di = kThreads >> log_ti;
-  uint32_t* wd = work + d * rs;
-  {
-    const uint32_t* src = x + (c << log_k) + i1_0 + d + ((int64_t)i2_0 << log_k1);
-    const int64_t sstep = (int64_t)di << log_k1;
-    for (int i2 = i2_0; i2 < k2; i2 += di, src += sstep) cp_async4(wd + pad(i2), src);
-  }
-  const uint32_t gs = mmul<F>(h, s ? omega_pow<F>(log_n, (uint32_t)s) : F::ONE);
-  const uint32_t G = mpow<F>(gs, (uint64_t)k1);
-  root_table<F>(tw, k2 > 1 ? k2 / 2 : 1, log_k2);
-  for (int i = threadIdx.x; i < TI; i += blockDim.x) gi[i] = mpow<F>(gs, (uint64_t)(i1_0 + i));
-  // word (d, i2) is scaled by gs^(i1_0 + d + k1 i2) = gi[d] G^i2: a running
-  // product per thread, G^i2_0 then times G^di per step (no table, no barriers)
-  const uint32_t g_first = mpow<F>(G, (uint64_t)i2_0), g_step = mpow<F>(G, (uint64_t)di);
-  __syncthreads();
-  cp_async_wait_all();
-  {  // each thread scales the words it loaded itself (no barrier needed)
-    int32_t fac = smul<F>((int32_t)gi[d], (int32_t)g_first);
-    for (int i2 = i2_0; i2 < k2; i2 += di) {
-      uint32_t* slot = wd + pad(i2);
-      *slot = snorm<F>(smul<F>((int32_t)*slot, fac));
-      fac = smul<F>(fac, (int32_t)g_step);
-    }
-  }
-  __syncthreads();
-  smem_ntt_dif<F>(work, log_ti, log_k2, rs, tw, max_r);
-  uint32_t* zd = z + ((c << log_b) + s) * ((int64_t)1 << log_k) + i1_0 + d;
-  for (int p = i2_0; p < k2; p += di) zd[(uint32_t)brev(p, log_k2) << log_k1] = wd[pad(p)];
-}
 
 // ---------------------------------------------------------- fused passes --
 // The four-step passes with the first radix pass fed straight from global
@@ -353,9 +319,6 @@ __device__ void lde_pass1_body(const uint32_t* x, uint32_t* z, int log_k1, int l
 // per-word cp.async copies, a separate scale loop and a separate output loop,
 // this removes one shared-memory round trip and two barrier-separated loops
 // per pass (the words, products and results are the same).
-#ifndef ZC_LDE_FUSED
-#define ZC_LDE_FUSED 1
-#endif
 
 // Balanced radix of pass q of `passes` over the stages left (h0 + 1).
 __host__ __device__ __forceinline__ int pass_radix(int h0, int passes, int q) {
@@ -373,11 +336,12 @@ __host__ __device__ __forceinline__ int first_stride_log(int logm, int max_r) {
 // k2 (the i2 index). first: the members come from x, scaled by
 // gs^(i1 + k1 i2) = gi[d] * G^off * (G^S)^j; last: the outputs go to z at the
 // bit-reversed position brev(p) << log_k1.
-template <class F, int R>
+template <class F, int R, bool REV>
 __device__ __forceinline__ void p1_pass(uint32_t* work, int rs, int log_ti, int log_k1,
-                                        int log_k2, int h0, bool first, bool last,
-                                        const uint32_t* xs, const uint32_t* gi, const uint32_t* Gt,
-                                        uint32_t GS, const uint32_t* tw, uint32_t* zd) {
+                                        int log_k2, int h0, bool first, bool last, bool unit,
+                                        const uint32_t* xc, int i1_0, const uint32_t* gi,
+                                        const uint32_t* Gt, uint32_t GS, const uint32_t* tw,
+                                        uint32_t* zd) {
   constexpr int G = 1 << R;
   const int lS = h0 - R + 1;
   const int total = 1 << (log_ti + log_k2 - R);
@@ -390,20 +354,32 @@ __device__ __forceinline__ void p1_pass(uint32_t* work, int rs, int log_ti, int 
     uint32_t* ar = work + d * rs + pad(base);
     uint32_t v[G];
     if (first) {
-      const uint32_t* src = xs + d + ((int64_t)off << log_k1);
+      const uint32_t i0 = (uint32_t)(i1_0 + d) + ((uint32_t)off << log_k1);
+      if (REV) {  // x at -i mod k
+        const uint32_t kmask = (1u << (log_k1 + log_k2)) - 1;
 #pragma unroll
-      for (int j = 0; j < G; j++) v[j] = __ldg(src + ((int64_t)j << (lS + log_k1)));
-      int32_t f = smul<F>((int32_t)gi[d], (int32_t)Gt[off]);
+        for (int j = 0; j < G; j++)
+          v[j] = __ldg(xc + ((0u - i0 - ((uint32_t)j << (lS + log_k1))) & kmask));
+      } else {
 #pragma unroll
-      for (int j = 0; j < G; j++) {
-        v[j] = snorm<F>(smul<F>((int32_t)v[j], f));
-        if (j + 1 < G) f = smul<F>(f, (int32_t)GS);
+        for (int j = 0; j < G; j++) v[j] = __ldg(xc + i0 + ((int64_t)j << (lS + log_k1)));
+      }
+      if (!unit) {
+        int32_t f = smul<F>((int32_t)gi[d], (int32_t)Gt[off]);
+#pragma unroll
+        for (int j = 0; j < G; j++) {
+          v[j] = snorm<F>(smul<F>((int32_t)v[j], f));
+          if (j + 1 < G) f = smul<F>(f, (int32_t)GS);
+        }
       }
     } else {
 #pragma unroll
       for (int j = 0; j < G; j++) v[j] = ar[pad(j << lS)];
     }
-    dif_group<F, R>(v, tw, off, lS, sh0);
+    if (last)
+      dif_group<F, R, true>(v, tw, 0, 0, sh0);
+    else
+      dif_group<F, R>(v, tw, off, lS, sh0);
     if (last) {  // lS == 0: members are the positions base + j, base = blk 2^R, so
                  // brev(base + j) = brev(base) + brev_R(j) 2^(log_k2 - R)
       uint32_t* zp = zd + d + ((uint32_t)brev(base, log_k2) << log_k1);
@@ -420,7 +396,8 @@ __device__ __forceinline__ void p1_pass(uint32_t* work, int rs, int log_ti, int 
 // Pass-1 item with fused load and store. Layout: work[TI][rs] | tw[k2/2] |
 // gi[TI] | Gt[S] (S = the first pass's member stride). MR: the largest radix
 // compiled in (max_r <= MR).
-template <class F, int MR = kMaxRadixLog>
+// REV: the message is read at -i mod k (an inverse transform's input order).
+template <class F, int MR = kMaxRadixLog, bool REV = false>
 __device__ void lde_pass1_fused(const uint32_t* x, uint32_t* z, int log_k1, int log_k2, int log_b,
                                 int log_ti, uint32_t h, int s, int tile, int64_t c, uint32_t* sm,
                                 int max_r) {
@@ -439,8 +416,9 @@ __device__ void lde_pass1_fused(const uint32_t* x, uint32_t* z, int log_k1, int 
   for (int i = threadIdx.x; i < TI; i += blockDim.x) gi[i] = mpow<F>(gs, (uint64_t)(i1_0 + i));
   for (int i = threadIdx.x; i < (1 << lS0); i += blockDim.x) Gt[i] = mpow<F>(G, (uint64_t)i);
   const uint32_t GS = mpow<F>(G, (uint64_t)1 << lS0);
+  const bool unit = gs == F::ONE;  // coset 1: nothing to scale
   __syncthreads();
-  const uint32_t* xs = x + (c << log_k) + i1_0;
+  const uint32_t* xc = x + (c << log_k);
   uint32_t* zd = z + ((c << log_b) + s) * ((int64_t)1 << log_k) + i1_0;
   const int passes = pass_count(log_k2, max_r);
   int h0 = log_k2 - 1;
@@ -448,11 +426,11 @@ __device__ void lde_pass1_fused(const uint32_t* x, uint32_t* z, int log_k1, int 
     const int R = pass_radix(h0, passes, q);
     const bool first = q == 0, last = q == passes - 1;
     switch (R) {
-      case 5: if constexpr (MR >= 5) p1_pass<F, 5>(work, rs, log_ti, log_k1, log_k2, h0, first, last, xs, gi, Gt, GS, tw, zd); break;
-      case 4: p1_pass<F, 4>(work, rs, log_ti, log_k1, log_k2, h0, first, last, xs, gi, Gt, GS, tw, zd); break;
-      case 3: p1_pass<F, 3>(work, rs, log_ti, log_k1, log_k2, h0, first, last, xs, gi, Gt, GS, tw, zd); break;
-      case 2: p1_pass<F, 2>(work, rs, log_ti, log_k1, log_k2, h0, first, last, xs, gi, Gt, GS, tw, zd); break;
-      default: p1_pass<F, 1>(work, rs, log_ti, log_k1, log_k2, h0, first, last, xs, gi, Gt, GS, tw, zd); break;
+      case 5: if constexpr (MR >= 5) p1_pass<F, 5, REV>(work, rs, log_ti, log_k1, log_k2, h0, first, last, unit, xc, i1_0, gi, Gt, GS, tw, zd); break;
+      case 4: p1_pass<F, 4, REV>(work, rs, log_ti, log_k1, log_k2, h0, first, last, unit, xc, i1_0, gi, Gt, GS, tw, zd); break;
+      case 3: p1_pass<F, 3, REV>(work, rs, log_ti, log_k1, log_k2, h0, first, last, unit, xc, i1_0, gi, Gt, GS, tw, zd); break;
+      case 2: p1_pass<F, 2, REV>(work, rs, log_ti, log_k1, log_k2, h0, first, last, unit, xc, i1_0, gi, Gt, GS, tw, zd); break;
+      default: p1_pass<F, 1, REV>(work, rs, log_ti, log_k1, log_k2, h0, first, last, unit, xc, i1_0, gi, Gt, GS, tw, zd); break;
     }
     if (!last) __syncthreads();
     h0 -= R;
@@ -467,7 +445,7 @@ template <class F, int R>
 __device__ __forceinline__ void p2_first(uint32_t* work, int rs, int log_b, int log_tt, int log_k1,
                                          int log_k, int t2_0, const uint32_t* zc_,
                                          const uint32_t* tw, bool last, uint32_t* oc,
-                                         int log_k2, int brev_out) {
+                                         int log_k2, int brev_out, uint32_t post) {
   constexpr int G = 1 << R;
   const int h0 = log_k1 - 1, lS = h0 - R + 1;
   const int total = 1 << (log_tt + lS);
@@ -477,7 +455,7 @@ __device__ __forceinline__ void p2_first(uint32_t* work, int rs, int log_b, int 
     const int off = it & ((1 << lS) - 1), dt = it >> lS;
     const uint32_t t = (uint32_t)(t2_0 + dt);
     int32_t f[G];
-    f[0] = (int32_t)omega_pow<F>(log_k, (t * (uint32_t)off) & kmask);
+    f[0] = (int32_t)mmul<F>(omega_pow<F>(log_k, (t * (uint32_t)off) & kmask), post);
     const int32_t step = (int32_t)omega_pow<F>(log_k, (t << lS) & kmask);
 #pragma unroll
     for (int j = 1; j < G; j++) f[j] = smul<F>(f[j - 1], step);
@@ -488,7 +466,10 @@ __device__ __forceinline__ void p2_first(uint32_t* work, int rs, int log_b, int 
       for (int j = 0; j < G; j++) v[j] = __ldg(src + (j << lS));
 #pragma unroll
       for (int j = 0; j < G; j++) v[j] = snorm<F>(smul<F>((int32_t)v[j], f[j]));
-      dif_group<F, R>(v, tw, off, lS, 0);
+      if (last)
+        dif_group<F, R, true>(v, tw, 0, 0, 0);
+      else
+        dif_group<F, R>(v, tw, off, lS, 0);
       if (last) {  // a single pass (k1 <= 16): off == 0, positions j
 #pragma unroll
         for (int j = 0; j < G; j++) {
@@ -526,7 +507,7 @@ __device__ __forceinline__ void p2_last(uint32_t* work, int rs, int log_b, int l
     uint32_t v[G];
 #pragma unroll
     for (int j = 0; j < G; j++) v[j] = ar[pad(j)];
-    dif_group<F, R>(v, tw, 0, 0, sh0);
+    dif_group<F, R, true>(v, tw, 0, 0, sh0);
     const int t = t2_0 + dt;
     if (brev_out) {
       uint32_t* orow = oc + ((int64_t)brev(s, log_b) << log_k) +
@@ -544,11 +525,12 @@ __device__ __forceinline__ void p2_last(uint32_t* work, int rs, int log_b, int l
   }
 }
 
-// Pass-2 item with fused load and store. Layout: work[b*TT][rs] | tw[k1/2].
+// Pass-2 item with fused load and store; every output is scaled by `post`.
+// Layout: work[b*TT][rs] | tw[k1/2].
 template <class F, int MR = kMaxRadixLog>
 __device__ void lde_pass2_fused(const uint32_t* z, uint32_t* out, int log_k1, int log_k2,
                                 int log_b, int log_tt, int tile, int64_t c, uint32_t* sm,
-                                int brev_out, int max_r) {
+                                int brev_out, int max_r, uint32_t post = F::ONE) {
   const int k1 = 1 << log_k1;
   const int log_k = log_k1 + log_k2, log_n = log_k + log_b;
   const int log_rows = log_b + log_tt;
@@ -571,11 +553,11 @@ __device__ void lde_pass2_fused(const uint32_t* z, uint32_t* out, int log_k1, in
     const bool first = q == 0, last = q == passes - 1;
     if (first) {
       switch (R) {
-        case 5: if constexpr (MR >= 5) p2_first<F, 5>(work, rs, log_b, log_tt, log_k1, log_k, t2_0, zc_, tw, last, oc, log_k2, brev_out); break;
-        case 4: p2_first<F, 4>(work, rs, log_b, log_tt, log_k1, log_k, t2_0, zc_, tw, last, oc, log_k2, brev_out); break;
-        case 3: p2_first<F, 3>(work, rs, log_b, log_tt, log_k1, log_k, t2_0, zc_, tw, last, oc, log_k2, brev_out); break;
-        case 2: p2_first<F, 2>(work, rs, log_b, log_tt, log_k1, log_k, t2_0, zc_, tw, last, oc, log_k2, brev_out); break;
-        default: p2_first<F, 1>(work, rs, log_b, log_tt, log_k1, log_k, t2_0, zc_, tw, last, oc, log_k2, brev_out); break;
+        case 5: if constexpr (MR >= 5) p2_first<F, 5>(work, rs, log_b, log_tt, log_k1, log_k, t2_0, zc_, tw, last, oc, log_k2, brev_out, post); break;
+        case 4: p2_first<F, 4>(work, rs, log_b, log_tt, log_k1, log_k, t2_0, zc_, tw, last, oc, log_k2, brev_out, post); break;
+        case 3: p2_first<F, 3>(work, rs, log_b, log_tt, log_k1, log_k, t2_0, zc_, tw, last, oc, log_k2, brev_out, post); break;
+        case 2: p2_first<F, 2>(work, rs, log_b, log_tt, log_k1, log_k, t2_0, zc_, tw, last, oc, log_k2, brev_out, post); break;
+        default: p2_first<F, 1>(work, rs, log_b, log_tt, log_k1, log_k, t2_0, zc_, tw, last, oc, log_k2, brev_out, post); break;
       }
     } else if (last) {
       switch (R) {
@@ -599,18 +581,13 @@ __device__ void lde_pass2_fused(const uint32_t* z, uint32_t* out, int log_k1, in
   }
 }
 
-template <class F, int MR = kMaxRadixLog>
+template <class F, int MR = kMaxRadixLog, bool REV = false>
 __global__ void __launch_bounds__(lde_threads<MR>(), lde_min_blocks<MR>()) k_lde_pass1(const uint32_t* x, uint32_t* z, int log_k1,
                                                         int log_k2, int log_b, int log_ti,
                                                         uint32_t h) {
   extern __shared__ uint32_t sm[];
-#if ZC_LDE_FUSED
-  lde_pass1_fused<F, MR>(x, z, log_k1, log_k2, log_b, log_ti, h, blockIdx.x, blockIdx.y,
-                         blockIdx.z, sm, MR);
-#else
-  lde_pass1_body<F>(x, z, log_k1, log_k2, log_b, log_ti, h, blockIdx.x, blockIdx.y, blockIdx.z,
-                    sm);
-#endif
+  lde_pass1_fused<F, MR, REV>(x, z, log_k1, log_k2, log_b, log_ti, h, blockIdx.x, blockIdx.y,
+                              blockIdx.z, sm, MR);
 }
 
 // Pass 2 item (t2 tile, column c): rows (s, t2) for all b cosets and TT
@@ -618,91 +595,14 @@ __global__ void __launch_bounds__(lde_threads<MR>(), lde_min_blocks<MR>()) k_lde
 // k1-point DIF NTT, and written to out[b (t2 + k2 t1) + s] (t1 = bit-reversed
 // position) in contiguous runs of b*TT words -- or, for a bit-reversed
 // codeword, row (s, t2) to the k1 contiguous words at brev_b(s) k + brev_k2(t2) k1.
-// Layout: work[b*TT][rs] | tw[k1/2].
-template <class F>
-__device__ void lde_pass2_body(const uint32_t* z, uint32_t* out, int log_k1, int log_k2,
-                               int log_b, int log_tt, int tile, int64_t c, uint32_t* sm,
-                               int brev_out, int max_r = kMaxRadixLog) {
-  const int k1 = 1 << log_k1, TT = 1 << log_tt;
-  const int log_k = log_k1 + log_k2, log_n = log_k + log_b;
-  const int log_rows = log_b + log_tt;
-  const int rs = row_stride(k1);
-  uint32_t* work = sm;
-  uint32_t* tw = work + (rs << log_rows);
-  const int t2_0 = tile * TT;
-  const uint32_t* zc_ = z + (c << log_n);
-  // Thread t owns positions i1 = t mod tpr, + tpr, ... (tpr = min(k1,
-  // kThreads) threads per row, consecutive threads on consecutive words) of
-  // rows dt = t / tpr, + dt_step, ... of every coset s; it loads and scales
-  // exactly these words, so the scale needs no barrier after the loads.
-  const int lt = log_k1 < kLogThreads ? log_k1 : kLogThreads;
-  const int tpr = 1 << lt;
-  const int i1_0 = threadIdx.x & (tpr - 1);
-  const int dt_0 = threadIdx.x >> lt, dt_step = kThreads >> lt;
-  const int b = 1 << log_b;
-  for (int i1 = i1_0; i1 < k1; i1 += tpr)
-    for (int s = 0; s < b; s++) {
-      uint32_t* wp = work + (s << log_tt) * rs + pad(i1);
-      const uint32_t* zp = zc_ + ((int64_t)s << log_k) + ((int64_t)t2_0 << log_k1) + i1;
-      for (int dt = dt_0; dt < TT; dt += dt_step)
-        cp_async4(wp + dt * rs, zp + ((uint32_t)dt << log_k1));
-    }
-  root_table<F>(tw, k1 > 1 ? k1 / 2 : 1, log_k1);
-  // word (s, dt, i1) is scaled by w_k^((t2_0 + dt) i1), the same for every
-  // coset s: a running product over this thread's rows, stepping by
-  // w_k^(dt_step i1)
-  const uint32_t kmask = (1u << log_k) - 1;
-  __syncthreads();
-  cp_async_wait_all();
-  for (int i1 = i1_0; i1 < k1; i1 += tpr) {
-    int32_t fac = (int32_t)omega_pow<F>(log_k, ((uint32_t)(t2_0 + dt_0) * (uint32_t)i1) & kmask);
-    const int32_t step = (int32_t)omega_pow<F>(log_k, ((uint32_t)dt_step * (uint32_t)i1) & kmask);
-    for (int dt = dt_0; dt < TT; dt += dt_step) {
-      uint32_t* wp = work + dt * rs + pad(i1);
-      for (int s = 0; s < b; s++) {
-        uint32_t* slot = wp + (s << log_tt) * rs;
-        *slot = snorm<F>(smul<F>((int32_t)*slot, fac));
-      }
-      fac = smul<F>(fac, step);
-    }
-  }
-  __syncthreads();
-  smem_ntt_dif<F>(work, log_rows, log_k1, rs, tw, max_r);
-  uint32_t* oc = out + (c << log_n);
-  const int rows = 1 << log_rows;
-  if (brev_out) {  // row (s, t2) -> the k1 contiguous words at brev_b(s) k + brev_k2(t2) k1
-    for (int s = 0; s < b; s++)
-      for (int dt = dt_0; dt < TT; dt += dt_step) {
-        const uint32_t* wr = work + ((s << log_tt) + dt) * rs;
-        uint32_t* orow = oc + ((int64_t)brev(s, log_b) << log_k) +
-                         ((int64_t)brev(t2_0 + dt, log_k2) << log_k1);
-        for (int p = i1_0; p < k1; p += tpr) orow[p] = wr[pad(p)];
-      }
-    return;
-  }
-  {  // out[b (t2 + k2 t1) + s]: thread t owns row (s, dt) = t mod rows and walks
-     // the positions p = t / rows, + kThreads / rows, ... (rows <= kThreads)
-    const int ri = threadIdx.x & (rows - 1);
-    const int s = ri & ((1 << log_b) - 1), dt = ri >> log_b;
-    const uint32_t* wr = work + ((s << log_tt) + dt) * rs;
-    uint32_t* ob = oc + ((int64_t)(t2_0 + dt) << log_b) + s;
-    const int sh = log_k2 + log_b;
-    for (int p = threadIdx.x >> log_rows; p < k1; p += kThreads >> log_rows)
-      ob[(uint32_t)brev(p, log_k1) << sh] = wr[pad(p)];  // offset < n <= 2^30
-  }
-}
-
 template <class F, int MR = kMaxRadixLog>
 __global__ void __launch_bounds__(lde_threads<MR>(), lde_min_blocks<MR>()) k_lde_pass2(const uint32_t* z, uint32_t* out,
                                                         int log_k1, int log_k2, int log_b,
-                                                        int log_tt, int brev_out) {
+                                                        int log_tt, int brev_out,
+                                                        uint32_t post) {
   extern __shared__ uint32_t sm[];
-#if ZC_LDE_FUSED
   lde_pass2_fused<F, MR>(z, out, log_k1, log_k2, log_b, log_tt, blockIdx.x, blockIdx.y, sm,
-                         brev_out, MR);
-#else
-  lde_pass2_body<F>(z, out, log_k1, log_k2, log_b, log_tt, blockIdx.x, blockIdx.y, sm, brev_out);
-#endif
+                         brev_out, MR, post);
 }
 
 struct LdePlan {
@@ -735,9 +635,7 @@ inline LdePlan plan_lde(int log_k, int log_b, int tile_log = 0, int max_r = kMax
   const int k1 = 1 << p.log_k1, k2 = 1 << p.log_k2;
   p.smem1 = 4 * ((size_t)(1 << p.log_ti) * row_stride(k2) + (k2 > 1 ? k2 / 2 : 1) +
                  (1 << p.log_ti));
-#if ZC_LDE_FUSED
   p.smem1 += (size_t)4 << first_stride_log(p.log_k2, max_r);  // the G^off table
-#endif
   p.smem2 = 4 * ((size_t)(b << p.log_tt) * row_stride(k1) + (k1 > 1 ? k1 / 2 : 1));
   return p;
 }
@@ -747,7 +645,6 @@ inline LdePlan plan_lde(int log_k, int log_b, int tile_log = 0, int max_r = kMax
 // one 512-thread CTA per SM: 2.10 ms against 2.23 ms for the radix-2^4 form
 // on the GB300).
 inline bool lde_wide(int64_t batch, int log_n) {
-#if ZC_LDE_FUSED
   static const int sms = [] {
     int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -757,27 +654,24 @@ inline bool lde_wide(int64_t batch, int log_n) {
   }();
   const int64_t tiles = log_n >= kWideTileLog ? batch << (log_n - kWideTileLog) : 0;
   return tiles >= 2 * (int64_t)sms;
-#else
-  (void)batch;
-  (void)log_n;
-  return false;
-#endif
 }
 
 template <class F, int MR>
 zc_status lde_four_step(const uint32_t* x, int64_t batch, int log_k, int log_b, uint32_t h,
                         uint32_t* out, void* ws, size_t ws_bytes, cudaStream_t st, int brev_out,
-                        const LdePlan& p);
+                        const LdePlan& p, int rev, uint32_t post);
 
+// rev: the message is read at -i mod k; every output is scaled by post (an
+// inverse transform: rev, post = 1/k).
 template <class F>
 zc_status lde_launch(const uint32_t* x, int64_t batch, int log_k, int log_b, uint32_t h,
                      uint32_t* out, void* ws, size_t ws_bytes, cudaStream_t st,
-                     int brev_out = 0) {
+                     int brev_out = 0, int rev = 0, uint32_t post = F::ONE) {
   if (!plan_lde(log_k, log_b).small && lde_wide(batch, log_k + log_b)) {
     const LdePlan pw = plan_lde(log_k, log_b, kWideTileLog, kWideRadixLog);
     if (pw.smem1 <= 227 * 1024 && pw.smem2 <= 227 * 1024)
       return lde_four_step<F, kWideRadixLog>(x, batch, log_k, log_b, h, out, ws, ws_bytes, st,
-                                             brev_out, pw);
+                                             brev_out, pw, rev, post);
   }
   const LdePlan p = plan_lde(log_k, log_b);
   const int log_n = log_k + log_b;
@@ -793,20 +687,20 @@ zc_status lde_launch(const uint32_t* x, int64_t batch, int log_k, int log_b, uin
     for (int64_t c0 = 0; c0 < batch; c0 += 0x7fffffff) {
       const int64_t cols = batch - c0 < 0x7fffffff ? batch - c0 : 0x7fffffff;
       k_lde_small<F><<<(unsigned)cols, kThreads, p.smem_small, st>>>(
-          x + (c0 << log_k), out + (c0 << log_n), log_k, log_b, h, brev_out);
+          x + (c0 << log_k), out + (c0 << log_n), log_k, log_b, h, brev_out, rev, post);
       ZC_TRY(launch_check());
     }
     return ZC_OK;
   }
   return lde_four_step<F, kMaxRadixLog>(x, batch, log_k, log_b, h, out, ws, ws_bytes, st,
-                                        brev_out, p);
+                                        brev_out, p, rev, post);
 }
 
 // The two four-step passes over column chunks that fit the workspace.
 template <class F, int MR>
 zc_status lde_four_step(const uint32_t* x, int64_t batch, int log_k, int log_b, uint32_t h,
                         uint32_t* out, void* ws, size_t ws_bytes, cudaStream_t st, int brev_out,
-                        const LdePlan& p) {
+                        const LdePlan& p, int rev, uint32_t post) {
   const int log_n = log_k + log_b;
   const size_t col_bytes = (size_t)4 << log_n;
   if (!ws || ws_bytes < col_bytes) {
@@ -817,21 +711,21 @@ zc_status lde_four_step(const uint32_t* x, int64_t batch, int log_k, int log_b, 
   int64_t chunk = (int64_t)(ws_bytes / col_bytes);
   if (chunk > 65535) chunk = 65535;
   if (chunk > batch) chunk = batch;
-  ZC_CUDA(cudaFuncSetAttribute(k_lde_pass1<F, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)p.smem1));
+  const auto pass1 = rev ? k_lde_pass1<F, MR, true> : k_lde_pass1<F, MR, false>;
+  ZC_CUDA(cudaFuncSetAttribute(pass1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem1));
   ZC_CUDA(cudaFuncSetAttribute(k_lde_pass2<F, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)p.smem2));
   uint32_t* z = (uint32_t*)ws;
   for (int64_t c0 = 0; c0 < batch; c0 += chunk) {
     const int64_t cols = batch - c0 < chunk ? batch - c0 : chunk;
     dim3 g1(1u << log_b, 1u << (p.log_k1 - p.log_ti), (unsigned)cols);
-    k_lde_pass1<F, MR><<<g1, lde_threads<MR>(), p.smem1, st>>>(x + (c0 << log_k), z, p.log_k1,
-                                                               p.log_k2, log_b, p.log_ti, h);
+    pass1<<<g1, lde_threads<MR>(), p.smem1, st>>>(x + (c0 << log_k), z, p.log_k1, p.log_k2, log_b,
+                                                  p.log_ti, h);
     ZC_TRY(launch_check());
     dim3 g2(1u << (p.log_k2 - p.log_tt), (unsigned)cols);
     k_lde_pass2<F, MR><<<g2, lde_threads<MR>(), p.smem2, st>>>(z, out + (c0 << log_n), p.log_k1,
                                                                p.log_k2, log_b, p.log_tt,
-                                                               brev_out);
+                                                               brev_out, post);
     ZC_TRY(launch_check());
   }
   return ZC_OK;
@@ -892,23 +786,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_lde_batch(const __grid_constant
       const int64_t per_col = (int64_t)b << (J.log_k1 - J.log_ti);
       const int64_t c = local / per_col;
       const int r = (int)(local - c * per_col);
-#if ZC_LDE_FUSED
       lde_pass1_fused<F>(J.x, J.z, J.log_k1, J.log_k2, J.log_b, J.log_ti, J.h, r & (b - 1),
                          r >> J.log_b, c, sm, J.max_r);
-#else
-      lde_pass1_body<F>(J.x, J.z, J.log_k1, J.log_k2, J.log_b, J.log_ti, J.h, r & (b - 1),
-                        r >> J.log_b, c, sm, J.max_r);
-#endif
     } else {
       const int64_t tiles = (int64_t)1 << (J.log_k2 - J.log_tt);
       const int64_t c = local / tiles;
-#if ZC_LDE_FUSED
       lde_pass2_fused<F>(J.z, J.out, J.log_k1, J.log_k2, J.log_b, J.log_tt,
                          (int)(local - c * tiles), c, sm, J.brev_out, J.max_r);
-#else
-      lde_pass2_body<F>(J.z, J.out, J.log_k1, J.log_k2, J.log_b, J.log_tt,
-                        (int)(local - c * tiles), c, sm, J.brev_out, J.max_r);
-#endif
     }
     __syncthreads();  // the item's shared memory is free again
   }
@@ -1102,6 +986,27 @@ zc_status zc_rs_encode_bitrev(zc_field field, const uint32_t* coeffs, int64_t ba
                               void* stream) {
   return rs_encode(field, coeffs, batch, log_k, log_blowup, shift_mont, generator, out,
                    workspace, workspace_bytes, stream, 1);
+}
+
+zc_status zc_intt(zc_field field, const uint32_t* evals, int64_t batch, int log_k,
+                  uint32_t generator, uint32_t* out, void* workspace, size_t workspace_bytes,
+                  void* stream) {
+  if (!evals || !out || batch < 0 || log_k < 0) return ZC_BAD_ARG;
+  if (batch == 0) return ZC_OK;
+  return with_field(field, [&](auto f) -> zc_status {
+    using F = decltype(f);
+    if (log_k > F::TWO_ADICITY || log_k > 24) {
+      set_error("transform size exceeds the supported two-adic range");
+      return ZC_BAD_SHAPE;
+    }
+    if (generator != 0 && generator != F::GEN) {
+      set_error("only the field's canonical generator is built");
+      return ZC_UNSUPPORTED;
+    }
+    ZC_TRY(ensure_init());
+    return lde_launch<F>(evals, batch, log_k, 0, F::ONE, out, workspace, workspace_bytes,
+                         (cudaStream_t)stream, 0, 1, mpow<F>(F::INV2, (uint64_t)log_k));
+  });
 }
 
 zc_status zc_rs_encode_noalloc(zc_field field, const uint32_t* coeffs, int64_t batch, int log_k,
