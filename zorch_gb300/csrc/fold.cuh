@@ -2,6 +2,7 @@
 // (zc_fold.cu) and the bit-reversed unit (zc_fold_bitrev.cu), which compile
 // in parallel.
 #pragma once
+#include "rounds.cuh"
 #include "tree.cuh"
 
 namespace zc {
@@ -122,7 +123,7 @@ template <class K, int LI, int LB, bool BR>
 zc_status fold_commit_launch(const uint32_t* cw, int64_t n, const uint32_t* beta,
                              uint32_t shift_mont, uint32_t generator, uint32_t* out,
                              uint32_t* layers, const P2Params* rt, cudaStream_t st,
-                             RootHop hop) {
+                             const RoundHop& hop) {
   using F = typename K::F;
   FoldScalars<F> fs;
   ZC_TRY(fold_scalars<F>(n, shift_mont, generator, &fs));
@@ -148,7 +149,7 @@ template <bool BR>
 zc_status fold_commit_any(const zc_poseidon2* p, const uint32_t* cw, int64_t n, int ef_in,
                           const uint32_t* beta, int ef_beta, uint32_t shift_mont,
                           uint32_t generator, uint32_t* out, uint32_t* layers, cudaStream_t st,
-                          RootHop hop = RootHop{nullptr, nullptr, 0}) {
+                          const RoundHop& hop = RoundHop{}) {
   return with_perm(p, [&](auto k, const P2Params* rt) {
     using K = decltype(k);
     if (ef_in && ef_beta)
@@ -164,11 +165,5 @@ zc_status fold_commit_any(const zc_poseidon2* p, const uint32_t* cw, int64_t n, 
                                            st, hop);
   });
 }
-
-// The bit-reversed fused fold-and-commit (zc_fold_bitrev.cu).
-zc_status fold_commit_bitrev(const zc_poseidon2* p, const uint32_t* cw, int64_t n, int ef_in,
-                             const uint32_t* beta, int ef_beta, uint32_t shift_mont,
-                             uint32_t generator, uint32_t* out, uint32_t* layers, cudaStream_t st,
-                             RootHop hop);
 
 }  // namespace zc

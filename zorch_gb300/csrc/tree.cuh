@@ -16,38 +16,12 @@
 
 #include <type_traits>
 
-#include "duplex.cuh"
 #include "internal.cuh"
+#include "roundhop.cuh"
 
 namespace zc {
 
 constexpr int kMaxT = 256;
-
-// A transcript hop run by the CTA that computes a tree's root, in the same
-// launch: observe the 8 root words, squeeze n words -- the observe(root) +
-// sample(beta) a pre-fold round makes right after committing its layer
-// (zorch/pcs/fold.py:106-113). state: the 34-word packed duplex state, read
-// and advanced in place; nullptr: no hop.
-struct RootHop {
-  uint32_t* state;
-  uint32_t* chal;
-  int n;
-};
-
-// One full warp (all 32 lanes: half-warp permutations shuffle across it).
-template <class K>
-__device__ __forceinline__ void root_hop(const RootHop hop, const uint32_t* root,
-                                         const P2Params* hp) {
-  const CallPerm<K> perm{hp};
-  LaneDuplex t;
-  t.load(hop.state);
-  t.observe(root, 8, perm);
-  for (int i = 0; i < hop.n; i++) {
-    const uint32_t w = t.sample(perm);
-    if (threadIdx.x == 0) hop.chal[i] = w;
-  }
-  t.store(hop.state);
-}
 
 // Leaf p = concat over q < G of base[q*gs + p*g .. +g] (zc_leaves).
 struct LayoutLeaf {
@@ -262,8 +236,7 @@ struct FoldLeaf {
 // half-warps above).
 constexpr int kSubT = 128;
 // Largest number of nodes per fused-subtree CTA (k_subtree) at its first
-// level; its threads: 4 per node (a quarter-warp permutation per parent), at
-// least a warp.
+// level.
 constexpr int kSubCap = 256;
 
 // The tree driver's shape: levels with more than `levelwise_min` nodes run one
@@ -293,9 +266,14 @@ inline const TreeShape& tree_shape() {
   return shape;
 }
 
+// Threads of a subtree CTA of T first-level nodes: a quarter-warp each, at least
+// a warp and at most kSubThreads (so the permutations keep their registers: at
+// most 128 CTAs are launched at the default shape, so one per SM does). A hop's
+// warp comes on top.
+constexpr int kSubThreads = 512;
 inline int subtree_threads(int T) {
-  const int t = 4 * T > 32 ? 4 * T : 32;
-  return t < 1024 ? t : 1024;
+  const int t = 4 * T < kSubThreads ? 4 * T : kSubThreads;
+  return t > 32 ? t : 32;
 }
 
 // The tree kernels' permutations for the provider K, inlined (out of line, as
@@ -324,16 +302,16 @@ constexpr int kHalfMaxWidth = 16;
 // One level of a subtree: parent i (< width) = compress(children 2i, 2i+1)
 // read from the digest slots `src` ([node][8 words], 16-byte aligned),
 // written to the `dst` slots and to the tree's level at `lay`. Wider levels run
-// on quarter-warps, Q = blockDim/4 parents a round; narrow ones on half-warps,
+// on quarter-warps, Q = W/4 parents a round; narrow ones on half-warps,
 // whose permutation has the shorter dependency chain. A warp with no parent in
 // a round skips it (a warp-uniform branch: the shuffles need every lane of a
-// running warp).
+// running warp). W: the threads (whole warps) that work on the tree.
 template <class K>
 __device__ __forceinline__ void subtree_level(const uint32_t* src, uint32_t* dst, uint32_t* lay,
-                                              int width, const P2Params* hp) {
+                                              int width, int W, const P2Params* hp) {
   const int t = threadIdx.x;
-  if (width > kHalfMaxWidth || width > (int)(blockDim.x >> 4)) {
-    const int q = t & 3, Q = blockDim.x >> 2;  // lane q holds words 4q .. 4q+3
+  if (width > kHalfMaxWidth || width > (W >> 4)) {
+    const int q = t & 3, Q = W >> 2;  // lane q holds words 4q .. 4q+3
     for (int r = 0; r < width; r += Q) {
       if (r + 8 * (t >> 5) >= width) continue;
       const int node = r + (t >> 2);
@@ -349,7 +327,7 @@ __device__ __forceinline__ void subtree_level(const uint32_t* src, uint32_t* dst
     }
     return;
   }
-  // half-warps (one round: width <= blockDim/16): lane l holds word l
+  // half-warps (one round: width <= W/16): lane l holds word l
   const int l = t & 15, node = t >> 4;
   if (2 * (t >> 5) >= width) return;
   const bool on = node < width;
@@ -361,27 +339,45 @@ __device__ __forceinline__ void subtree_level(const uint32_t* src, uint32_t* dst
   }
 }
 
-// One subtree of T first-level nodes per CTA (blockDim = subtree_threads(T)):
+// One subtree of T first-level nodes per CTA:
 // the first level is T leaf digests (a quarter-warp each: the chain of a
 // thread's permutation is 3x as long; for NodeLeaf, stored children
 // compressed), then every level up to the subtree root is compressed out of
 // ping-pong shared-memory slots (subtree_level), each level written to
-// `layers`.
-template <class K, class Leaf>
-__global__ void __launch_bounds__(1024) k_subtree(Leaf leaf, uint32_t* layers, int64_t L,
+// `layers`. A launch that ends at the root can run the layer's transcript step
+// as well (hop): one warp more than the tree's W threads does what does not
+// need the root -- the sumcheck message, its observe, SP1's separator -- beside
+// the levels, and the rest once the root stands. As a launch of its own the step
+// came 2 us after the root and took 4 to 8 (Basefold open of 2^20 x 8 with it:
+// 2.19 ms, without 2.08). Without a hop the kernel is built without its code (a
+// commit of 2^16: 111 us against 115). Barrier 1 is the tree's, 2 the root's;
+// every warp of the tree reaches both.
+template <class K, class Leaf, bool HOP>
+__global__ void __launch_bounds__(kSubThreads + 32, 1) k_subtree(Leaf leaf, uint32_t* layers, int64_t L,
                                                        int l0, int T, const P2Params* rt,
-                                                       RootHop hop) {
+                                                       const RoundHop hop) {
   __shared__ P2Params s_rt;
   __shared__ __align__(16) uint32_t sm[2][8 * kSubCap];  // [node][word] digest slots
   KIn<K>::make(rt, &s_rt);
   const P2Params* hp = KIn<K>::half(rt, &s_rt);
   const int t = threadIdx.x;
+  const int W = blockDim.x - (HOP ? 32 : 0);
+  if constexpr (HOP) {
+    if (t >= W) {  // the hop's warp
+      __shared__ uint32_t vals[16];
+      HopWarp<K> side;
+      side.begin(hop, vals, hp);
+      asm volatile("bar.sync 2, %0;" ::"r"((int)blockDim.x) : "memory");
+      side.end(hop, vals, sm[(31 - __clz(T)) & 1], hp);
+      return;
+    }
+  }
   const int64_t base = (int64_t)blockIdx.x * T;
   uint32_t* lay0 = layers + 8 * (level_offset(L, l0) + base);
   if constexpr (std::is_same<Leaf, NodeLeaf>::value) {
-    subtree_level<K>(leaf.in + 16 * base, sm[0], lay0, T, hp);
+    subtree_level<K>(leaf.in + 16 * base, sm[0], lay0, T, W, hp);
   } else {
-    const int q = t & 3, Q = blockDim.x >> 2;
+    const int q = t & 3, Q = W >> 2;
     const auto perm = [&](uint32_t (&x)[4]) { quarter_perm_k<K>(x, hp); };
     for (int r = 0; r < T; r += Q) {
       if (r + 8 * (t >> 5) >= T) continue;  // warp-uniform
@@ -398,17 +394,19 @@ __global__ void __launch_bounds__(1024) k_subtree(Leaf leaf, uint32_t* layers, i
   }
   int cur = 0, lvl = l0, width = T;
   while (width > 1) {
-    __syncthreads();
+    if constexpr (HOP)
+      asm volatile("bar.sync 1, %0;" ::"r"(W) : "memory");  // the tree's warps
+    else
+      __syncthreads();
     width >>= 1;
     lvl++;
     subtree_level<K>(sm[cur], sm[cur ^ 1],
-                     layers + 8 * (level_offset(L, lvl) + (int64_t)blockIdx.x * width), width, hp);
+                     layers + 8 * (level_offset(L, lvl) + (int64_t)blockIdx.x * width), width, W,
+                     hp);
     cur ^= 1;
   }
-  if (hop.state) {  // passed only to a one-CTA launch that ends at the root
-    __syncthreads();
-    if (threadIdx.x < 32) root_hop<K>(hop, sm[cur], hp);
-  }
+  if constexpr (HOP)  // the root, in sm[cur], for the hop's warp
+    asm volatile("bar.sync 2, %0;" ::"r"((int)blockDim.x) : "memory");
 }
 
 // Threads of a k_leaf CTA, and the CTAs per SM it is compiled for: eight for the
@@ -487,6 +485,19 @@ __global__ void __launch_bounds__(kStridedT, 4) k_strided(LayoutLeaf rows, int64
   if (t < width) store_digest(out + 8 * (y0 + t), d);
 }
 
+// `ctas` subtrees of T nodes at level l0; a hop only with ctas == 1.
+template <class K, class Leaf>
+zc_status subtree_launch(const Leaf& leaf, uint32_t* layers, int64_t L, int l0, int T, int64_t ctas,
+                         const P2Params* rt, cudaStream_t st, const RoundHop& hop) {
+  const int threads = subtree_threads(T);
+  if (hop.state)
+    k_subtree<K, Leaf, true><<<(unsigned)ctas, threads + 32, 0, st>>>(leaf, layers, L, l0, T, rt,
+                                                                      hop);
+  else
+    k_subtree<K, Leaf, false><<<(unsigned)ctas, threads, 0, st>>>(leaf, layers, L, l0, T, rt, hop);
+  return launch_check();
+}
+
 // Levels with more than tree_shape().levelwise_min nodes run one thread per
 // node (k_leaf with NodeLeaf, throughput-bound: a level this wide fills the
 // GPU); the narrower top of the tree is latency-bound and runs as fused CTA
@@ -494,7 +505,7 @@ __global__ void __launch_bounds__(kStridedT, 4) k_strided(LayoutLeaf rows, int64
 // Launches the levels above `l_done` (all levels <= l_done already stored).
 template <class K>
 zc_status finish_tree(uint32_t* layers, int64_t L, int l_done, const P2Params* rt,
-                      cudaStream_t st, RootHop hop = RootHop{nullptr, nullptr, 0}) {
+                      cudaStream_t st, const RoundHop& hop = RoundHop{}) {
   const int depth = ilog2(L);
   const int sub_t = tree_shape().subtree_t;
   int l = l_done;
@@ -510,9 +521,7 @@ zc_status finish_tree(uint32_t* layers, int64_t L, int l_done, const P2Params* r
     }
     const int T = parents < sub_t ? (int)parents : sub_t;
     const bool top = parents == T;  // this launch's single CTA makes the root
-    k_subtree<K, NodeLeaf><<<(unsigned)(parents / T), subtree_threads(T), 0, st>>>(
-        nl, layers, L, l + 1, T, rt, top ? hop : RootHop{nullptr, nullptr, 0});
-    ZC_TRY(launch_check());
+    ZC_TRY(subtree_launch<K>(nl, layers, L, l + 1, T, parents / T, rt, st, top ? hop : RoundHop{}));
     l += 1 + ilog2(T);
   }
   return ZC_OK;
@@ -520,7 +529,7 @@ zc_status finish_tree(uint32_t* layers, int64_t L, int l_done, const P2Params* r
 
 template <class K, class Leaf>
 zc_status commit_tree(const Leaf& leaf, uint32_t* layers, int64_t L, const P2Params* rt,
-                      cudaStream_t st, RootHop hop = RootHop{nullptr, nullptr, 0}) {
+                      cudaStream_t st, const RoundHop& hop = RoundHop{}) {
   if (L > tree_shape().levelwise_min) {
     k_leaf<K, Leaf><<<(unsigned)((L + kLeafT - 1) / kLeafT), kLeafT, 0, st>>>(leaf, layers, L, rt);
     ZC_TRY(launch_check());
@@ -529,9 +538,7 @@ zc_status commit_tree(const Leaf& leaf, uint32_t* layers, int64_t L, const P2Par
   const int sub_t = tree_shape().subtree_t;
   const int T0 = L < sub_t ? (int)L : sub_t;
   const bool top = L == T0;
-  k_subtree<K, Leaf><<<(unsigned)(L / T0), subtree_threads(T0), 0, st>>>(
-      leaf, layers, L, 0, T0, rt, top ? hop : RootHop{nullptr, nullptr, 0});
-  ZC_TRY(launch_check());
+  ZC_TRY(subtree_launch<K>(leaf, layers, L, 0, T0, L / T0, rt, st, top ? hop : RoundHop{}));
   return finish_tree<K>(layers, L, ilog2(T0), rt, st, hop);
 }
 

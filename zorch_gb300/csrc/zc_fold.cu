@@ -3,6 +3,18 @@
 // transcript hop in the root's launch).
 #include "fold.cuh"
 
+namespace zc {
+
+zc_status fold_commit_natural(const zc_poseidon2* p, const uint32_t* cw, int64_t n, int ef_in,
+                              const uint32_t* beta, int ef_beta, uint32_t shift_mont,
+                              uint32_t generator, uint32_t* out, uint32_t* layers, cudaStream_t st,
+                              const RoundHop& hop) {
+  return fold_commit_any<false>(p, cw, n, ef_in, beta, ef_beta, shift_mont, generator, out, layers,
+                                st, hop);
+}
+
+}  // namespace zc
+
 using namespace zc;
 
 extern "C" {
@@ -68,7 +80,10 @@ zc_status zc_fri_fold_commit_hop(const zc_poseidon2* p, const uint32_t* cw, int6
   }
   if ((uintptr_t)next_layers % 16) return ZC_BAD_ARG;
   ZC_TRY(check_hop(state, n_chal, chal));
-  const RootHop hop{state, chal, n_chal};
+  RoundHop hop{};
+  hop.state = state;
+  hop.n = n_chal;
+  hop.chal = chal;
   cudaStream_t st = (cudaStream_t)stream;
   return bit_reversed ? fold_commit_bitrev(p, cw, n, ef_in, beta, ef_beta, shift_mont,
                                            generator, out, next_layers, st, hop)

@@ -9,7 +9,7 @@ namespace zc {
 zc_status fold_commit_bitrev(const zc_poseidon2* p, const uint32_t* cw, int64_t n, int ef_in,
                              const uint32_t* beta, int ef_beta, uint32_t shift_mont,
                              uint32_t generator, uint32_t* out, uint32_t* layers, cudaStream_t st,
-                             RootHop hop) {
+                             const RoundHop& hop) {
   return fold_commit_any<true>(p, cw, n, ef_in, beta, ef_beta, shift_mont, generator, out, layers,
                                st, hop);
 }

@@ -5,6 +5,7 @@
 
 #include <type_traits>
 
+#include "rounds.cuh"
 #include "tree.cuh"
 
 namespace zc {
@@ -165,7 +166,8 @@ __global__ void __launch_bounds__(4 * kSubT) k_tree_top(const __grid_constant__ 
     __syncthreads();
     width >>= 1;
     lvl++;
-    subtree_level<K>(sm[cur], sm[cur ^ 1], lay + 8 * level_offset(J.L, lvl), width, hp);
+    subtree_level<K>(sm[cur], sm[cur ^ 1], lay + 8 * level_offset(J.L, lvl), width,
+                     (int)blockDim.x, hp);
     cur ^= 1;
   }
 }
@@ -224,6 +226,15 @@ zc_status tree_batch_wave(const zc_merkle_job* jobs, int n, unsigned long long* 
   if (trees > 0x7fffffff) return ZC_BAD_SHAPE;
   k_tree_top<K><<<(unsigned)trees, 4 * kSubT, 0, st>>>(B, rt);
   return launch_check();
+}
+
+zc_status merkle_commit_hop(const zc_poseidon2* p, const zc_leaves& lv, uint32_t* layers,
+                            const RoundHop& hop, cudaStream_t st) {
+  const LayoutLeaf leaf{lv.base, lv.groups, lv.group_len, lv.group_stride};
+  return with_perm(p, [&](auto k, const P2Params* rt) {
+    using K = decltype(k);
+    return commit_tree<K>(leaf, layers, lv.num_leaves, rt, st, hop);
+  });
 }
 
 // Seeded synthetic field data: SplitMix64(seed, index) reduced mod p.
@@ -337,7 +348,10 @@ zc_status zc_merkle_commit_hop(const zc_poseidon2* p, zc_leaves lv, uint32_t* la
   ZC_TRY(check_hop(state, n_chal, chal));
   cudaStream_t st = (cudaStream_t)stream;
   LayoutLeaf leaf{lv.base, lv.groups, lv.group_len, lv.group_stride};
-  const RootHop hop{state, chal, n_chal};
+  RoundHop hop{};
+  hop.state = state;
+  hop.n = n_chal;
+  hop.chal = chal;
   return with_perm(p, [&](auto k, const P2Params* rt) {
     using K = decltype(k);
     return commit_tree<K>(leaf, layers, lv.num_leaves, rt, st, hop);

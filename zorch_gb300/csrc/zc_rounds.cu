@@ -3,112 +3,28 @@
 // 90-115, zorch/pcs/basefold/prover.py:419-480, zorch/pcs/jagged/open.py:
 // 237-330). A round used to be six to eight calls from Python, 60-80 us of
 // host time where the GPU needs 60 for a small layer; here it is launches only,
-// and its transcript step, root binding and sumcheck message are one kernel.
-#include "duplex.cuh"
-#include "ef4.cuh"
+// and its sumcheck message, root binding and transcript step run in the launch
+// that computes the layer's root.
 #include "internal.cuh"
+#include "roundhop.cuh"
 #include "rounds.cuh"
 
 namespace zc {
 
-struct RoundHop1 {
-  uint32_t* state;
-  // sumcheck message (msg == nullptr: none): np partial sums of s0
-  const uint32_t* partial;
-  int np;
-  const uint32_t* claim;
-  const uint32_t* zinv;
-  uint32_t* msg;
-  // the layer's root; bind: SP1's separator over [log_height, width]
-  const uint32_t* root;
-  int bind;
-  uint32_t log_height, width;
-  uint32_t* raw_out;
-  uint32_t* root_out;
-  int n_chal;
-  uint32_t* chal;
-};
-
-// Threads of a round's hop: the CTA sums the message's partials (608 of them took
-// one warp 20 us), then its first warp goes on alone.
-constexpr int kHopT = 256;
-
-// The round's message (s0 = the partials' sum, s1 = (claim - s0) /
-// z_last + s0, zorch/pcs/basefold/kernel.py:52-66), observed; the layer's root,
-// bound if asked (k_bind_root's two permutations), observed; n_chal challenge
-// words squeezed. A chain of 1 to 5 permutations; as separate launches it was
-// three to five of them with a launch gap between each.
+// The hop of a layer whose tree stands already.
 template <class K>
-__global__ void __launch_bounds__(kHopT) k_round_hop(const P2Params* rt, const RoundHop1 a) {
-  using F = typename K::F;
+__global__ void __launch_bounds__(32) k_round_hop(const P2Params* rt, const RoundHop a,
+                                                  const uint32_t* root) {
   __shared__ P2Params s_rt;
   __shared__ uint32_t vals[16];
-  const int lane = threadIdx.x & 31, l = lane & 15;
-  LaneDuplex t;
-  uint32_t raw = 0;
-  if (threadIdx.x < 32) {
-    t.load(a.state);
-    raw = a.root[l & 7];
-  }
+  const P2Params* hp = rt;
   if constexpr (!K::kOwnTables) {
-    KIn<K>::make(rt, &s_rt);  // staged by the whole CTA
-    KIn<K>::half(rt, &s_rt);
+    KIn<K>::make(rt, &s_rt);
+    hp = KIn<K>::half(rt, &s_rt);
   }
-  if (a.msg) {
-    ef4 s0{{0, 0, 0, 0}};
-    for (int i = threadIdx.x; i < a.np; i += blockDim.x)
-      s0 = ef_add<F>(s0, ld4(a.partial + 4 * i));
-    s0 = block_sum<F>(s0);
-    if (threadIdx.x == 0) {
-      const ef4 s1 = ef_add<F>(ef_mul<F>(ef_sub<F>(ld4(a.claim), s0), ld4(a.zinv)), s0);
-      st4(a.msg, s0);
-      st4(a.msg + 4, s1);
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        vals[e] = s0.c[e];
-        vals[4 + e] = s1.c[e];
-      }
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x >= 32) return;
-  const auto body = [&](const auto& perm) {
-    // SP1's separator: compress([root, sponge([log_height, width])]). Its first
-    // permutation runs on the upper half while the lower one observes the
-    // message, when that is one permutation (nothing pending).
-    uint32_t sep = l == 0 ? to_mont<F>(a.log_height) : (l == 1 ? to_mont<F>(a.width) : 0u);
-    bool sep_done = false;
-    if (a.msg) {
-      if (a.bind && (t.in_pos & 7) == 0) {
-        uint32_t x = lane < 16 ? (l < 8 ? vals[l] : t.x) : sep;
-        x = perm.half(x);
-        sep = __shfl_sync(kFullMask, x, 16 | l);
-        t.absorbed(__shfl_sync(kFullMask, x, l));
-        sep_done = true;
-      } else {
-        t.observe(vals, 8, perm);
-      }
-    }
-    uint32_t root = raw;
-    if (a.bind) {
-      if (!sep_done) sep = perm.half(sep);
-      const uint32_t par = __shfl_sync(kFullMask, sep, (lane & 16) | (l & 7));
-      root = perm.half(l < 8 ? raw : par);
-    }
-    if (lane < 8) {
-      if (a.raw_out) a.raw_out[lane] = raw;
-      a.root_out[lane] = root;
-      vals[8 + lane] = root;
-    }
-    __syncwarp();
-    t.observe(vals + 8, 8, perm);
-    for (int i = 0; i < a.n_chal; i++) {
-      const uint32_t w = t.sample(perm);
-      if (lane == 0) a.chal[i] = w;
-    }
-  };
-  body(CallPerm<K>{K::kOwnTables ? rt : &s_rt});
-  t.store(a.state);
+  HopWarp<K> w;
+  w.begin(a, vals, hp);
+  w.end(a, vals, root, hp);
 }
 
 // Rows and sibling paths of the same q positions in up to kMaxOpen layers, one
@@ -192,22 +108,13 @@ zc_status zc_fold_rounds(const zc_poseidon2* p, const zc_fold_rounds_desc* d, vo
   const zc_field field = p->field;
   const int ef_beta = d->beta_limbs == 4;
   const uint32_t *cw = d->codeword, *mle = d->mle, *eq = d->eq;
-  uint32_t *tree = d->first_tree, *layers = d->layers, *trees = d->trees;
+  uint32_t *layers = d->layers, *trees = d->trees;
   int ef = d->ef_in ? 1 : 0, np = 0;
-  if (!d->first_committed) {
-    const int64_t L = (int64_t)1 << (d->log_n - 1);
-    const int limbs = ef ? 4 : 1;
-    const zc_leaves lv = d->bit_reversed ? zc_leaves{cw, L, 1, 2 * limbs, 0}
-                                         : zc_leaves{cw, L, 2, limbs, L * limbs};
-    ZC_TRY(zc_merkle_commit(p, lv, tree, stream));
-  }
-  if (sc) ZC_TRY(sc_first_partials(field, mle, (int64_t)1 << (d->rounds - 1), eq, w + ws.partial,
-                                   &np, st));
-  for (int r = 0; r < d->rounds; r++) {
-    const int64_t n = (int64_t)1 << (d->log_n - r), L = n >> 1;
-    uint32_t* beta = d->betas + (size_t)r * d->beta_limbs;
-    RoundHop1 h{};
+  const auto hop_of = [&](int r, int layer_ef) {
+    RoundHop h{};
     h.state = d->state;
+    h.n = d->beta_limbs;
+    h.chal = d->betas + (size_t)r * d->beta_limbs;
     if (sc) {
       h.partial = w + ws.partial;
       h.np = np;
@@ -215,46 +122,63 @@ zc_status zc_fold_rounds(const zc_poseidon2* p, const zc_fold_rounds_desc* d, vo
       h.zinv = d->zinv + 4 * (size_t)(d->rounds - 1 - r);
       h.msg = d->msgs + 8 * (size_t)r;
     }
-    h.root = tree + 8 * level_offset(L, d->log_n - r - 1);
     h.bind = d->bind;
     h.log_height = (uint32_t)(d->log_n - r - 1);
-    h.width = (uint32_t)(2 * (ef ? 4 : 1));
+    h.width = (uint32_t)(2 * (layer_ef ? 4 : 1));
     h.raw_out = d->raw_roots ? d->raw_roots + 8 * (size_t)r : nullptr;
     h.root_out = d->roots + 8 * (size_t)r;
-    h.n_chal = d->beta_limbs;
-    h.chal = beta;
-    ZC_TRY(with_perm(p, [&](auto k, const P2Params* rt) {
-      k_round_hop<decltype(k)><<<1, kHopT, 0, st>>>(rt, h);
-      return launch_check();
-    }));
-    const bool last = r == d->rounds - 1;
-    uint32_t* out = last ? d->final_layer : layers;
-    if (last) {
-      ZC_TRY((d->bit_reversed ? zc_fri_fold_bitrev : zc_fri_fold)(
-          field, cw, n, ef, beta, ef_beta, d->shifts[r], d->generator, out, stream));
+    return h;
+  };
+  if (sc) ZC_TRY(sc_first_partials(field, mle, (int64_t)1 << (d->rounds - 1), eq, w + ws.partial,
+                                   &np, st));
+  {
+    const int64_t L = (int64_t)1 << (d->log_n - 1);
+    const RoundHop h = hop_of(0, ef);
+    if (d->first_committed) {
+      ZC_TRY(with_perm(p, [&](auto k, const P2Params* rt) {
+        k_round_hop<decltype(k)><<<1, 32, 0, st>>>(rt, h,
+                                                   d->first_tree + 8 * level_offset(L, d->log_n - 1));
+        return launch_check();
+      }));
     } else {
-      ZC_TRY((d->bit_reversed ? zc_fri_fold_commit_bitrev : zc_fri_fold_commit)(
-          p, cw, n, ef, beta, ef_beta, d->shifts[r], d->generator, out, trees, stream));
-      tree = trees;
-      trees += 8 * (n / 2 - 1);  // 2 (n / 4) - 1 digests
+      const int limbs = ef ? 4 : 1;
+      const zc_leaves lv = d->bit_reversed ? zc_leaves{cw, L, 1, 2 * limbs, 0}
+                                           : zc_leaves{cw, L, 2, limbs, L * limbs};
+      ZC_TRY(merkle_commit_hop(p, lv, d->first_tree, h, st));
     }
-    ef |= ef_beta;
-    cw = out;
-    layers += last ? 0 : (n / 2) * (ef ? 4 : 1);
-    if (sc) {
+  }
+  for (int r = 0; r < d->rounds; r++) {
+    const int64_t n = (int64_t)1 << (d->log_n - r);
+    const uint32_t* beta = d->betas + (size_t)r * d->beta_limbs;
+    const bool last = r == d->rounds - 1;
+    if (sc) {  // before the next layer's hop, which takes the partials
       const int64_t M = (int64_t)1 << (d->rounds - 1 - r);
+      const uint32_t* msg = d->msgs + 8 * (size_t)r;
       uint32_t* mle_out = w + ws.mle[r & 1];
       if (M >= 2) {
         uint32_t* eq_out = w + ws.eq[r & 1];
-        ZC_TRY(sc_fold_partials(field, mle, M, beta, d->beta_limbs, h.msg, mle_out, eq, eq_out,
+        ZC_TRY(sc_fold_partials(field, mle, M, beta, d->beta_limbs, msg, mle_out, eq, eq_out,
                                 d->claim, w + ws.partial, &np, st));
         eq = eq_out;
       } else {
-        ZC_TRY(zc_sumcheck_fold(field, mle, M, beta, d->beta_limbs, h.msg, mle_out, nullptr,
-                                nullptr, d->claim, stream));
+        ZC_TRY(zc_sumcheck_fold(field, mle, M, beta, d->beta_limbs, msg, mle_out, nullptr, nullptr,
+                                d->claim, stream));
       }
       mle = mle_out;
     }
+    if (last) {
+      ZC_TRY((d->bit_reversed ? zc_fri_fold_bitrev : zc_fri_fold)(
+          field, cw, n, ef, beta, ef_beta, d->shifts[r], d->generator, d->final_layer, stream));
+      break;
+    }
+    const int out_ef = ef | ef_beta;
+    const RoundHop h = hop_of(r + 1, out_ef);
+    ZC_TRY((d->bit_reversed ? fold_commit_bitrev : fold_commit_natural)(
+        p, cw, n, ef, beta, ef_beta, d->shifts[r], d->generator, layers, trees, st, h));
+    trees += 8 * (n / 2 - 1);  // 2 (n / 4) - 1 digests
+    ef = out_ef;
+    cw = layers;
+    layers += (n / 2) * (ef ? 4 : 1);
   }
   return ZC_OK;
 }
