@@ -10,13 +10,14 @@ namespace zc {
 template <class F, int LI, int LB, bool BR>
 __global__ void k_fold(const uint32_t* f, int64_t n, const uint32_t* beta, uint32_t inv2s,
                        uint32_t winv, uint32_t* g) {
+  pdl_wait();
   using M = FoldMath<F, LI, LB>;
   const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t half = n >> 1;
   if (j >= half) return;
   uint32_t bt[4];
 #pragma unroll
-  for (int e = 0; e < LB; e++) bt[e] = __ldg(beta + e);
+  for (int e = 0; e < LB; e++) bt[e] = gld(beta + e);
   uint32_t out[4];
   if (BR)  // pair (f[2j], f[2j+1]) at x_j = shift w^brev(j)
     M::fold(f + 2 * j * LI, 1, 0,
@@ -36,6 +37,7 @@ __global__ void k_fold(const uint32_t* f, int64_t n, const uint32_t* beta, uint3
 template <class F, int LI, int LB, int K>
 __global__ void k_fold_k(const uint32_t* f, int64_t n, const uint32_t* beta, uint32_t shinv,
                          uint32_t winv, uint32_t wkinv, uint32_t kinv, uint32_t* g) {
+  pdl_wait();
   constexpr int LO = (LI == 4 || LB == 4) ? 4 : 1;
   const int64_t sub = n / K;
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -45,7 +47,7 @@ __global__ void k_fold_k(const uint32_t* f, int64_t n, const uint32_t* beta, uin
   for (int m = 0; m < K; m++) {
     v[m] = ef4{{0, 0, 0, 0}};
 #pragma unroll
-    for (int e = 0; e < LI; e++) v[m].c[e] = __ldg(f + (p + m * sub) * LI + e);
+    for (int e = 0; e < LI; e++) v[m].c[e] = gld(f + (p + m * sub) * LI + e);
   }
   uint32_t wk[K];  // w_K^(-j)
   wk[0] = F::ONE;
@@ -54,7 +56,7 @@ __global__ void k_fold_k(const uint32_t* f, int64_t n, const uint32_t* beta, uin
   const uint32_t x0inv = mmul<F>(shinv, mpow<F>(winv, (uint64_t)p));
   ef4 u{{0, 0, 0, 0}};
 #pragma unroll
-  for (int e = 0; e < LB; e++) u.c[e] = mmul<F>(__ldg(beta + e), x0inv);
+  for (int e = 0; e < LB; e++) u.c[e] = mmul<F>(gld(beta + e), x0inv);
   ef4 acc{{0, 0, 0, 0}};
 #pragma unroll
   for (int j = K - 1; j >= 0; j--) {
@@ -79,10 +81,10 @@ zc_status fold_k_launch(const uint32_t* cw, int64_t n, const uint32_t* beta, int
   const int64_t sub = n >> log_k;
   const unsigned grid = (unsigned)((sub + 127) / 128);
   switch (log_k) {
-    case 1: k_fold_k<F, LI, LB, 2><<<grid, 128, 0, st>>>(cw, n, beta, shinv, winv, wkinv, kinv, out); break;
-    case 2: k_fold_k<F, LI, LB, 4><<<grid, 128, 0, st>>>(cw, n, beta, shinv, winv, wkinv, kinv, out); break;
-    case 3: k_fold_k<F, LI, LB, 8><<<grid, 128, 0, st>>>(cw, n, beta, shinv, winv, wkinv, kinv, out); break;
-    default: k_fold_k<F, LI, LB, 16><<<grid, 128, 0, st>>>(cw, n, beta, shinv, winv, wkinv, kinv, out); break;
+    case 1: pdl_launch(k_fold_k<F, LI, LB, 2>, grid, 128, 0, st, cw, n, beta, shinv, winv, wkinv, kinv, out); break;
+    case 2: pdl_launch(k_fold_k<F, LI, LB, 4>, grid, 128, 0, st, cw, n, beta, shinv, winv, wkinv, kinv, out); break;
+    case 3: pdl_launch(k_fold_k<F, LI, LB, 8>, grid, 128, 0, st, cw, n, beta, shinv, winv, wkinv, kinv, out); break;
+    default: pdl_launch(k_fold_k<F, LI, LB, 16>, grid, 128, 0, st, cw, n, beta, shinv, winv, wkinv, kinv, out); break;
   }
   return launch_check();
 }
@@ -114,7 +116,7 @@ zc_status fold_launch(const uint32_t* cw, int64_t n, const uint32_t* beta, uint3
   ZC_TRY(fold_scalars<F>(n, shift_mont, generator, &fs));
   const int64_t half = n >> 1;
   const int B = 256;
-  k_fold<F, LI, LB, BR><<<(unsigned)((half + B - 1) / B), B, 0, st>>>(cw, n, beta, fs.inv2s,
+  pdl_launch(k_fold<F, LI, LB, BR>, (unsigned)((half + B - 1) / B), B, 0, st, cw, n, beta, fs.inv2s,
                                                                       fs.winv, out);
   return launch_check();
 }

@@ -41,7 +41,7 @@ struct LayoutLeaf {
 #pragma unroll
       for (int j = 0; j < 8; j++) {
         if (e + j < w) {
-          s[j] = __ldg(src + (int64_t)q * gs + r);
+          s[j] = gld(src + (int64_t)q * gs + r);
           if (++r == g) {
             r = 0;
             q++;
@@ -71,7 +71,7 @@ struct LayoutLeaf {
           const int i = e + q4 + k;
           if (i < w) {
             const int gi = i / g;
-            x[k] = __ldg(src + (int64_t)gi * gs + (i - gi * g));
+            x[k] = gld(src + (int64_t)gi * gs + (i - gi * g));
           }
         }
       }
@@ -104,8 +104,8 @@ struct FoldMath {
     uint32_t a[4] = {0, 0, 0, 0}, b[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int e = 0; e < LI; e++) {
-      a[e] = __ldg(f + j * LI + e);
-      b[e] = __ldg(f + (j + half) * LI + e);
+      a[e] = gld(f + j * LI + e);
+      b[e] = gld(f + (j + half) * LI + e);
     }
     uint32_t sum[4], d[4];
 #pragma unroll
@@ -160,7 +160,7 @@ struct FoldLeaf {
     const int64_t quarter = n >> 2, half = n >> 1;
     uint32_t bt[4];
 #pragma unroll
-    for (int e = 0; e < LB; e++) bt[e] = __ldg(beta + e);
+    for (int e = 0; e < LB; e++) bt[e] = gld(beta + e);
     uint32_t o0[4], o1[4];
     int64_t i0, i1;
     if (BR) {
@@ -201,7 +201,7 @@ struct FoldLeaf {
       const int64_t quarter = n >> 2, half = n >> 1;
       uint32_t bt[4];
 #pragma unroll
-      for (int e = 0; e < LB; e++) bt[e] = __ldg(beta + e);
+      for (int e = 0; e < LB; e++) bt[e] = gld(beta + e);
       uint32_t o[4];
       int64_t i;
       if (BR) {
@@ -360,6 +360,7 @@ __global__ void __launch_bounds__(kSubThreads + 32, 1) k_subtree(Leaf leaf, uint
   __shared__ __align__(16) uint32_t sm[2][8 * kSubCap];  // [node][word] digest slots
   KIn<K>::make(rt, &s_rt);
   const P2Params* hp = KIn<K>::half(rt, &s_rt);
+  pdl_wait();
   const int t = threadIdx.x;
   const int W = blockDim.x - (HOP ? 32 : 0);
   if constexpr (HOP) {
@@ -434,6 +435,7 @@ __global__ void __launch_bounds__(kLeafT, HashOcc<K>::v) k_leaf(Leaf leaf, uint3
                                                 const P2Params* rt) {
   __shared__ P2Params s_rt;
   K k = KIn<K>::make(rt, &s_rt);
+  pdl_wait();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= count) return;
   uint32_t d[8];
@@ -459,6 +461,7 @@ __global__ void __launch_bounds__(kStridedT, 4) k_strided(LayoutLeaf rows, int64
   __shared__ P2Params s_rt;
   __shared__ __align__(16) uint32_t sm[8 * kStridedT];
   K k = KIn<K>::make(rt, &s_rt);
+  pdl_wait();
   const int t = threadIdx.x;
   const int64_t y0 = (int64_t)blockIdx.x * np;
   int width = np << log_rpq;  // digests of the current level
@@ -491,10 +494,10 @@ zc_status subtree_launch(const Leaf& leaf, uint32_t* layers, int64_t L, int l0, 
                          const P2Params* rt, cudaStream_t st, const RoundHop& hop) {
   const int threads = subtree_threads(T);
   if (hop.state)
-    k_subtree<K, Leaf, true><<<(unsigned)ctas, threads + 32, 0, st>>>(leaf, layers, L, l0, T, rt,
+    pdl_launch(k_subtree<K, Leaf, true>, (unsigned)ctas, threads + 32, 0, st, leaf, layers, L, l0, T, rt,
                                                                       hop);
   else
-    k_subtree<K, Leaf, false><<<(unsigned)ctas, threads, 0, st>>>(leaf, layers, L, l0, T, rt, hop);
+    pdl_launch(k_subtree<K, Leaf, false>, (unsigned)ctas, threads, 0, st, leaf, layers, L, l0, T, rt, hop);
   return launch_check();
 }
 
@@ -513,7 +516,7 @@ zc_status finish_tree(uint32_t* layers, int64_t L, int l_done, const P2Params* r
     const int64_t parents = (L >> l) >> 1;
     NodeLeaf nl{layers + 8 * level_offset(L, l)};
     if (parents > tree_shape().levelwise_min) {
-      k_leaf<K, NodeLeaf><<<(unsigned)((parents + kLeafT - 1) / kLeafT), kLeafT, 0, st>>>(
+      pdl_launch(k_leaf<K, NodeLeaf>, (unsigned)((parents + kLeafT - 1) / kLeafT), kLeafT, 0, st, 
           nl, layers + 8 * level_offset(L, l + 1), parents, rt);
       ZC_TRY(launch_check());
       l += 1;
@@ -531,7 +534,7 @@ template <class K, class Leaf>
 zc_status commit_tree(const Leaf& leaf, uint32_t* layers, int64_t L, const P2Params* rt,
                       cudaStream_t st, const RoundHop& hop = RoundHop{}) {
   if (L > tree_shape().levelwise_min) {
-    k_leaf<K, Leaf><<<(unsigned)((L + kLeafT - 1) / kLeafT), kLeafT, 0, st>>>(leaf, layers, L, rt);
+    pdl_launch(k_leaf<K, Leaf>, (unsigned)((L + kLeafT - 1) / kLeafT), kLeafT, 0, st, leaf, layers, L, rt);
     ZC_TRY(launch_check());
     return finish_tree<K>(layers, L, 0, rt, st, hop);
   }

@@ -59,8 +59,9 @@ __global__ void __launch_bounds__(32) k_duplex_step(const P2Params* rt, uint32_t
                                                     int64_t block_len) {
   __shared__ P2Params s_rt;
   LaneDuplex t;
-  t.load(state);
   with_half_perm<K>(rt, &s_rt, [&](const auto& perm) {
+    pdl_wait();
+    t.load(state);
     t.observe(values, m, perm);
     for (int i = 0; i < n; i++) {
       const uint32_t w = t.sample(CallPerm<K>{K::kOwnTables ? rt : &s_rt});
@@ -81,8 +82,9 @@ __global__ void __launch_bounds__(32) k_duplex_hop(
     uint32_t* out_pos_o, uint32_t* chal) {
   __shared__ P2Params s_rt;
   LaneDuplex t;
-  t.load(in_buf, out_buf, sponge, in_pos, out_pos);
   with_half_perm<K>(rt, &s_rt, [&](const auto& perm) {
+    pdl_wait();
+    t.load(in_buf, out_buf, sponge, in_pos, out_pos);
     t.observe(values, m, perm);
     for (int i = 0; i < n; i++) {
       const uint32_t w = t.sample(CallPerm<K>{K::kOwnTables ? rt : &s_rt});
@@ -94,6 +96,7 @@ __global__ void __launch_bounds__(32) k_duplex_hop(
 
 template <class F>
 __global__ void k_convert(const uint32_t* in, uint32_t* out, int64_t n, int to) {
+  pdl_wait();
   // 16-byte accesses when both sides are aligned (more bytes in flight per
   // thread, which a read of page-locked host memory over the host link needs)
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -117,6 +120,7 @@ __global__ void k_convert(const uint32_t* in, uint32_t* out, int64_t n, int to) 
 
 template <class F>
 __global__ void k_scale(const uint32_t* in, uint32_t* out, int64_t n, uint32_t s) {
+  pdl_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     out[i] = mmul<F>(in[i], s);
@@ -126,6 +130,7 @@ template <class K>
 __global__ void k_permute(const P2Params* rt, uint32_t* states, int64_t count) {
   __shared__ P2Params s_rt;
   K k = KIn<K>::make(rt, &s_rt);
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   uint32_t s[16];
@@ -154,6 +159,7 @@ __global__ void __launch_bounds__(kGrindT) k_grind(const P2Params* rt, const uin
   using F = typename K::F;
   __shared__ P2Params s_rt;
   K k = KIn<K>::make(rt, &s_rt);
+  pdl_wait();
   const Duplex* t = reinterpret_cast<const Duplex*>(state);
   const int in_pos = t->in_pos & 7;
   uint32_t base[16];
@@ -332,7 +338,7 @@ zc_status zc_poseidon2_permute(const zc_poseidon2* p, uint32_t* states, int64_t 
   return with_perm(p, [&](auto k, const P2Params* rt) {
     using K = decltype(k);
     int64_t blocks = (count + 127) / 128;
-    k_permute<K><<<(unsigned)blocks, 128, 0, st>>>(rt, states, count);
+    pdl_launch(k_permute<K>, (unsigned)blocks, 128, 0, st, rt, states, count);
     return launch_check();
   });
 }
@@ -349,7 +355,7 @@ static zc_status convert(zc_field field, const uint32_t* in, uint32_t* out, int6
     using F = decltype(f);
     int64_t blocks = (n + 255) / 256;
     if (blocks > 152 * 16) blocks = 152 * 16;
-    k_convert<F><<<(unsigned)blocks, 256, 0, st>>>(in, out, n, to);
+    pdl_launch(k_convert<F>, (unsigned)blocks, 256, 0, st, in, out, n, to);
     return launch_check();
   });
 }
@@ -368,7 +374,7 @@ zc_status zc_to_mont_from_host(zc_field field, const void* host, uint32_t* out, 
     using F = decltype(f);
     int64_t blocks = (n + 1023) / 1024;
     if (blocks > cap) blocks = cap;
-    k_convert<F><<<(unsigned)blocks, 1024, 0, st>>>(static_cast<const uint32_t*>(src), out, n, 1);
+    pdl_launch(k_convert<F>, (unsigned)blocks, 1024, 0, st, static_cast<const uint32_t*>(src), out, n, 1);
     return launch_check();
   });
 }
@@ -417,7 +423,7 @@ zc_status zc_scale(zc_field field, const uint32_t* in, uint32_t* out, int64_t n,
     using F = decltype(f);
     int64_t blocks = (n + 255) / 256;
     if (blocks > 152 * 16) blocks = 152 * 16;
-    k_scale<F><<<(unsigned)blocks, 256, 0, st>>>(in, out, n, s_mont);
+    pdl_launch(k_scale<F>, (unsigned)blocks, 256, 0, st, in, out, n, s_mont);
     return launch_check();
   });
 }
@@ -430,7 +436,7 @@ zc_status zc_duplex_step(const zc_poseidon2* p, uint32_t* state, const uint32_t*
   cudaStream_t st = (cudaStream_t)stream;
   return with_perm(p, [&](auto k, const P2Params* rt) {
     using K = decltype(k);
-    k_duplex_step<K><<<1, 32, 0, st>>>(rt, state, values, m, n, out, positions, block_len);
+    pdl_launch(k_duplex_step<K>, 1, 32, 0, st, rt, state, values, m, n, out, positions, block_len);
     return launch_check();
   });
 }
@@ -455,7 +461,7 @@ zc_status zc_duplex_grind(const zc_poseidon2* p, const uint32_t* state, int32_t 
   const uint32_t mask = (uint32_t)((1ull << pow_bits) - 1);
   return with_perm(p, [&](auto k, const P2Params* rt) {
     using K = decltype(k);
-    k_grind<K><<<blocks, kGrindT, 0, st>>>(rt, state, mask, witness);
+    pdl_launch(k_grind<K>, blocks, kGrindT, 0, st, rt, state, mask, witness);
     ZC_TRY(launch_check());
     k_grind_finish<typename K::F><<<1, 1, 0, st>>>(witness);
     return launch_check();
@@ -474,7 +480,7 @@ zc_status zc_duplex_hop(const zc_poseidon2* p, const uint32_t* in_buf, const uin
   cudaStream_t st = (cudaStream_t)stream;
   return with_perm(p, [&](auto k, const P2Params* rt) {
     using K = decltype(k);
-    k_duplex_hop<K><<<1, 32, 0, st>>>(rt, in_buf, out_buf, sponge, in_pos, out_pos, values, m,
+    pdl_launch(k_duplex_hop<K>, 1, 32, 0, st, rt, in_buf, out_buf, sponge, in_pos, out_pos, values, m,
                                       n, in_buf_o, out_buf_o, sponge_o, in_pos_o, out_pos_o,
                                       challenges);
     return launch_check();

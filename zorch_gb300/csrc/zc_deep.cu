@@ -75,6 +75,7 @@ template <class F, int L>
 __global__ void __launch_bounds__(kEvalT) k_eval_partial(const uint32_t* c, int64_t k,
                                                          const uint32_t* z, int log_threads,
                                                          uint32_t* part) {
+  pdl_wait();
   __shared__ ef4 sm[kEvalT];
   const ef4 zz = e_load<L>(z);
   ef4 u = zz;  // z^T, T = 2^log_threads
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(kEvalT) k_eval_partial(const uint32_t* c, int6
     int64_t j = (k - 1 - t) / T;  // last j with t + jT < k
     for (; j >= 0; j--) {
       acc = e_mul<F, L>(acc, u);
-      acc.c[0] = madd<F>(acc.c[0], __ldg(c + t + j * T));
+      acc.c[0] = madd<F>(acc.c[0], gld(c + t + j * T));
     }
   }
   sm[threadIdx.x] = acc;
@@ -97,6 +98,7 @@ __global__ void __launch_bounds__(kEvalT) k_eval_partial(const uint32_t* c, int6
 template <class F, int L>
 __global__ void __launch_bounds__(kEvalMaxBlocks) k_eval_final(const uint32_t* part, int blocks,
                                                                const uint32_t* z, uint32_t* out) {
+  pdl_wait();
   __shared__ ef4 sm[kEvalMaxBlocks];
   ef4 zz = e_load<L>(z);  // z^kEvalT between consecutive block partials
   for (int i = 0; (1 << i) < kEvalT; i++) zz = e_mul<F, L>(zz, zz);
@@ -115,6 +117,7 @@ __global__ void __launch_bounds__(256) k_deep_quotient(const uint32_t* cw, int64
                                                        const uint32_t* z, const uint32_t* v,
                                                        uint32_t shift, uint32_t w,
                                                        uint32_t* out) {
+  pdl_wait();
   const int64_t j0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * kDeepM;
   if (j0 >= n) return;
   const ef4 zz = e_load<L>(z), vv = e_load<L>(v);
@@ -134,7 +137,7 @@ __global__ void __launch_bounds__(256) k_deep_quotient(const uint32_t* cw, int64
     if (L == 1) di.c[1] = di.c[2] = di.c[3] = 0u;
     zero[i] = !on || e_zero<L>(di);
     d[i] = zero[i] ? ef4{{F::ONE, 0u, 0u, 0u}} : di;
-    f[i] = on ? __ldg(cw + j) : 0u;
+    f[i] = on ? gld(cw + j) : 0u;
     pre[i] = i ? e_mul<F, L>(pre[i - 1], d[i]) : d[i];
     if (!BR) x = mmul<F>(x, w);
   }
@@ -183,13 +186,13 @@ zc_status zc_eval_poly(zc_field field, const uint32_t* coeffs, int64_t k, const 
   return with_field(field, [&](auto f) -> zc_status {
     using F = decltype(f);
     if (z_limbs == 1) {
-      k_eval_partial<F, 1><<<(unsigned)blocks, kEvalT, 0, st>>>(coeffs, k, z, log_threads, part);
+      pdl_launch(k_eval_partial<F, 1>, (unsigned)blocks, kEvalT, 0, st, coeffs, k, z, log_threads, part);
       ZC_TRY(launch_check());
-      k_eval_final<F, 1><<<1, kEvalMaxBlocks, 0, st>>>(part, (int)blocks, z, out);
+      pdl_launch(k_eval_final<F, 1>, 1, kEvalMaxBlocks, 0, st, part, (int)blocks, z, out);
     } else {
-      k_eval_partial<F, 4><<<(unsigned)blocks, kEvalT, 0, st>>>(coeffs, k, z, log_threads, part);
+      pdl_launch(k_eval_partial<F, 4>, (unsigned)blocks, kEvalT, 0, st, coeffs, k, z, log_threads, part);
       ZC_TRY(launch_check());
-      k_eval_final<F, 4><<<1, kEvalMaxBlocks, 0, st>>>(part, (int)blocks, z, out);
+      pdl_launch(k_eval_final<F, 4>, 1, kEvalMaxBlocks, 0, st, part, (int)blocks, z, out);
     }
     return launch_check();
   });
@@ -215,14 +218,14 @@ zc_status zc_deep_quotient(zc_field field, const uint32_t* cw, int64_t n, const 
     const uint32_t sh = shift_mont ? shift_mont : F::ONE;
     if (z_limbs == 1) {
       if (bit_reversed)
-        k_deep_quotient<F, 1, true><<<grid, 256, 0, st>>>(cw, n, log_n, z, v, sh, w, out);
+        pdl_launch(k_deep_quotient<F, 1, true>, grid, 256, 0, st, cw, n, log_n, z, v, sh, w, out);
       else
-        k_deep_quotient<F, 1, false><<<grid, 256, 0, st>>>(cw, n, log_n, z, v, sh, w, out);
+        pdl_launch(k_deep_quotient<F, 1, false>, grid, 256, 0, st, cw, n, log_n, z, v, sh, w, out);
     } else {
       if (bit_reversed)
-        k_deep_quotient<F, 4, true><<<grid, 256, 0, st>>>(cw, n, log_n, z, v, sh, w, out);
+        pdl_launch(k_deep_quotient<F, 4, true>, grid, 256, 0, st, cw, n, log_n, z, v, sh, w, out);
       else
-        k_deep_quotient<F, 4, false><<<grid, 256, 0, st>>>(cw, n, log_n, z, v, sh, w, out);
+        pdl_launch(k_deep_quotient<F, 4, false>, grid, 256, 0, st, cw, n, log_n, z, v, sh, w, out);
     }
     return launch_check();
   });

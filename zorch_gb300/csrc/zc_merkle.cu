@@ -17,6 +17,7 @@ namespace zc {
 // computed here rather than by the caller.
 __global__ void k_open(zc_leaves lv, const uint32_t* layers, const int32_t* idx, int q, int depth,
                        uint32_t* rows, uint32_t* paths, uint32_t* oob, int reduce, int shift) {
+  pdl_wait();
   const int qi = blockIdx.x;
   int64_t i = idx[qi];
   if (reduce)
@@ -48,6 +49,7 @@ __global__ void __launch_bounds__(32) k_bind_root(const P2Params* rt, const uint
   __shared__ P2Params s_rt;
   KIn<K>::make(rt, &s_rt);
   const P2Params* hp = KIn<K>::half(rt, &s_rt);
+  pdl_wait();
   const int lane = threadIdx.x & 31, l = lane & 15;
   // sponge: state = [log_height, width, 0 ...] (one absorb block), permute
   uint32_t x = l == 0 ? to_mont<F>(log_height) : (l == 1 ? to_mont<F>(width) : 0u);
@@ -304,7 +306,7 @@ zc_status zc_strided_merkle_commit(const zc_poseidon2* p, zc_leaves lv, int32_t 
   return with_perm(p, [&](auto k, const P2Params* rt) -> zc_status {
     using K = decltype(k);
     const int threads = (np << log_rpq) < 32 ? 32 : np << log_rpq;
-    k_strided<K><<<(unsigned)(s / np), threads, 0, st>>>(rows, s, log_rpq, np, layers, rt);
+    pdl_launch(k_strided<K>, (unsigned)(s / np), threads, 0, st, rows, s, log_rpq, np, layers, rt);
     ZC_TRY(launch_check());
     return finish_tree<K>(layers, s, 0, rt, st);
   });
@@ -316,7 +318,7 @@ zc_status zc_merkle_open(zc_leaves lv, const uint32_t* layers, const int32_t* id
   if (!is_pow2(lv.num_leaves)) return ZC_NOT_POW2;
   if (q == 0) return ZC_OK;
   const int depth = ilog2(lv.num_leaves);
-  k_open<<<q, 128, 0, (cudaStream_t)stream>>>(lv, layers, idx, q, depth, rows, paths, oob_flag,
+  pdl_launch(k_open, q, 128, 0, (cudaStream_t)stream, lv, layers, idx, q, depth, rows, paths, oob_flag,
                                               0, 0);
   return launch_check();
 }
@@ -329,7 +331,7 @@ zc_status zc_merkle_open_reduced(zc_leaves lv, const uint32_t* layers, const int
   if (!is_pow2(lv.num_leaves) || lv.num_leaves > (1ll << 32)) return ZC_NOT_POW2;
   if (q == 0) return ZC_OK;
   const int depth = ilog2(lv.num_leaves);
-  k_open<<<q, 128, 0, (cudaStream_t)stream>>>(lv, layers, idx, q, depth, rows, paths, nullptr,
+  pdl_launch(k_open, q, 128, 0, (cudaStream_t)stream, lv, layers, idx, q, depth, rows, paths, nullptr,
                                               1, shift);
   return launch_check();
 }
@@ -364,7 +366,7 @@ zc_status zc_smcs_bind_root(const zc_poseidon2* p, const uint32_t* raw_root, uin
   cudaStream_t st = (cudaStream_t)stream;
   return with_perm(p, [&](auto k, const P2Params* rt) {
     using K = decltype(k);
-    k_bind_root<K><<<1, 32, 0, st>>>(rt, raw_root, log_height, width, out);
+    pdl_launch(k_bind_root<K>, 1, 32, 0, st, rt, raw_root, log_height, width, out);
     return launch_check();
   });
 }

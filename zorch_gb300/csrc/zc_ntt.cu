@@ -300,6 +300,7 @@ template <class F>
 __global__ void __launch_bounds__(kThreads, 2) k_lde_small(const uint32_t* x, uint32_t* out,
                                                         int log_k, int log_b, uint32_t h,
                                                         int brev_out, int rev, uint32_t post) {
+  pdl_wait();
   extern __shared__ uint32_t sm[];
   lde_small_body<F>(x, out, log_k, log_b, h, blockIdx.x, sm, brev_out, kMaxRadixLog, rev, post);
 }
@@ -359,10 +360,10 @@ __device__ __forceinline__ void p1_pass(uint32_t* work, int rs, int log_ti, int 
         const uint32_t kmask = (1u << (log_k1 + log_k2)) - 1;
 #pragma unroll
         for (int j = 0; j < G; j++)
-          v[j] = __ldg(xc + ((0u - i0 - ((uint32_t)j << (lS + log_k1))) & kmask));
+          v[j] = gld(xc + ((0u - i0 - ((uint32_t)j << (lS + log_k1))) & kmask));
       } else {
 #pragma unroll
-        for (int j = 0; j < G; j++) v[j] = __ldg(xc + i0 + ((int64_t)j << (lS + log_k1)));
+        for (int j = 0; j < G; j++) v[j] = gld(xc + i0 + ((int64_t)j << (lS + log_k1)));
       }
       if (!unit) {
         int32_t f = smul<F>((int32_t)gi[d], (int32_t)Gt[off]);
@@ -463,7 +464,7 @@ __device__ __forceinline__ void p2_first(uint32_t* work, int rs, int log_b, int 
       const uint32_t* src = zc_ + ((int64_t)s << log_k) + ((int64_t)t << log_k1) + off;
       uint32_t v[G];
 #pragma unroll
-      for (int j = 0; j < G; j++) v[j] = __ldg(src + (j << lS));
+      for (int j = 0; j < G; j++) v[j] = gld(src + (j << lS));
 #pragma unroll
       for (int j = 0; j < G; j++) v[j] = snorm<F>(smul<F>((int32_t)v[j], f[j]));
       if (last)
@@ -585,6 +586,7 @@ template <class F, int MR = kMaxRadixLog, bool REV = false>
 __global__ void __launch_bounds__(lde_threads<MR>(), lde_min_blocks<MR>()) k_lde_pass1(const uint32_t* x, uint32_t* z, int log_k1,
                                                         int log_k2, int log_b, int log_ti,
                                                         uint32_t h) {
+  pdl_wait();
   extern __shared__ uint32_t sm[];
   lde_pass1_fused<F, MR, REV>(x, z, log_k1, log_k2, log_b, log_ti, h, blockIdx.x, blockIdx.y,
                               blockIdx.z, sm, MR);
@@ -600,6 +602,7 @@ __global__ void __launch_bounds__(lde_threads<MR>(), lde_min_blocks<MR>()) k_lde
                                                         int log_k1, int log_k2, int log_b,
                                                         int log_tt, int brev_out,
                                                         uint32_t post) {
+  pdl_wait();
   extern __shared__ uint32_t sm[];
   lde_pass2_fused<F, MR>(z, out, log_k1, log_k2, log_b, log_tt, blockIdx.x, blockIdx.y, sm,
                          brev_out, MR, post);
@@ -686,7 +689,7 @@ zc_status lde_launch(const uint32_t* x, int64_t batch, int log_k, int log_b, uin
                                  (int)p.smem_small));
     for (int64_t c0 = 0; c0 < batch; c0 += 0x7fffffff) {
       const int64_t cols = batch - c0 < 0x7fffffff ? batch - c0 : 0x7fffffff;
-      k_lde_small<F><<<(unsigned)cols, kThreads, p.smem_small, st>>>(
+      pdl_launch(k_lde_small<F>, (unsigned)cols, kThreads, p.smem_small, st, 
           x + (c0 << log_k), out + (c0 << log_n), log_k, log_b, h, brev_out, rev, post);
       ZC_TRY(launch_check());
     }
@@ -719,11 +722,11 @@ zc_status lde_four_step(const uint32_t* x, int64_t batch, int log_k, int log_b, 
   for (int64_t c0 = 0; c0 < batch; c0 += chunk) {
     const int64_t cols = batch - c0 < chunk ? batch - c0 : chunk;
     dim3 g1(1u << log_b, 1u << (p.log_k1 - p.log_ti), (unsigned)cols);
-    pass1<<<g1, lde_threads<MR>(), p.smem1, st>>>(x + (c0 << log_k), z, p.log_k1, p.log_k2, log_b,
+    pdl_launch(pass1, g1, lde_threads<MR>(), p.smem1, st, x + (c0 << log_k), z, p.log_k1, p.log_k2, log_b,
                                                   p.log_ti, h);
     ZC_TRY(launch_check());
     dim3 g2(1u << (p.log_k2 - p.log_tt), (unsigned)cols);
-    k_lde_pass2<F, MR><<<g2, lde_threads<MR>(), p.smem2, st>>>(z, out + (c0 << log_n), p.log_k1,
+    pdl_launch(k_lde_pass2<F, MR>, g2, lde_threads<MR>(), p.smem2, st, z, out + (c0 << log_n), p.log_k1,
                                                                p.log_k2, log_b, p.log_tt,
                                                                brev_out, post);
     ZC_TRY(launch_check());

@@ -22,6 +22,7 @@ __global__ void __launch_bounds__(32) k_round_hop(const P2Params* rt, const Roun
     KIn<K>::make(rt, &s_rt);
     hp = KIn<K>::half(rt, &s_rt);
   }
+  pdl_wait();
   HopWarp<K> w;
   w.begin(a, vals, hp);
   w.end(a, vals, root, hp);
@@ -37,6 +38,7 @@ struct OpenTable {
 
 __global__ void __launch_bounds__(128) k_open_layers(const __grid_constant__ OpenTable T,
                                                      const int32_t* idx, int q) {
+  pdl_wait();
   const zc_open_job& j = T.job[blockIdx.y];
   const zc_leaves& lv = j.leaves;
   const int qi = blockIdx.x;
@@ -136,7 +138,7 @@ zc_status zc_fold_rounds(const zc_poseidon2* p, const zc_fold_rounds_desc* d, vo
     const RoundHop h = hop_of(0, ef);
     if (d->first_committed) {
       ZC_TRY(with_perm(p, [&](auto k, const P2Params* rt) {
-        k_round_hop<decltype(k)><<<1, 32, 0, st>>>(rt, h,
+        pdl_launch(k_round_hop<decltype(k)>, 1, 32, 0, st, rt, h,
                                                    d->first_tree + 8 * level_offset(L, d->log_n - 1));
         return launch_check();
       }));
@@ -199,7 +201,7 @@ zc_status zc_open_layers(const zc_open_job* jobs, int32_t count, const int32_t* 
     const int n = count - i < kMaxOpen ? count - i : kMaxOpen;
     for (int k = 0; k < n; k++) T.job[k] = jobs[i + k];
     for (int k = n; k < kMaxOpen; k++) T.job[k] = zc_open_job{};
-    k_open_layers<<<dim3((unsigned)q, (unsigned)n), 128, 0, (cudaStream_t)stream>>>(T, idx, q);
+    pdl_launch(k_open_layers, dim3((unsigned)q, (unsigned)n), 128, 0, (cudaStream_t)stream, T, idx, q);
     ZC_TRY(launch_check());
   }
   return ZC_OK;

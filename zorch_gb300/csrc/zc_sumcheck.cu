@@ -28,6 +28,7 @@ struct EqTable {
 };
 template <class F>
 __global__ void __launch_bounds__(512) k_eq_small(const EqTable t0, const EqTable t1) {
+  pdl_wait();
   constexpr int H = kEqSmall / 2;
   __shared__ __align__(16) uint32_t tab[2][2][4 << H];  // [parity of the step][half][entry]
   const EqTable t = blockIdx.x ? t1 : t0;
@@ -57,6 +58,7 @@ __global__ void __launch_bounds__(512) k_eq_small(const EqTable t0, const EqTabl
 template <class F>
 __global__ void k_eq_outer(const uint32_t* hi, const uint32_t* lo, int m2, int64_t total,
                            uint32_t* out) {
+  pdl_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x)
     st4(out + 4 * i, ef_mul<F>(ld4(hi + 4 * (i >> m2)), ld4(lo + 4 * (i & ((1ll << m2) - 1)))));
@@ -78,16 +80,16 @@ inline size_t eq_ws_bytes(int m) {
 template <class F>
 zc_status eq_expand(const uint32_t* z, int m, uint32_t* out, uint32_t* ws, cudaStream_t st) {
   if (m <= kEqSmall) {
-    k_eq_small<F><<<1, 512, 0, st>>>(EqTable{z, m, out}, EqTable{});
+    pdl_launch(k_eq_small<F>, 1, 512, 0, st, EqTable{z, m, out}, EqTable{});
     return launch_check();
   }
   const int m1 = m / 2, m2 = m - m1;
   uint32_t* th = ws;
   uint32_t* tl = ws + ((size_t)4 << m1);
-  k_eq_small<F><<<2, 512, 0, st>>>(EqTable{z, m1, th}, EqTable{z + 4 * m1, m2, tl});
+  pdl_launch(k_eq_small<F>, 2, 512, 0, st, EqTable{z, m1, th}, EqTable{z + 4 * m1, m2, tl});
   ZC_TRY(launch_check());
   const int64_t total = (int64_t)1 << m;
-  k_eq_outer<F><<<grid_for(total, 256), 256, 0, st>>>(th, tl, m2, total, out);
+  pdl_launch(k_eq_outer<F>, grid_for(total, 256), 256, 0, st, th, tl, m2, total, out);
   return launch_check();
 }
 
@@ -114,6 +116,7 @@ template <class F>
 __global__ void __launch_bounds__(256) k_eval_inner(const uint32_t* cols, int w, int64_t S, int m2,
                                                     const uint32_t* lo, uint32_t* partial,
                                                     int64_t H) {
+  pdl_wait();
   const int64_t h = blockIdx.x;
   const int c0 = blockIdx.y * kEvalCols;
   const int64_t L = (int64_t)1 << m2;
@@ -128,7 +131,7 @@ __global__ void __launch_bounds__(256) k_eval_inner(const uint32_t* cols, int w,
     for (int c = 0; c < kEvalCols; c++) {
       if (c0 + c >= w) break;
       const uint32_t* col = cols + (c0 + c) * S + h * L + l;
-      ef_dot2<F>(acc[c], w0, __ldg(col), w1, two ? __ldg(col + blockDim.x) : 0u);
+      ef_dot2<F>(acc[c], w0, gld(col), w1, two ? gld(col + blockDim.x) : 0u);
     }
   }
 #pragma unroll
@@ -143,6 +146,7 @@ __global__ void __launch_bounds__(256) k_eval_inner(const uint32_t* cols, int w,
 template <class F>
 __global__ void __launch_bounds__(256) k_eval_outer(const uint32_t* partial, const uint32_t* hi,
                                                     int64_t H, uint32_t* out) {
+  pdl_wait();
   const int64_t c = blockIdx.x;
   ef4 acc{{0, 0, 0, 0}};
   for (int64_t h = threadIdx.x; h < H; h += blockDim.x)
@@ -175,16 +179,16 @@ zc_status eval_mle(const uint32_t* cols, int w, int m, const uint32_t* z, uint32
   uint32_t* eqws = partial + 4 * (size_t)w * H;
   // z[0 .. m1): high index bits, z[m1 .. m): low ones (m2 <= kEqSmall)
   if (m1 <= kEqSmall) {
-    k_eq_small<F><<<2, 512, 0, st>>>(EqTable{z, m1, hi}, EqTable{z + 4 * m1, m2, lo});
+    pdl_launch(k_eq_small<F>, 2, 512, 0, st, EqTable{z, m1, hi}, EqTable{z + 4 * m1, m2, lo});
     ZC_TRY(launch_check());
   } else {
     ZC_TRY(eq_expand<F>(z, m1, hi, eqws, st));
     ZC_TRY(eq_expand<F>(z + 4 * m1, m2, lo, eqws, st));
   }
-  k_eval_inner<F><<<dim3((unsigned)H, (unsigned)((w + kEvalCols - 1) / kEvalCols)), 256, 0, st>>>(
+  pdl_launch(k_eval_inner<F>, dim3((unsigned)H, (unsigned)((w + kEvalCols - 1) / kEvalCols)), 256, 0, st, 
       cols, w, S, m2, lo, partial, H);
   ZC_TRY(launch_check());
-  k_eval_outer<F><<<(unsigned)w, 256, 0, st>>>(partial, hi, H, out);
+  pdl_launch(k_eval_outer<F>, (unsigned)w, 256, 0, st, partial, hi, H, out);
   return launch_check();
 }
 
@@ -193,6 +197,7 @@ zc_status eval_mle(const uint32_t* cols, int w, int m, const uint32_t* z, uint32
 template <class F>
 __global__ void __launch_bounds__(256) k_sc_reduce(const uint32_t* mle, const uint32_t* eq,
                                                    int64_t M, uint32_t* partial) {
+  pdl_wait();
   ef4 acc{{0, 0, 0, 0}};
   for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < M;
        j += (int64_t)gridDim.x * blockDim.x)
@@ -207,6 +212,7 @@ template <class F>
 __global__ void __launch_bounds__(256) k_sc_message(const uint32_t* partial, int np,
                                                     const uint32_t* claim, const uint32_t* zinv,
                                                     uint32_t* msg) {
+  pdl_wait();
   ef4 acc{{0, 0, 0, 0}};
   for (int i = threadIdx.x; i < np; i += blockDim.x) acc = ef_add<F>(acc, ld4(partial + 4 * i));
   acc = block_sum<F>(acc);
@@ -225,7 +231,8 @@ template <class F>
 __global__ void k_sc_fold(const uint32_t* mle, int64_t M, const uint32_t* beta, int beta_limbs,
                           const uint32_t* msg, uint32_t* mle_out, const uint32_t* eq,
                           uint32_t* eq_out, uint32_t* claim) {
-  ef4 b{{__ldg(beta), 0, 0, 0}};
+  pdl_wait();
+  ef4 b{{gld(beta), 0, 0, 0}};
   if (beta_limbs == 4) b = ld4(beta);
   for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < M;
        j += (int64_t)gridDim.x * blockDim.x) {
@@ -250,7 +257,8 @@ __global__ void __launch_bounds__(256) k_sc_fold_reduce(const uint32_t* mle, int
                                                         const uint32_t* msg, uint32_t* mle_out,
                                                         const uint32_t* eq, uint32_t* eq_out,
                                                         uint32_t* claim, uint32_t* partial) {
-  ef4 b{{__ldg(beta), 0, 0, 0}};
+  pdl_wait();
+  ef4 b{{gld(beta), 0, 0, 0}};
   if (beta_limbs == 4) b = ld4(beta);
   const auto mul = [&](const ef4& x) { return beta_limbs == 4 ? ef_mul<F>(b, x) : ef_base<F>(x, b.c[0]); };
   ef4 acc{{0, 0, 0, 0}};
@@ -278,8 +286,8 @@ template <class F>
 __device__ __forceinline__ ef4 rlc_weight(const uint32_t* chal, int nbv, int idx) {
   ef4 w{{F::ONE, 0, 0, 0}};
   for (int j = 0; j < nbv; j++) {
-    const ef4 wr = ef_mul<F>(w, ef4{{__ldg(chal + 4 * j), __ldg(chal + 4 * j + 1),
-                                     __ldg(chal + 4 * j + 2), __ldg(chal + 4 * j + 3)}});
+    const ef4 wr = ef_mul<F>(w, ef4{{gld(chal + 4 * j), gld(chal + 4 * j + 1),
+                                     gld(chal + 4 * j + 2), gld(chal + 4 * j + 3)}});
     w = (idx >> (nbv - 1 - j)) & 1 ? wr : ef_sub<F>(w, wr);
   }
   return w;
@@ -295,6 +303,7 @@ template <class F>
 __global__ void __launch_bounds__(256) k_rlc_ex(const uint32_t* cw, int64_t n, int w,
                                                 const uint32_t* chal, int nbv, int offset,
                                                 int accumulate, uint32_t* out) {
+  pdl_wait();
   extern __shared__ __align__(16) uint32_t wt[];  // w x 4
   for (int c = threadIdx.x; c < w; c += blockDim.x)
     st4(wt + 4 * c, rlc_weight<F>(chal, nbv, offset + c));
@@ -306,15 +315,15 @@ __global__ void __launch_bounds__(256) k_rlc_ex(const uint32_t* cw, int64_t n, i
     const uint32_t* x = cw + j;
     int c = 0;
     for (; c + 4 <= w; c += 4) {
-      const uint32_t x0 = __ldg(x + c * n), x1 = __ldg(x + (c + 1) * n),
-                     x2 = __ldg(x + (c + 2) * n), x3 = __ldg(x + (c + 3) * n);
+      const uint32_t x0 = gld(x + c * n), x1 = gld(x + (c + 1) * n),
+                     x2 = gld(x + (c + 2) * n), x3 = gld(x + (c + 3) * n);
       ef_dot2<F>(r, ld4(wt + 4 * c), x0, ld4(wt + 4 * c + 4), x1);
       ef_dot2<F>(r, ld4(wt + 4 * c + 8), x2, ld4(wt + 4 * c + 12), x3);
     }
     for (; c < w; c += 2) {
       const bool two = c + 1 < w;
-      ef_dot2<F>(r, ld4(wt + 4 * c), __ldg(x + c * n),
-                 two ? ld4(wt + 4 * c + 4) : ef4{{0, 0, 0, 0}}, two ? __ldg(x + (c + 1) * n) : 0u);
+      ef_dot2<F>(r, ld4(wt + 4 * c), gld(x + c * n),
+                 two ? ld4(wt + 4 * c + 4) : ef4{{0, 0, 0, 0}}, two ? gld(x + (c + 1) * n) : 0u);
     }
     st4(out + 4 * j, r);
   }
@@ -326,6 +335,7 @@ template <class F>
 __global__ void __launch_bounds__(256) k_rlc_values(const uint32_t* values, int w,
                                                     const uint32_t* chal, int nbv, int offset,
                                                     int accumulate, uint32_t* out) {
+  pdl_wait();
   ef4 acc{{0, 0, 0, 0}};
   for (int c = threadIdx.x; c < w; c += blockDim.x)
     acc = ef_add<F>(acc, ef_mul<F>(rlc_weight<F>(chal, nbv, offset + c), ld4(values + 4 * c)));
@@ -336,6 +346,7 @@ __global__ void __launch_bounds__(256) k_rlc_values(const uint32_t* values, int 
 // [4][n] limbs <-> [n] EF4 words, for a transform that acts limb by limb.
 __global__ void __launch_bounds__(256) k_ef4_limbs(const uint32_t* in, int64_t n, int to_limbs,
                                                    uint32_t* out) {
+  pdl_wait();
   for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n;
        j += (int64_t)gridDim.x * blockDim.x) {
     if (to_limbs) {
@@ -358,7 +369,7 @@ zc_status rlc_launch(const uint32_t* cw, int64_t n, int w, const uint32_t* chal,
                                  (int)smem));
   int64_t blocks = (n + 255) / 256;
   if (blocks > 152 * 8) blocks = 152 * 8;
-  k_rlc_ex<F><<<(unsigned)blocks, 256, smem, st>>>(cw, n, w, chal, nbv, offset, accumulate, out);
+  pdl_launch(k_rlc_ex<F>, (unsigned)blocks, 256, smem, st, cw, n, w, chal, nbv, offset, accumulate, out);
   return launch_check();
 }
 
@@ -366,6 +377,7 @@ constexpr int kReduceBlocks = 256;
 
 template <class F>
 __global__ void k_ef4_inv(const uint32_t* in, uint32_t* out, int64_t count) {
+  pdl_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
        i += (int64_t)gridDim.x * blockDim.x)
     st4(out + 4 * i, ef_inv<F>(ld4(in + 4 * i)));
@@ -384,7 +396,7 @@ zc_status sc_first_partials(zc_field field, const uint32_t* mle, int64_t M, cons
   return with_field(field, [&](auto f) {
     using F = decltype(f);
     *np = sc_blocks(M);
-    k_sc_reduce<F><<<*np, 256, 0, st>>>(mle, eq, M, partial);
+    pdl_launch(k_sc_reduce<F>, *np, 256, 0, st, mle, eq, M, partial);
     return launch_check();
   });
 }
@@ -396,7 +408,7 @@ zc_status sc_fold_partials(zc_field field, const uint32_t* mle, int64_t M, const
   return with_field(field, [&](auto f) {
     using F = decltype(f);
     *np = sc_blocks(M / 2);
-    k_sc_fold_reduce<F><<<*np, 256, 0, st>>>(mle, M, beta, beta_limbs, msg, mle_out, eq, eq_out,
+    pdl_launch(k_sc_fold_reduce<F>, *np, 256, 0, st, mle, M, beta, beta_limbs, msg, mle_out, eq, eq_out,
                                              claim, partial);
     return launch_check();
   });
@@ -473,7 +485,7 @@ zc_status zc_ef4_limbs(const uint32_t* in, int64_t n, int32_t to_limbs, uint32_t
   if (n < 0 || (n > 0 && (!in || !out))) return ZC_BAD_ARG;
   if ((uintptr_t)(to_limbs ? in : out) % 16) return ZC_BAD_ARG;
   if (n == 0) return ZC_OK;
-  k_ef4_limbs<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(in, n, to_limbs, out);
+  pdl_launch(k_ef4_limbs, grid_for(n, 256), 256, 0, (cudaStream_t)stream, in, n, to_limbs, out);
   return launch_check();
 }
 
@@ -486,7 +498,7 @@ zc_status zc_rlc_values(zc_field field, const uint32_t* values, int32_t w,
   cudaStream_t st = (cudaStream_t)stream;
   return with_field(field, [&](auto f) {
     using F = decltype(f);
-    k_rlc_values<F><<<1, 256, 0, st>>>(values, w, challenges, nbv, offset, accumulate, out);
+    pdl_launch(k_rlc_values<F>, 1, 256, 0, st, values, w, challenges, nbv, offset, accumulate, out);
     return launch_check();
   });
 }
@@ -503,7 +515,7 @@ zc_status zc_ef4_inv(zc_field field, const uint32_t* in, uint32_t* out, int64_t 
   return with_field(field, [&](auto f) {
     using F = decltype(f);
     const int64_t blocks = std::min<int64_t>((count + 127) / 128, 152 * 4);
-    k_ef4_inv<F><<<(unsigned)blocks, 128, 0, st>>>(in, out, count);
+    pdl_launch(k_ef4_inv<F>, (unsigned)blocks, 128, 0, st, in, out, count);
     return launch_check();
   });
 }
@@ -522,9 +534,9 @@ zc_status zc_sumcheck_message(zc_field field, const uint32_t* mle, int64_t M, co
   return with_field(field, [&](auto f) -> zc_status {
     using F = decltype(f);
     const int blocks = (int)((M + 255) / 256 < kReduceBlocks ? (M + 255) / 256 : kReduceBlocks);
-    k_sc_reduce<F><<<blocks, 256, 0, st>>>(mle, eq, M, (uint32_t*)ws);
+    pdl_launch(k_sc_reduce<F>, blocks, 256, 0, st, mle, eq, M, (uint32_t*)ws);
     ZC_TRY(launch_check());
-    k_sc_message<F><<<1, 256, 0, st>>>((const uint32_t*)ws, blocks, claim, zinv, msg);
+    pdl_launch(k_sc_message<F>, 1, 256, 0, st, (const uint32_t*)ws, blocks, claim, zinv, msg);
     return launch_check();
   });
 }
@@ -541,7 +553,7 @@ zc_status zc_sumcheck_fold(zc_field field, const uint32_t* mle, int64_t M, const
   cudaStream_t st = (cudaStream_t)stream;
   return with_field(field, [&](auto f) {
     using F = decltype(f);
-    k_sc_fold<F><<<grid_for(M, 256), 256, 0, st>>>(mle, M, beta, beta_limbs, msg, mle_out, eq,
+    pdl_launch(k_sc_fold<F>, grid_for(M, 256), 256, 0, st, mle, M, beta, beta_limbs, msg, mle_out, eq,
                                                    eq_out, claim);
     return launch_check();
   });
