@@ -21,8 +21,6 @@
 
 namespace zc {
 
-constexpr int kMaxT = 256;
-
 // Leaf p = concat over q < G of base[q*gs + p*g .. +g] (zc_leaves).
 struct LayoutLeaf {
   const uint32_t* base;
@@ -232,7 +230,7 @@ struct FoldLeaf {
 
 // Nodes per tree-top CTA of the batched commit (k_tree_top) at its first
 // level; its threads: 4 per node, so every level above is one round
-// (subtree_level: quarter-warps while a level has more than 32 parents,
+// (subtree_level: quarter-warps while a level has more than 16 parents,
 // half-warps above).
 constexpr int kSubT = 128;
 // Largest number of nodes per fused-subtree CTA (k_subtree) at its first
@@ -353,9 +351,9 @@ __device__ __forceinline__ void subtree_level(const uint32_t* src, uint32_t* dst
 // commit of 2^16: 111 us against 115). Barrier 1 is the tree's, 2 the root's;
 // every warp of the tree reaches both.
 template <class K, class Leaf, bool HOP>
-__global__ void __launch_bounds__(kSubThreads + 32, 1) k_subtree(Leaf leaf, uint32_t* layers, int64_t L,
-                                                       int l0, int T, const P2Params* rt,
-                                                       const RoundHop hop) {
+__global__ void __launch_bounds__(kSubThreads + 32, 1)
+    k_subtree(Leaf leaf, uint32_t* layers, int64_t L, int l0, int T, const P2Params* rt,
+              const RoundHop hop) {
   __shared__ P2Params s_rt;
   __shared__ __align__(16) uint32_t sm[2][8 * kSubCap];  // [node][word] digest slots
   KIn<K>::make(rt, &s_rt);
@@ -415,9 +413,7 @@ __global__ void __launch_bounds__(kSubThreads + 32, 1) k_subtree(Leaf leaf, uint
 // threads measured 1.74 ms where 256 took 1.76-1.79 for 2^20 x 8 permutations);
 // no bound for run-time parameter sets, whose constants come from shared memory
 // and which would spill under it. Small CTAs also spread a narrow level over
-// every SM: 2^15 parents are 256 CTAs, not 128. The batched tree kernel keeps
-// the compiler's choice: bounding it to five or six resident CTAs measured
-// slower on the served stream (1.136 / 1.153 against 1.163 G elem/s).
+// every SM: 2^15 parents are 256 CTAs, not 128.
 constexpr int kLeafT = 128;
 template <class K>
 struct HashOcc {

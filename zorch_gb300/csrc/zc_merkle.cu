@@ -64,8 +64,8 @@ __global__ void __launch_bounds__(32) k_bind_root(const P2Params* rt, const uint
 
 // ------------------------------------------------------------ batched ----
 // Many trees (leaf layouts of different widths and heights) per launch: a leaf
-// launch over (tree, 256-leaf chunk) items, one launch per level over
-// (tree, 256-parent chunk) items for every tree that still has a wide level,
+// launch over (tree, 128-leaf chunk) items, one launch per level over
+// (tree, 128-parent chunk) items for every tree that still has a wide level,
 // and one top launch with one CTA per tree compressing its last <= 256 nodes
 // to the root in shared memory. The tree table is a __grid_constant__ kernel
 // parameter; CTAs claim items from an atomic counter (dynamic balance across
@@ -82,7 +82,7 @@ struct TreeJobDev {
   int64_t L;
   int64_t gs;
   int64_t bstride, lstride;
-  int64_t chunks;  // 256-node chunks per tree at the level being produced
+  int64_t chunks;  // kBatchT-node chunks per tree at the level being produced
   int32_t G, g;
   int32_t depth, top;
   int32_t count;
@@ -107,25 +107,43 @@ __device__ __forceinline__ int find_tree(const int64_t* prefix, int njobs, int64
   return lo;
 }
 
-// LEVEL = 0: leaf chunks; LEVEL = 1: parent chunks of B.level.
+// Nodes per work item and threads per CTA of k_tree_batch, and the CTAs per SM it
+// is compiled for: k_leaf's shape, for the same reason (the built-in permutation
+// at 62 registers instead of 40). A batch of 16 uneven matrices 13.18 -> 12.69 ms,
+// the served per-polynomial stream 1.24 -> 1.31 G elem/s; items of 256 on four
+// CTAs: 12.88 ms and 1.28. Without the early claim below 13.23.
+constexpr int kBatchT = 128;
+template <class K>
+struct BatchOcc {
+  static constexpr int v = 1;
+};
+template <>
+struct BatchOcc<Bb16Builtin> {
+  static constexpr int v = 8;
+};
+
+// LEVEL = 0: leaf chunks; LEVEL = 1: parent chunks of B.level. The next item is
+// claimed while this one is computed.
 template <class K, int LEVEL>
-__global__ void __launch_bounds__(kMaxT) k_tree_batch(const __grid_constant__ TreeBatch B,
-                                                      unsigned long long* counter,
-                                                      const P2Params* rt) {
+__global__ void __launch_bounds__(kBatchT, BatchOcc<K>::v)
+    k_tree_batch(const __grid_constant__ TreeBatch B, unsigned long long* counter,
+                 const P2Params* rt) {
   __shared__ P2Params s_rt;
-  __shared__ long long s_item;
+  __shared__ long long s_item[2];
   K k = KIn<K>::make(rt, &s_rt);
+  long long next = 0;
+  if (threadIdx.x == 0) s_item[0] = (long long)atomicAdd(counter, 1ull);
   for (int done = 0; kItemsPerCta == 0 || done < kItemsPerCta; done++) {
-    if (threadIdx.x == 0) s_item = (long long)atomicAdd(counter, 1ull);
     __syncthreads();
-    const int64_t it = s_item;
-    __syncthreads();
+    const int64_t it = s_item[done & 1];
     if (it >= B.total) break;
+    if (threadIdx.x == 0 && (kItemsPerCta == 0 || done + 1 < kItemsPerCta))
+      next = (long long)atomicAdd(counter, 1ull);
     const int j = find_tree(B.prefix, B.njobs, it);
     const TreeJobDev& J = B.job[j];
     const int64_t local = it - B.prefix[j];
     const int64_t tree = local / J.chunks;
-    const int64_t p = (local - tree * J.chunks) * kMaxT + threadIdx.x;
+    const int64_t p = (local - tree * J.chunks) * kBatchT + threadIdx.x;
     uint32_t* lay = J.layers + tree * J.lstride;
     uint32_t d[8];
     if (LEVEL == 0) {
@@ -142,12 +160,13 @@ __global__ void __launch_bounds__(kMaxT) k_tree_batch(const __grid_constant__ Tr
         store_digest(lay + 8 * (level_offset(J.L, l) + p), d);
       }
     }
+    if (threadIdx.x == 0) s_item[(done + 1) & 1] = next;
   }
 }
 
 // One CTA per tree: level `top` (<= 256 nodes, already stored) to the root,
 // each level compressed in one round (subtree_level: quarter-warps for the
-// levels wider than 32 parents, half-warps above).
+// levels wider than 16 parents, half-warps above).
 template <class K>
 __global__ void __launch_bounds__(4 * kSubT) k_tree_top(const __grid_constant__ TreeBatch B,
                                                        const P2Params* rt) {
@@ -205,13 +224,13 @@ zc_status tree_batch_wave(const zc_merkle_job* jobs, int n, unsigned long long* 
   int dev = 0, sms = 0, occ = 0;
   ZC_CUDA(cudaGetDevice(&dev));
   ZC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  ZC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tree_batch<K, 0>, kMaxT, 0));
+  ZC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tree_batch<K, 0>, kBatchT, 0));
   for (int l = 0; l <= max_top; l++) {
     int64_t tot = 0;
     for (int i = 0; i < n; i++) {
       TreeJobDev& d = B.job[i];
       B.prefix[i] = tot;
-      d.chunks = ((d.L >> l) + kMaxT - 1) / kMaxT;
+      d.chunks = ((d.L >> l) + kBatchT - 1) / kBatchT;
       if (l == 0 || l <= d.top) tot += d.chunks * d.count;
     }
     B.prefix[n] = tot;
@@ -220,9 +239,9 @@ zc_status tree_batch_wave(const zc_merkle_job* jobs, int n, unsigned long long* 
     if (tot == 0) continue;
     const int64_t grid = batch_grid(tot, occ, sms);
     if (l == 0)
-      k_tree_batch<K, 0><<<(unsigned)grid, kMaxT, 0, st>>>(B, ctr + l, rt);
+      k_tree_batch<K, 0><<<(unsigned)grid, kBatchT, 0, st>>>(B, ctr + l, rt);
     else
-      k_tree_batch<K, 1><<<(unsigned)grid, kMaxT, 0, st>>>(B, ctr + l, rt);
+      k_tree_batch<K, 1><<<(unsigned)grid, kBatchT, 0, st>>>(B, ctr + l, rt);
     ZC_TRY(launch_check());
   }
   if (trees > 0x7fffffff) return ZC_BAD_SHAPE;
