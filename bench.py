@@ -1085,17 +1085,17 @@ def main():
     # Hash kernel (dominant): integer instructions executed per Poseidon2
     # permutation of the built-in BabyBear-16 instance, from the ncu capture
     # summarised in profiles/ (thread-level SASS instructions).
-    inst_per_perm = float(os.environ.get("ZC_INST_PER_PERM", "6070"))
-    # DRAM bytes per hashed LDE word of the k_leaf launch (134.27 MB read +
-    # 8.60 MB written for 2^19 leaves x 64 words, profiles/), scaled to this
+    inst_per_perm = float(os.environ.get("ZC_INST_PER_PERM", "5407"))
+    # DRAM bytes per hashed LDE word of the k_leaf launch (134.25 MB read +
+    # 8.98 MB written for 2^19 leaves x 64 words, profiles/), scaled to this
     # workload's leaf launch by its word count.
-    traffic_per_word = (134.273792e6 + 8.598272e6) / float(1 << 25)
+    traffic_per_word = (134.249728e6 + 8.975616e6) / float(1 << 25)
     perms = info["perms_leaf"] + info["perms_node"]
     sms = torch.cuda.get_device_properties(device).multi_processor_count
     int_peak = sms * 128 * sm_mhz * 1e6 / 1e9  # Ginst/s: SMs x 128 lanes x clock
     peak_src = (f"{sms} SMs (cudaDevAttrMultiProcessorCount) x 128 lanes x sm_max_mhz "
                 "(MEASURED_PEAKS.json): the thread-instruction issue peak")
-    binding = ("FMA-heavy pipe (the Montgomery products' wide and high multiplies): 81 % of "
+    binding = ("FMA-heavy pipe (the Montgomery products' wide and high multiplies): 92 % of "
                "its peak cycles in the ncu capture of the leaf launch "
                "(profiles/k_leaf_poseidon2_trace_2p17x64_blowup4.md)")
 
@@ -1111,9 +1111,9 @@ def main():
     # butterflies' own: log2(k)/2 = 8.5 radix-2 butterflies per output word at
     # ~11 field instructions each.
     lde_wide = {"binding_unit": "integer issue at 512 threads per SM (128 registers per "
-                                "thread; issue active 49-55 % in the ncu capture), not HBM",
-                "inst_per_output_word": 136.7, "butterfly_floor_per_output_word": 93.5,
-                "issue_frac": 93.5 / 136.7,
+                                "thread; issue active 51-54 % in the ncu capture), not HBM",
+                "inst_per_output_word": 129.8, "butterfly_floor_per_output_word": 93.5,
+                "issue_frac": 93.5 / 129.8,
                 "issue_source": "profiles/k_lde_wide_trace_2p17x64_blowup4.md"}
 
     def ntt_roof(bytes_, ms_, kernel, issue):
