@@ -239,8 +239,10 @@ constexpr int kSubCap = 256;
 
 // The tree driver's shape: levels with more than `levelwise_min` nodes run one
 // thread per node; the top runs as fused subtrees of `subtree_t` first-level
-// nodes per CTA. Defaults 2^14 and 128 (the 2^22 FRI commit phase, graphed:
-// 6.01 ms against 6.08 at 2^13, 6.12 at 2^15, 6.18 with 256-node subtrees).
+// nodes per CTA. Defaults 2^14 and 128 (the 2^22 FRI commit phase, event-timed
+// call by call: 4.82 ms against 4.84 at 2^13, 4.99 at 2^15, 5.00 with 256-node
+// subtrees; 64-node ones 4.78 there, but 2.15 against 2.13 ms for the Basefold
+// open of 2^20 x 8).
 // The environment variables ZC_LEVELWISE_MIN_LOG (8..20) and ZC_SUBTREE_T (a
 // power of two in 2..256) override them for tuning (read once; no byte of any
 // result depends on them).
@@ -409,7 +411,7 @@ __global__ void __launch_bounds__(kSubThreads + 32, 1)
 }
 
 // Threads of a k_leaf CTA, and the CTAs per SM it is compiled for: eight for the
-// built-in instance (46 registers; the register file then holds ten, and 128
+// built-in instance (54 registers; the register file then holds nine, and 128
 // threads measured 1.74 ms where 256 took 1.76-1.79 for 2^20 x 8 permutations);
 // no bound for run-time parameter sets, whose constants come from shared memory
 // and which would spill under it. Small CTAs also spread a narrow level over
