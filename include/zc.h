@@ -110,6 +110,9 @@ zc_status zc_poseidon2_create(zc_field field, int alpha, int rounds_f_half, int 
                               const uint32_t* int_rc, const uint32_t* diag,
                               uint32_t j_scale, zc_poseidon2** out);
 zc_status zc_poseidon2_destroy(zc_poseidon2* p);
+/* 1 if the two handles are one permutation (the same field, exponent, rounds and
+ * constants), else 0. Host only. */
+int32_t zc_poseidon2_equal(const zc_poseidon2* a, const zc_poseidon2* b);
 /* Permute `count` independent 16-word states in place (hash-frx Permutation.permute). */
 zc_status zc_poseidon2_permute(const zc_poseidon2* p, uint32_t* states, int64_t count,
                                void* stream);
@@ -415,7 +418,8 @@ typedef struct {
   uint32_t* layers;        /* layers 1 .. rounds-1, one after the other */
   uint32_t* trees;         /* their digest layers, one after the other */
   uint32_t* final_layer;   /* layer `rounds` */
-  uint32_t* state;         /* the 34-word duplex state, advanced in place */
+  uint32_t* state;         /* the 34-word duplex state over the call's permutation,
+                            * advanced in place */
   uint32_t* betas;         /* [rounds][beta_limbs] */
   uint32_t* roots;         /* [rounds][8], as observed */
   uint32_t* raw_roots;     /* [rounds][8] before binding, or NULL */

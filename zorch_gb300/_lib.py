@@ -83,6 +83,7 @@ def _declare(lib: C.CDLL) -> None:
         "zc_poseidon2_create": (st, [st, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, u32,
                                      C.POINTER(vp)]),
         "zc_poseidon2_destroy": (st, [vp]),
+        "zc_poseidon2_equal": (i32, [vp, vp]),
         "zc_poseidon2_permute": (st, [vp, vp, i64, vp]),
         "zc_poseidon2_permute_host": (st, [vp, vp, i64]),
         "zc_rs_encode_workspace_bytes": (sz, [i64, C.c_int, C.c_int]),

@@ -57,6 +57,11 @@ class Poseidon2:
     def handle(self) -> int:
         return self._h
 
+    def same_as(self, other: "Poseidon2") -> bool:
+        """Whether both are one permutation: the same handle or equal constants."""
+        return (self._h == other._h
+                or bool(_lib.lib().zc_poseidon2_equal(self._h, other._h)))
+
     def permute(self, states: torch.Tensor) -> torch.Tensor:
         """Permute [count, 16] states (a copy is returned)."""
         s = states.contiguous().clone()

@@ -323,6 +323,11 @@ zc_status zc_poseidon2_create(zc_field field, int alpha, int rounds_f_half, int 
   return ZC_OK;
 }
 
+// host is zeroed before its words are set, so the whole block compares.
+int32_t zc_poseidon2_equal(const zc_poseidon2* a, const zc_poseidon2* b) {
+  return a && b && a->field == b->field && memcmp(&a->host, &b->host, sizeof(a->host)) == 0;
+}
+
 zc_status zc_poseidon2_destroy(zc_poseidon2* p) {
   if (!p || p->builtin) return ZC_BAD_ARG;
   if (p->dev) cudaFree(p->dev);

@@ -20,7 +20,8 @@ import torch
 
 from . import _lib
 from .coding import ReedSolomon
-from .commit import DigestLayers, MerkleTree, Opening, leaves_layout
+from .commit import (DigestLayers, MerkleTree, Opening, Poseidon2, SingleMatrixCommitmentScheme,
+                     leaves_layout)
 from .field import full_u32, parts_to_bytes, ptr, stream_handle, to_host
 from .stage import (OpeningClaim, OpeningProof, OpeningWitness, ProveResult, TrivialClaim,
                     VerifyResult)
@@ -58,6 +59,12 @@ def pair_layout(layer: torch.Tensor, bit_reversed: bool = False) -> _lib.Leaves:
     if bit_reversed:
         return leaves_layout(layer, n // 2, 1, 2 * limbs, 0)
     return leaves_layout(layer, n // 2, 2, limbs, (n // 2) * limbs)
+
+
+def hop_in_tree(perm: Poseidon2, t) -> bool:
+    """Whether the launches of a tree over `perm` can run `t`'s steps: a device
+    transcript over the same permutation."""
+    return type(t) is DuplexTranscript and perm.same_as(t.permutation)
 
 
 @dataclass
@@ -108,7 +115,8 @@ class PreFoldPairCommitRound:
     # computes the root (zc_merkle_commit_hop / zc_fri_fold_commit_hop): one
     # launch fewer per round. The transcript a round returns is then already
     # past the next round's hop, so this is only for rounds that follow each
-    # other directly on one transcript (FriProver.commit_phase).
+    # other directly on one transcript. The launch has one permutation: over
+    # another one than the tree's, the transcript keeps its own launch.
     fuse_hop: bool = False
 
     def commit_layer(self, cw: torch.Tensor) -> CommittedLayer:
@@ -117,6 +125,9 @@ class PreFoldPairCommitRound:
 
     def commit_layer_hop(self, cw: torch.Tensor, t: DuplexTranscript):
         """commit_layer, then observe(root) + sample(beta) in the root's launch."""
+        if not hop_in_tree(self.tree.perm, t):
+            layer = self.commit_layer(cw)
+            return layer, t.observe_and_sample_(layer.root, self.challenge_limbs)
         L = cw.shape[0] // 2
         flat = torch.empty((2 * L - 1, 8), dtype=torch.int32, device=cw.device)
         beta = torch.empty(self.challenge_limbs, dtype=torch.int32, device=cw.device)
@@ -154,6 +165,9 @@ class PreFoldPairCommitRound:
         """The fold of this round fused with the commit of the next layer;
         with `hop`, also that layer's observe(root) + sample(beta) on `hop`
         (in place), returning the sampled beta as a third value."""
+        if hop is not None and not hop_in_tree(self.tree.perm, hop):
+            out, layer = self.fold_commit(cw, beta, level)
+            return out, layer, hop.observe_and_sample_(layer.root, self.challenge_limbs)
         n = cw.shape[0]
         ef_in = cw.dim() == 2
         ef_beta = beta.numel() == 4
@@ -289,7 +303,13 @@ def run_fold_rounds(perm, code, codeword: torch.Tensor, rounds: int, limbs: int,
     (zorch/pcs/fold.py:90-115), launched by one call (zc_fold_rounds). `t`
     advances in place. `bind` observes SP1's bound roots; `sumcheck` = (mle
     [2^rounds, 4], eq, claim, zinv) interleaves the sumcheck of the Basefold
-    opens, advancing `claim`."""
+    opens, advancing `claim`. The call has one permutation and one field: a
+    transcript over another permutation than the tree's `perm` takes the same
+    rounds step by step (step_fold_rounds), and so does a code over another
+    field."""
+    if not (hop_in_tree(perm, t) and perm.field.id == code.field.id and limbs in (1, 4)):
+        return step_fold_rounds(MerkleTree(perm), code, codeword, rounds, limbs, t, first_layer,
+                                bind, sumcheck)
     dev = codeword.device
     n = codeword.shape[0]
     log_n = n.bit_length() - 1
@@ -335,6 +355,54 @@ def run_fold_rounds(perm, code, codeword: torch.Tensor, rounds: int, limbs: int,
         layers += [CommittedLayer(c.view(-1, 4) if lo == 4 else c, DigestLayers(tr, m))
                    for c, tr, m in zip(cw_parts, tree_parts, leaves)]
     return FoldRounds(layers, roots, raw, betas, final, msgs)
+
+
+def step_fold_rounds(tree: MerkleTree, code, codeword: torch.Tensor, rounds: int, limbs: int,
+                     t: DuplexTranscript, first_layer: CommittedLayer | None = None,
+                     bind: bool = False, sumcheck: tuple | None = None) -> FoldRounds:
+    """run_fold_rounds with a launch for each step: the tree's steps run `tree`'s
+    permutation and the transcript's its own."""
+    f, dev, L = code.field, codeword.device, _lib.lib()
+    rnd = PreFoldPairCommitRound(code, tree, limbs)
+    layers, roots, raws, betas = [], [], [], []
+    msgs = scws = None
+    scb = L.zc_sumcheck_workspace_bytes()
+    if sumcheck is not None:
+        mle, eq, claim, zinv = sumcheck
+        msgs = torch.empty((rounds, 8), dtype=torch.int32, device=dev)
+        scws = torch.empty((scb + 3) // 4, dtype=torch.int32, device=dev)
+    cw, pending = codeword, first_layer
+    for i in range(rounds):
+        M = 1 << (rounds - 1 - i)
+        if sumcheck is not None:
+            _lib.check(L.zc_sumcheck_message(f.id, ptr(mle), M, ptr(eq), ptr(claim),
+                                             ptr(zinv[rounds - 1 - i]), ptr(msgs[i]), ptr(scws),
+                                             scb, stream_handle()), "sumcheck_message")
+            t.observe_(msgs[i])
+        layer = pending if pending is not None else rnd.commit_layer(cw)
+        root = layer.root
+        if bind:
+            raws.append(root)
+            root = SingleMatrixCommitmentScheme(tree.perm).bind_root(
+                root, layer.digest_layers.depth, 2 * layer.limbs)
+        beta = t.observe_and_sample_(root, limbs)
+        if i < rounds - 1 and cw.shape[0] >= 4:
+            cw, pending = rnd.fold_commit(cw, beta, i)
+        else:
+            cw, pending = code.fold(cw, beta), None
+        if sumcheck is not None:
+            mle_next = torch.empty((M, 4), dtype=torch.int32, device=dev)
+            eq_next = torch.empty((M // 2, 4), dtype=torch.int32, device=dev) if M >= 2 else None
+            _lib.check(L.zc_sumcheck_fold(f.id, ptr(mle), M, ptr(beta), limbs, ptr(msgs[i]),
+                                          ptr(mle_next), ptr(eq) if M >= 2 else None,
+                                          ptr(eq_next), ptr(claim), stream_handle()),
+                       "sumcheck_fold")
+            mle, eq = mle_next, eq_next
+        layers.append(layer)
+        roots.append(root)
+        betas.append(beta)
+    return FoldRounds(layers, stack_rows(roots, (8,), dev), stack_rows(raws) if bind else None,
+                      stack_rows(betas, (limbs,), dev), cw, msgs)
 
 
 def open_layers(specs: Sequence[tuple], positions: torch.Tensor) -> list[Opening]:
@@ -454,16 +522,11 @@ class FriProver:
         if 1 <= p.num_rounds <= n0.bit_length() - 1 and n0 & (n0 - 1) == 0:
             fr = run_fold_rounds(p.tree.perm, p.code, codeword, p.num_rounds, p.challenge_limbs,
                                  t, first_layer)
-            betas, roots = fr.betas.unbind(0), fr.roots
-            state = FoldState(fr.final_layer, tuple(fr.layers), None, betas)
         else:  # no round, or more rounds than halvings (refused by the rounds)
-            rnd = PreFoldPairCommitRound(p.code, p.tree, p.challenge_limbs,
-                                         last_round=p.num_rounds - 1)
-            state, moved, msgs = fold_rounds(rnd, FoldState(codeword, (), first_layer), t,
-                                             p.num_rounds)
-            t.state = moved.state
-            betas, roots = state.betas, stack_rows(msgs, (8,), codeword.device)
-        final = state.codeword
+            fr = step_fold_rounds(p.tree, p.code, codeword, p.num_rounds, p.challenge_limbs, t,
+                                  first_layer)
+        betas, roots, final = fr.betas.unbind(0), fr.roots, fr.final_layer
+        state = FoldState(final, tuple(fr.layers), None if fr.layers else first_layer, betas)
         positions = t.sample_positions_(n0, p.num_queries, values=final)
         specs = [layer_spec(layer, i, br) for i, layer in enumerate(state.layers)]
         ops = open_layers([*specs, *extra], positions) if specs or extra else []
