@@ -295,6 +295,31 @@ class FoldRounds:
     msgs: torch.Tensor | None = None
 
 
+def check_fold_rounds(codeword: torch.Tensor, rounds: int,
+                      first_layer: CommittedLayer | None, sumcheck: tuple | None) -> None:
+    """The sizes that run_fold_rounds' launches take from the codeword and the
+    number of rounds alone (ValueError)."""
+    n = codeword.shape[0]
+    if n < 2 or n & (n - 1) or codeword.shape[1:] not in ((), (4,)):
+        raise ValueError("the fold rounds take a codeword [n] or [n, 4], n >= 2 a power of two, "
+                         f"got {tuple(codeword.shape)}")
+    if not 1 <= rounds <= n.bit_length() - 1:
+        raise ValueError(f"a codeword of {n} takes 1 to {n.bit_length() - 1} rounds, got {rounds}")
+    if first_layer is not None:
+        dl = first_layer.digest_layers
+        if (first_layer.codeword.shape != codeword.shape or dl.num_leaves != n // 2
+                or dl.flat.numel() != 8 * (n - 1)):
+            raise ValueError(f"the first layer is not the pair commit of a codeword of {n}: "
+                             f"{tuple(first_layer.codeword.shape)} with {dl.num_leaves} leaves "
+                             f"and {tuple(dl.flat.shape)} digest words")
+    if sumcheck is not None:
+        want = (4 << rounds, 2 << rounds, 4, 4 * rounds)  # EF4 mle, eq, claim, zinv
+        got = tuple(x.numel() for x in sumcheck)
+        if got != want:
+            raise ValueError(f"a sumcheck of {rounds} rounds takes mle, eq, claim and zinv of "
+                             f"{want} words, got {got}")
+
+
 def run_fold_rounds(perm, code, codeword: torch.Tensor, rounds: int, limbs: int,
                     t: DuplexTranscript, first_layer: CommittedLayer | None = None,
                     bind: bool = False, sumcheck: tuple | None = None) -> FoldRounds:
@@ -306,7 +331,8 @@ def run_fold_rounds(perm, code, codeword: torch.Tensor, rounds: int, limbs: int,
     opens, advancing `claim`. The call has one permutation and one field: a
     transcript over another permutation than the tree's `perm` takes the same
     rounds step by step (step_fold_rounds), and so does a code over another
-    field."""
+    field. Shapes that do not fit one another are refused before any launch."""
+    check_fold_rounds(codeword, rounds, first_layer, sumcheck)
     if not (hop_in_tree(perm, t) and perm.field.id == code.field.id and limbs in (1, 4)):
         return step_fold_rounds(MerkleTree(perm), code, codeword, rounds, limbs, t, first_layer,
                                 bind, sumcheck)
@@ -408,7 +434,14 @@ def step_fold_rounds(tree: MerkleTree, code, codeword: torch.Tensor, rounds: int
 def open_layers(specs: Sequence[tuple], positions: torch.Tensor) -> list[Opening]:
     """Openings of the same positions in several trees, one launch
     (zc_open_layers): specs are (leaf layout, digest layers, leaf width, shift),
-    each opened at leaf (position >> shift) mod num_leaves."""
+    each opened at leaf (position >> shift) mod num_leaves. A tree that is not the
+    layout's is refused (ValueError): the kernel takes its depth from the layout."""
+    for lv, dl, width, _ in specs:
+        if (dl.num_leaves != lv.num_leaves or dl.flat.numel() != 8 * (2 * lv.num_leaves - 1)
+                or width != lv.groups * lv.group_len):
+            raise ValueError(f"opening of {lv.num_leaves} leaves of {lv.groups * lv.group_len} "
+                             f"words: the tree has {dl.num_leaves} leaves and "
+                             f"{tuple(dl.flat.shape)} digest words, the width is {width}")
     idx = positions.to(torch.int32).contiguous()
     q = idx.numel()
     sizes = []
