@@ -101,6 +101,10 @@ zc_status fold_scalars(int64_t n, uint32_t shift_mont, uint32_t generator, FoldS
     return ZC_UNSUPPORTED;
   }
   const int log_n = ilog2(n);
+  if (log_n > F::TWO_ADICITY) {
+    set_error("a layer exceeds the field's two-adic range");
+    return ZC_BAD_SHAPE;
+  }
   const uint32_t w = root_of_unity<F>(log_n, generator);
   o->winv = minv<F>(w);
   const uint32_t sh = shift_mont ? shift_mont : F::ONE;

@@ -106,8 +106,27 @@ zc_status zc_fold_rounds(const zc_poseidon2* p, const zc_fold_rounds_desc* d, vo
       return ZC_BAD_ARG;
     if (d->workspace_bytes < 4 * ws.total) return ZC_OOM;
   }
-  cudaStream_t st = (cudaStream_t)stream;
   const zc_field field = p->field;
+  // Whatever the folds would refuse is refused here, before the first hop moves
+  // the transcript.
+  ZC_TRY(with_field(field, [&](auto f) -> zc_status {
+    using F = decltype(f);
+    if (d->log_n > F::TWO_ADICITY) {
+      set_error("fold rounds: the codeword exceeds the field's two-adic range");
+      return ZC_BAD_SHAPE;
+    }
+    if (d->generator != 0 && d->generator != F::GEN) {
+      set_error("only the field's canonical generator is built");
+      return ZC_UNSUPPORTED;
+    }
+    for (int r = 0; r < d->rounds; r++)
+      if (d->shifts[r] >= F::P) {
+        set_error("fold rounds: a coset shift is no field element");
+        return ZC_BAD_ARG;
+      }
+    return ZC_OK;
+  }));
+  cudaStream_t st = (cudaStream_t)stream;
   const int ef_beta = d->beta_limbs == 4;
   const uint32_t *cw = d->codeword, *mle = d->mle, *eq = d->eq;
   uint32_t *layers = d->layers, *trees = d->trees;
