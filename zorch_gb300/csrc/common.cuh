@@ -54,6 +54,19 @@ inline void pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// Lets a launch of `kernel` use `smem` bytes of dynamic shared memory. The limit is
+// a property of the kernel, shared by all threads: it is always set to the largest
+// value (an SM's 227 KB, less `fixed` for the kernel's own arrays), so that no
+// thread lowers it between another's call and launch. Up to 48 KB need no limit.
+constexpr size_t kSmemMax = 227 * 1024;
+template <class... P>
+inline zc_status allow_smem(void (*kernel)(P...), size_t smem, size_t fixed = 0) {
+  if (smem <= 48 * 1024) return ZC_OK;
+  const size_t limit = smem > kSmemMax - fixed ? smem : kSmemMax - fixed;
+  ZC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+  return ZC_OK;
+}
+
 // Once the previous kernel is complete and its writes are visible.
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -685,8 +685,7 @@ zc_status lde_launch(const uint32_t* x, int64_t batch, int log_k, int log_b, uin
     return ZC_UNSUPPORTED;
   }
   if (p.small) {
-    ZC_CUDA(cudaFuncSetAttribute(k_lde_small<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)p.smem_small));
+    ZC_TRY(allow_smem(k_lde_small<F>, p.smem_small));
     for (int64_t c0 = 0; c0 < batch; c0 += 0x7fffffff) {
       const int64_t cols = batch - c0 < 0x7fffffff ? batch - c0 : 0x7fffffff;
       pdl_launch(k_lde_small<F>, (unsigned)cols, kThreads, p.smem_small, st, 
@@ -715,9 +714,8 @@ zc_status lde_four_step(const uint32_t* x, int64_t batch, int log_k, int log_b, 
   if (chunk > 65535) chunk = 65535;
   if (chunk > batch) chunk = batch;
   const auto pass1 = rev ? k_lde_pass1<F, MR, true> : k_lde_pass1<F, MR, false>;
-  ZC_CUDA(cudaFuncSetAttribute(pass1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem1));
-  ZC_CUDA(cudaFuncSetAttribute(k_lde_pass2<F, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)p.smem2));
+  ZC_TRY(allow_smem(pass1, p.smem1));
+  ZC_TRY(allow_smem(k_lde_pass2<F, MR>, p.smem2));
   uint32_t* z = (uint32_t*)ws;
   for (int64_t c0 = 0; c0 < batch; c0 += chunk) {
     const int64_t cols = batch - c0 < chunk ? batch - c0 : chunk;
@@ -860,8 +858,7 @@ zc_status lde_batch_wave(const zc_lde_job* jobs, int n, uint32_t* zbase, unsigne
     B.phase = phase;
     B.total = total;
     if (phase) memcpy(B.prefix, prefB, sizeof(prefB));
-    ZC_CUDA(cudaFuncSetAttribute(k_lde_batch<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
+    ZC_TRY(allow_smem(k_lde_batch<F>, smem, 1024));
     int dev = 0, sms = 0, occ = 0;
     ZC_CUDA(cudaGetDevice(&dev));
     ZC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

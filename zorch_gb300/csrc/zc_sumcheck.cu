@@ -364,9 +364,7 @@ template <class F>
 zc_status rlc_launch(const uint32_t* cw, int64_t n, int w, const uint32_t* chal, int nbv,
                      int offset, int accumulate, uint32_t* out, cudaStream_t st) {
   const size_t smem = (size_t)16 * w;
-  if (smem > 48 * 1024)
-    ZC_CUDA(cudaFuncSetAttribute(k_rlc_ex<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
+  ZC_TRY(allow_smem(k_rlc_ex<F>, smem));
   int64_t blocks = (n + 255) / 256;
   if (blocks > 152 * 8) blocks = 152 * 8;
   pdl_launch(k_rlc_ex<F>, (unsigned)blocks, 256, smem, st, cw, n, w, chal, nbv, offset, accumulate, out);
