@@ -22,8 +22,8 @@ struct Duplex {
 // _observe_body (zorch/transcript.py:637-748): the stream in_buf[0:in_pos] ++
 // values is absorbed a full rate block at a time (overwrite sponge[0:8],
 // permute); the tail stays pending; a fresh output iff no tail remains.
-// `perm(s)` permutes the 16-word sponge in place: one thread on the host, a
-// half-warp on the device (HalfPerm).
+// `perm(s)` permutes the 16-word sponge in place. The host's form; the device's is
+// LaneDuplex.
 #pragma nv_exec_check_disable
 template <class Perm>
 ZC_HD void duplex_observe(Duplex& t, const uint32_t* v, int64_t m, const Perm& perm) {

@@ -172,9 +172,8 @@ static __constant__ uint32_t c_zero = 0;
 // high product takes it 4 cycles of a warp, a low product 2, 10 in all per
 // Montgomery product; measured), and the compiler likes to spread two-operand
 // adds onto that pipe as multiply-adds. A third operand it cannot see to be
-// zero keeps the subtraction on the ALU pipe: 8 % less time for the whole
-// permutation (1.90 against 2.03 ms for 2^20 threads x 8 permutations, before
-// the partial rounds below were rearranged; 1.74 against 1.83 ms after).
+// zero keeps the subtraction on the ALU pipe: 5 % less time for the whole
+// permutation (1.74 against 1.83 ms for 2^20 threads x 8 permutations).
 template <class F>
 __device__ __forceinline__ int32_t smul3(int32_t a, int32_t b) {
   const int64_t c = (int64_t)a * b;
@@ -190,25 +189,6 @@ __device__ __forceinline__ int32_t sredc(int64_t c) {
   return (int32_t)(c >> 32) - __mulhi((int32_t)m, (int32_t)F::P);
 }
 
-// The built-in BabyBear-16 instance (x^7, 4 + 4 full and 13 partial rounds),
-// one state per thread.
-//
-// What bounds it: the FMA pipe's multiplier (564 Montgomery products, 5,640
-// cycles of a warp) and the ALU pipe, which every high or wide product also
-// holds for 2 cycles and every other instruction for 2; together 93 % of what
-// the two pipes can give. So an instruction saved is about a cycle saved, and
-// the partial rounds, 13 x 118 instructions as written in the definition, are
-// rearranged to need fewer:
-//  - The diagonal [-2, 1, 2, 1/2, 3, 4, -1/2, -3, -4, 2^-8, 1/4, 1/8, 2^-27,
-//    -2^-8, -1/16, -2^-27] holds five pairs (d, -d), at words (3, 6), (4, 7),
-//    (5, 8), (9, 13), (12, 15). A pair (a, b) is carried as h = (a + b)/2 and
-//    g = (a - b)/2: then h' = sum + d g and g' = d h, so the sum over the
-//    words needs one addition per pair, the update one addition per pair, and
-//    over two rounds h'' = sum' + d^2 h with no g at all.
-//  - Multiplications by 2^-k need no product: p = 15 * 2^27 + 1, so with q the
-//    low k bits of x, x 2^-k = (x >> k) - q * 15 * 2^(27-k), in (-p, p).
-// 87 instructions per partial round, 5,190 per permutation (5,880 before):
-// 1.654 against 1.911 ms for 2^20 threads x 8 permutations at the same clock.
 // Products by small constants and powers of two in a field p = A 2^T + 1 with
 // 2^31 = p + 2^T - 1 (BabyBear: 15, 27; KoalaBear: 127, 24).
 template <class F>
@@ -264,6 +244,27 @@ struct Pow2 {
   }
 };
 
+// The built-in BabyBear-16 instance (x^7, 4 + 4 full and 13 partial rounds),
+// one state per thread.
+//
+// What bounds it: the FMA pipe's multiplier (564 Montgomery products, 5,640
+// cycles of a warp) and the ALU pipe, which every high or wide product also
+// holds for 2 cycles and each of the 3,498 other instructions for 2. Were both
+// always busy, that is (5,640 + 2,256 + 6,996) / 2 = 7,446 cycles; 8,100 measured
+// with eight warps a sub-partition, 92 % of it. So an instruction saved is about a cycle saved, and
+// the partial rounds, 13 x 118 instructions as written in the definition, are
+// rearranged to need fewer:
+//  - The diagonal [-2, 1, 2, 1/2, 3, 4, -1/2, -3, -4, 2^-8, 1/4, 1/8, 2^-27,
+//    -2^-8, -1/16, -2^-27] holds five pairs (d, -d), at words (3, 6), (4, 7),
+//    (5, 8), (9, 13), (12, 15). A pair (a, b) is carried as h = (a + b)/2 and
+//    g = (a - b)/2: then h' = sum + d g and g' = d h, so the sum over the
+//    words needs one addition per pair, the update one addition per pair, and
+//    over two rounds h'' = sum' + d^2 h with no g at all.
+//  - Multiplications by 2^-k need no product: p = 15 * 2^27 + 1, so with q the
+//    low k bits of x, x 2^-k = (x >> k) - q * 15 * 2^(27-k), in (-p, p).
+// 87 instructions per partial round and 5,190 per permutation, where the rounds as
+// written in the definition make 5,880: 1.654 against 1.911 ms for 2^20 threads x
+// 8 permutations at the same clock.
 struct Bb16Builtin {
   using F = BabyBear;
   static constexpr bool kOwnPermute = true;
@@ -724,8 +725,9 @@ ZC_HD void p2_compress(const uint32_t* l, const uint32_t* r, uint32_t* out,
 //    come by three independent shuffles each: two shuffle latencies per layer,
 //    not four (a butterfly's);
 //  - partial rounds: half_partials.
-// 3,725 cycles for the built-in instance (9 external layers of 118, 8 S-boxes of
-// 102, 1,912 for the partial rounds); 4,900 with butterfly sums throughout.
+// 3,720 to 3,930 cycles for the built-in instance by the code around it; 4,900 with
+// butterfly sums throughout. Its parts, each repeated by itself: an external layer
+// 122 (nine of them), an S-box 108 (eight), the partial rounds 1,837; 3,800 in all.
 // Constants come from a P2Params in shared memory. Every lane of the warp must
 // make the call (full-warp shuffles), active half or not.
 constexpr unsigned kFullMask = 0xffffffffu;

@@ -305,10 +305,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_lde_small(const uint32_t* x, ui
   lde_small_body<F>(x, out, log_k, log_b, h, blockIdx.x, sm, brev_out, kMaxRadixLog, rev, post);
 }
 
-// Pass 1 item (coset s, i1 tile, column c): the k2-point DIF NTTs down the
-// strided columns i1 of the message scaled by g_s^(i1 + k1 i2); writes the
-// untwiddled intermediate z[c][s][t2][i1] (t2 = bit-reversed position).
-
 // ---------------------------------------------------------- fused passes --
 // The four-step passes with the first radix pass fed straight from global
 // memory and the last radix pass writing straight to global memory: each
@@ -316,10 +312,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_lde_small(const uint32_t* x, ui
 // warp, all loads in flight at once), applies the coset / four-step scale
 // there, runs the R stages and writes shared memory; the middle passes are
 // dif_pass; the last pass reads shared memory, runs its stages and stores the
-// outputs at their final positions. Compared with staging the tile through
-// per-word cp.async copies, a separate scale loop and a separate output loop,
-// this removes one shared-memory round trip and two barrier-separated loops
-// per pass (the words, products and results are the same).
+// outputs at their final positions.
 
 // Balanced radix of pass q of `passes` over the stages left (h0 + 1).
 __host__ __device__ __forceinline__ int pass_radix(int h0, int passes, int q) {
@@ -394,7 +387,10 @@ __device__ __forceinline__ void p1_pass(uint32_t* work, int rs, int log_ti, int 
   }
 }
 
-// Pass-1 item with fused load and store. Layout: work[TI][rs] | tw[k2/2] |
+// Pass 1 item (coset s, i1 tile, column c): the k2-point DIF NTTs down the
+// strided columns i1 of the message scaled by g_s^(i1 + k1 i2); writes the
+// untwiddled intermediate z[c][s][t2][i1] (t2 = bit-reversed position), with
+// fused load and store. Layout: work[TI][rs] | tw[k2/2] |
 // gi[TI] | Gt[S] (S = the first pass's member stride). MR: the largest radix
 // compiled in (max_r <= MR).
 // REV: the message is read at -i mod k (an inverse transform's input order).
@@ -644,9 +640,12 @@ inline LdePlan plan_lde(int log_k, int log_b, int tile_log = 0, int max_r = kMax
 }
 
 // Whether a four-step LDE of `batch` columns of 2^log_n outputs takes the
-// wide variant: at least two of its tiles per SM (2^20 x 64 at blowup 4 with
-// one 512-thread CTA per SM: 2.10 ms against 2.23 ms for the radix-2^4 form
-// on the GB300).
+// wide variant: at least two of its tiles per SM. Wide against radix-2^4 by the
+// number of tiles, from HBM: 128 tiles 33 against 25 us (2^16 x 16 at blowup 2) and
+// 33 against 29 (2^20 x 1), 256 tiles 37.5 each (2^16 x 16 at blowup 4) and 44
+// against 46 (2^20 x 2), 384 tiles 62 against 66 (2^20 x 3), 1,024 tiles 128 against
+// 140, 16,384 tiles (2^20 x 64 at blowup 4) 1,864 against 2,045. For rows of 2^16
+// and less the even point lies higher: 2^16 x 99 at blowup 1 (396 tiles) 58 against 54.
 inline bool lde_wide(int64_t batch, int log_n) {
   static const int sms = [] {
     int dev = 0, n = 0;

@@ -1,8 +1,8 @@
 // The commit-and-fold rounds of an open in one call: what FriProver's commit
 // phase, the Basefold open and the SP1 stacked open share (zorch/pcs/fold.py:
 // 90-115, zorch/pcs/basefold/prover.py:419-480, zorch/pcs/jagged/open.py:
-// 237-330). A round used to be six to eight calls from Python, 60-80 us of
-// host time where the GPU needs 60 for a small layer; here it is launches only,
+// 237-330). A round as six to eight calls from Python is 60-80 us of host time
+// where the GPU needs 60 for a small layer; here it is launches only,
 // and its sumcheck message, root binding and transcript step run in the launch
 // that computes the layer's root.
 #include "internal.cuh"

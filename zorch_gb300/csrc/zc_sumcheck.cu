@@ -18,8 +18,8 @@ namespace zc {
 // (z[0] ends on the top bit): the tables of the upper and the lower half of the
 // variables are doubled up side by side in shared memory (out[2i] = s - s z_j,
 // out[2i+1] = s z_j), at most six dependent products, and the table is their
-// outer product. Twelve variables took 14.5 us doubled through global memory,
-// one step after another.
+// outer product. Doubled through global memory, one step after another,
+// twelve variables take 14.5 us.
 constexpr int kEqSmall = 12;
 struct EqTable {
   const uint32_t* z;
@@ -295,10 +295,10 @@ __device__ __forceinline__ ef4 rlc_weight(const uint32_t* chal, int nbv, int idx
 
 // Staggered batching with an offset into the weight table and accumulation
 // (batch_staggered, zorch/pcs/basefold/batching.py:66-80): out[j] (+)= sum_c
-// weights[offset + c] cw[c][j]. A CTA forms its w weights one per thread (one
-// thread doubling up the whole table took 10 us and more before the first
-// word), then two columns go to a reduction (ef_dot2). Bound by the columns'
-// bytes: 2^21 x 8 words in 45 us before.
+// weights[offset + c] cw[c][j]. A CTA forms its w weights one per thread, then
+// two columns go to a reduction (ef_dot2). 2^21 x 8 words from HBM take 31 us, of
+// which the bytes 15; 52 with the whole table doubled up by one thread, 10 us and
+// more before the first word, and a reduction a column.
 template <class F>
 __global__ void __launch_bounds__(256) k_rlc_ex(const uint32_t* cw, int64_t n, int w,
                                                 const uint32_t* chal, int nbv, int offset,
