@@ -26,7 +26,7 @@ from . import _lib
 from .coding import BitReversedReedSolomon
 from .commit import DigestLayers, SingleMatrixCommitmentScheme, leaves_layout
 from .field import from_mont, full_u32, ptr, stream_handle, to_host
-from .pcs import layer_spec, open_layers, run_fold_rounds
+from .pcs import check_specs, layer_spec, open_layers, run_fold_rounds
 from .transcript import DuplexTranscript
 
 
@@ -262,9 +262,10 @@ def stacked_basefold_open(smcs: SingleMatrixCommitmentScheme, code: BitReversedR
     for rd in rounds:
         K = rd.codeword.shape[0]
         specs.append((leaves_layout(rd.codeword, n, K, 1, n), rd.digest_layers, K, 0))
+    check_specs(specs)
     opened = [(op.row, op.path) for op in
               open_layers(specs + [layer_spec(ly, i, True) for i, ly in enumerate(fr.layers)],
-                          positions)]
+                          positions, check=False)]
     proof = StackedOpenProof(
         [rd.commitment for rd in rounds], fr.raw_roots, fr.roots, fr.msgs.view(v, 2, 4),
         final_poly, witness, batch_evals, opened[:len(specs)], opened[len(specs):], positions)

@@ -431,17 +431,26 @@ def step_fold_rounds(tree: MerkleTree, code, codeword: torch.Tensor, rounds: int
                       stack_rows(betas, (limbs,), dev), cw, msgs)
 
 
-def open_layers(specs: Sequence[tuple], positions: torch.Tensor) -> list[Opening]:
-    """Openings of the same positions in several trees, one launch
-    (zc_open_layers): specs are (leaf layout, digest layers, leaf width, shift),
-    each opened at leaf (position >> shift) mod num_leaves. A tree that is not the
-    layout's is refused (ValueError): the kernel takes its depth from the layout."""
+def check_specs(specs: Sequence[tuple]) -> None:
+    """Refuses (ValueError) an open_layers spec whose tree is not its layout's: the
+    kernel takes a tree's depth from the layout."""
     for lv, dl, width, _ in specs:
         if (dl.num_leaves != lv.num_leaves or dl.flat.numel() != 8 * (2 * lv.num_leaves - 1)
                 or width != lv.groups * lv.group_len):
             raise ValueError(f"opening of {lv.num_leaves} leaves of {lv.groups * lv.group_len} "
                              f"words: the tree has {dl.num_leaves} leaves and "
                              f"{tuple(dl.flat.shape)} digest words, the width is {width}")
+
+
+def open_layers(specs: Sequence[tuple], positions: torch.Tensor,
+                check: bool = True) -> list[Opening]:
+    """Openings of the same positions in several trees, one launch
+    (zc_open_layers): specs are (leaf layout, digest layers, leaf width, shift),
+    each opened at leaf (position >> shift) mod num_leaves. `check` (check_specs)
+    is a microsecond a tree: an open checks the caller's trees and leaves out the
+    layers of its own rounds."""
+    if check:
+        check_specs(specs)
     idx = positions.to(torch.int32).contiguous()
     q = idx.numel()
     sizes = []
@@ -552,6 +561,7 @@ class FriProver:
         p = self.params
         n0 = codeword.shape[0]
         br = p.code.bit_reversed
+        check_specs(extra)
         if 1 <= p.num_rounds <= n0.bit_length() - 1 and n0 & (n0 - 1) == 0:
             fr = run_fold_rounds(p.tree.perm, p.code, codeword, p.num_rounds, p.challenge_limbs,
                                  t, first_layer)
@@ -562,7 +572,7 @@ class FriProver:
         state = FoldState(final, tuple(fr.layers), None if fr.layers else first_layer, betas)
         positions = t.sample_positions_(n0, p.num_queries, values=final)
         specs = [layer_spec(layer, i, br) for i, layer in enumerate(state.layers)]
-        ops = open_layers([*specs, *extra], positions) if specs or extra else []
+        ops = open_layers([*specs, *extra], positions, check=False) if specs or extra else []
         proof = CommitPhaseProof(roots, list(betas), final, positions, ops[:len(specs)])
         return proof, state, ops[len(specs):]
 
@@ -979,8 +989,9 @@ class BasefoldProver:
         for pd in rounds:
             K, nc = pd.codeword.shape
             specs.append((leaves_layout(pd.codeword, nc, K, 1, nc), pd.digest_layers, K, 0))
+        check_specs(specs)
         ops = open_layers(specs + [layer_spec(ly, i, code.bit_reversed)
-                                   for i, ly in enumerate(fr.layers)], positions)
+                                   for i, ly in enumerate(fr.layers)], positions, check=False)
         proof = BasefoldProof(fr.msgs, fr.roots, final, ops[:len(specs)], ops[len(specs):],
                               positions)
         return values, proof, t
