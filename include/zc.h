@@ -402,7 +402,10 @@ zc_status zc_ef4_limbs(const uint32_t* in, int64_t n, int32_t to_limbs, uint32_t
  * prover.py:419-480) and the SP1 stacked open (zorch/pcs/jagged/open.py:237-330)
  * run them: per round commit the layer's pair leaves, observe the sumcheck
  * message (if any) and the root, squeeze beta, fold. No host synchronisation,
- * no allocation. */
+ * no allocation. A call that is refused -- log_n past the field's two-adicity
+ * (ZC_BAD_SHAPE), a generator that is not built (ZC_UNSUPPORTED), a shift that is
+ * no field element or a misaligned buffer (ZC_BAD_ARG), a short workspace
+ * (ZC_OOM) -- queues nothing and leaves the state as it was. */
 typedef struct {
   int32_t rounds;        /* >= 1 */
   int32_t log_n;         /* layer 0 has 2^log_n points, log_n >= rounds */
